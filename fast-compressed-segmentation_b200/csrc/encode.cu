@@ -20,7 +20,7 @@
 //      out nibbles with a block scan and packs them.  Also records, for the
 //      seek index, the nibble and palette index of every S-th op.
 //   K2 model: buildRansModel on the shared 16-bin histogram.
-//   K3 rans: one thread per brick, symbols in reverse; while encoding it also
+//   K3 rans: one chain per brick, symbols in reverse; while encoding it also
 //      records the decoder state at the seek checkpoints (the decoder's state
 //      before symbol i is the encoder's state after symbol i).
 //   K4 serialize: header + records, file order.
@@ -615,95 +615,223 @@ __global__ void model_kernel(const unsigned long long* hist, uint32_t* model) {
 }
 
 // ------------------------------------------------------------ K3 rANS
-// One encode step (ransEncodeSymbol, brickEncoding.cpp:202-219).  tab: f |
-// start << 13 | shift << 25 | M << 32.  The state is below 2^31 before the step
-// (brickEncoding: 2^19 f after renormalisation, times 4096 / f), so at most two
-// bytes leave per symbol and the reciprocal division is exact.
-__device__ __forceinline__ void rans_enc_step(uint32_t& x, uint32_t& emitted, uint8_t* __restrict__ out,
-                                              uint64_t e) {
-    const uint32_t f = (uint32_t)e & 0x1FFFu;
-    const uint32_t bound = ((kRansL >> kTotBits) << 8) * f;
-    if (x >= bound) {
-        out[emitted++] = (uint8_t)(x & 0xFF);
-        x >>= 8;
-        if (x >= bound) {
-            out[emitted++] = (uint8_t)(x & 0xFF);
-            x >>= 8;
-        }
-    }
-    const uint32_t qd = (uint32_t)(((uint64_t)x * (uint32_t)(e >> 32)) >> ((uint32_t)(e >> 25) & 63u));
-    x = (qd << kTotBits) + (x - qd * f) + (((uint32_t)e >> 13) & 0xFFFu);
+// ransEncodeSymbol (brickEncoding.cpp:202-219) on the state x < 2^31 (brickEncoding:
+// 2^19 f after renormalisation, times 4096 / f):
+//     y = x without the bytes that leave (one when x >= f << 19, a second when
+//         x >= f << 27, which takes f < 16)
+//     x' = y + start + (y / f) (4096 - f)
+// as a chain of steps that put out at most one byte each, all of one form:
+//     x' = x >= bound ? (x >> 8) + start + ((h >> s) >> 8) mul : x + start + (h >> s) mul,
+//     h = the high half of x M
+// With M = ceil(2^(31 + ceil(log2 f)) / f), h >> s is exactly x / f (Granlund &
+// Montgomery, as model_kernel), and (x >> 8) / f is (x / f) >> 8, so both outcomes come
+// from one multiplication and the comparison is off the chain of multiply, shift,
+// multiply-add, select: 23 cycles (measured; 38 with the select first, whose comparison
+// alone takes about 14).  A symbol with f < 16 takes a step before that only drops a
+// byte (M = mul = 0); f = 1, which has no such M, takes two, then M = 2^32 - 1, which
+// gives x - 1, and start + 4095.  An entry is {M, bound, mul, start << 5 | s}.
+__device__ __forceinline__ uint4 rans_entry(const uint32_t* __restrict__ md, uint32_t s) {
+    const uint32_t f = md[s], start = md[16 + s], sh = md[49 + s] - 31;
+    return f == 1 ? make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, kTot - f, (start + kTot - 1) << 5)
+                  : make_uint4(md[33 + s], f << 19, kTot - f, start << 5 | (sh - 1));
+}
+__device__ __forceinline__ void rans_enc_step(uint32_t& x, const uint4 t) {
+    const uint32_t h = __umulhi(x, t.x), start = t.w >> 5;
+    const uint32_t xa = x + start + __funnelshift_r(h, 0u, t.w) * t.z;  // (shifts by t.w & 31)
+    const uint32_t xb = (x >> 8) + start + __funnelshift_r(h, 0u, t.w + 8) * t.z;
+    x = x >= t.y ? xb : xa;
 }
 
-__global__ void __launch_bounds__(128) enc_rans_kernel(EncMeta* __restrict__ meta, uint32_t nb,
-                                                       const uint8_t* __restrict__ nib_pool,
-                                                       const uint64_t* __restrict__ enc_off,
-                                                       uint8_t* __restrict__ enc_pool, const uint32_t* __restrict__ model,
-                                                       uint32_t n_tables, Checkpoint* __restrict__ ck_all,
-                                                       uint32_t lanes) {
-    __shared__ uint64_t tabs[kMaxTables * 16];
-    for (uint32_t k = threadIdx.x; k < 16 * n_tables; k += blockDim.x) {
-        const uint32_t* md = model + (k >> 4) * kModelWords;
-        const uint32_t s = k & 15u;
-        tabs[k] = (uint64_t)md[s] | ((uint64_t)md[16 + s] << 13) | ((uint64_t)md[49 + s] << 25) |
-                  ((uint64_t)md[33 + s] << 32);
-    }
-    __syncthreads();
-    // One serial chain per brick; a warp takes only `lanes` bricks (lanes
-    // 0 .. lanes-1) when there are few bricks, so that lanes do not run the
-    // union of other bricks' branch paths and the SM interleaves many warps.
-    const uint32_t lane = threadIdx.x & 31;
-    if (lane >= lanes) return;
-    const uint32_t i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lanes + lane;
-    if (i >= nb) return;
-    const EncMeta m = meta[i];
-    if (m.flags & EF_OVERFLOW) return;
-    const uint64_t* tab = tabs + 16 * min((m.sel >> 4) & 15u, n_tables - 1);
-    // the packed nibbles of a brick start 16-byte aligned and are padded to 16
-    const uint4* src4 = reinterpret_cast<const uint4*>(nib_pool + m.nib_off);
-    uint8_t* out = enc_pool + enc_off[i];
-    Checkpoint* ck = ck_all + m.ck_off;
-    int k = (int)m.n_ck - 1;
-    // the next checkpoint's symbol index, and the one after it loaded a
-    // checkpoint ahead so that the load is off the serial chain
-    uint32_t next = k >= 0 ? ck[k].sym : 0xFFFFFFFFu;
-    uint32_t after = k >= 1 ? ck[k - 1].sym : 0xFFFFFFFFu;
-    uint32_t x = kRansL, emitted = 0;
-    const int nchunk = (int)((m.nbytes + 15) / 16);
-    uint4 cur = nchunk > 0 ? src4[nchunk - 1] : make_uint4(0, 0, 0, 0);
-    for (int c16 = nchunk - 1; c16 >= 0; --c16) {
-        const uint4 nxt = c16 > 0 ? src4[c16 - 1] : make_uint4(0, 0, 0, 0);  // prefetch
-        const uint32_t words[4] = {cur.x, cur.y, cur.z, cur.w};
+// A brick's symbols are one dependent chain, and the longest brick's is the kernel's
+// time, so one warp of a block does nothing else: lane k runs brick k's steps, in
+// batches of 64 or 128, on entries read ahead from shared memory, and leaves the states
+// there.  Each of the K bricks has a warp of its own that meanwhile turns the next
+// symbols into steps and works out from the last batch's states the bytes they put out,
+// their place (a ballot prefix) and the seek checkpoints among them; its global loads
+// come 1024 symbols (nibbles) or 32 checkpoints at a time.  K = 1 while there are no
+// more bricks than warp schedulers, so that no chain shares one; beyond, several chains
+// per warp, since a chain's step costs the scheduler as much for one lane as for many.
+// Measured against one lane per brick that did all of it (165 cycles per symbol): 512
+// bricks of 64^3, longest 84,720 symbols, 7.24 -> 1.45 ms (K = 1, 33 cycles per
+// symbol); 8192 bricks of 32^3 0.91 -> 0.30 ms (K = 8; 0.67 with K = 1); 60 bricks of
+// 32^3 0.60 -> 0.11 ms.  Batches of 128 against 64 with K = 1: 1.45 against 1.55 ms.
+template <uint32_t kRansBatch>
+struct RansBrick {
+    static constexpr uint32_t kRing = 4 * kRansBatch;
+    uint4 ring[kRing];          // steps, in order, modulo kRing
+    uint4 tab[16];              // the model's entries
+    uint4 nib[32];              // packed nibbles of 1024 symbols
+    uint32_t x[2][kRansBatch];  // the state before each step of two batches
+    uint32_t end[2];            // and after their last one
+    uint16_t ck[kRing];         // 1 + the checkpoint whose symbol the step completes, or 0
+};
+static_assert(sizeof(RansBrick<64>) % 128 == 16, "eight bricks' entries are read from different banks");
+template <int K, uint32_t kRansBatch>
+__global__ void __launch_bounds__(32 * (K + 1)) enc_rans_kernel(EncMeta* __restrict__ meta, uint32_t nb,
+                                                                const uint8_t* __restrict__ nib_pool,
+                                                                const uint64_t* __restrict__ enc_off,
+                                                                uint8_t* __restrict__ enc_pool,
+                                                                const uint32_t* __restrict__ model, uint32_t n_tables,
+                                                                Checkpoint* __restrict__ ck_all, uint32_t n_sm) {
+    constexpr uint32_t kRansRing = RansBrick<kRansBatch>::kRing;
+    __shared__ RansBrick<kRansBatch> s_bricks[K];
+    const uint32_t lane = threadIdx.x & 31, FULL = 0xFFFFFFFFu;
+    // the chain's warp: the first or the last one, in turn, so that the chains of an SM's blocks (of two
+    // warps each) do not meet on two of its four schedulers
+    const uint32_t chain_warp = (blockIdx.x / n_sm) & 1u ? K : 0u, warp = threadIdx.x >> 5;
+    if (warp == chain_warp) {
+        auto& B = s_bricks[min(lane, (uint32_t)K - 1)];
+        uint32_t x = kRansL;
+        uint4 ea[8], eb[8];
+        auto fetch = [&](const uint4* r, uint4 (&e)[8]) {
 #pragma unroll
-        for (int b = 15; b >= 0; --b) {
-            const uint32_t q = 16u * (uint32_t)c16 + (uint32_t)b;
-            if (q >= m.nbytes) continue;
-            const uint32_t byte = (words[b >> 2] >> (8 * (b & 3))) & 0xFFu;
-            // low nibble (symbol 2q+1) first: the symbols go in reverse order
-            rans_enc_step(x, emitted, out, tab[byte & 15u]);
-            if (2 * q + 1 == next) {
-                ck[k].state = x;
-                ck[k].pos = emitted;
-                --k;
-                next = after;
-                after = k >= 1 ? ck[k - 1].sym : 0xFFFFFFFFu;
+            for (int k = 0; k < 8; ++k) e[k] = r[k];
+        };
+        auto code = [&](const uint4 (&e)[8], uint4* xs) {
+            uint32_t st[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                st[k] = x;
+                rans_enc_step(x, e[k]);
             }
-            rans_enc_step(x, emitted, out, tab[byte >> 4]);
-            if (2 * q == next) {
-                ck[k].state = x;
-                ck[k].pos = emitted;
-                --k;
-                next = after;
-                after = k >= 1 ? ck[k - 1].sym : 0xFFFFFFFFu;
+            xs[0] = make_uint4(st[0], st[1], st[2], st[3]);
+            xs[1] = make_uint4(st[4], st[5], st[6], st[7]);
+        };
+        __syncthreads();
+        for (uint32_t n = 0;; ++n) {
+            if (lane < K) {
+                const uint4* ring = B.ring + (n * kRansBatch) % kRansRing;
+                uint4* xs = reinterpret_cast<uint4*>(B.x[n & 1]);
+                fetch(ring, ea);
+#pragma unroll 1
+                for (uint32_t k = 0; k < kRansBatch / 16; ++k) {
+                    fetch(ring + 8, eb);
+                    code(ea, xs);
+                    ring += 16;
+                    if (k + 1 < kRansBatch / 16) fetch(ring, ea);
+                    code(eb, xs + 2);
+                    xs += 4;
+                }
+                B.end[n & 1] = x;
+            }
+            if (!__syncthreads_or(0)) return;
+        }
+    }
+    const uint32_t kb = chain_warp ? warp : warp - 1, i = blockIdx.x * K + kb;
+    auto& B = s_bricks[kb];
+    uint32_t n_sym = 0, n_ck = 0, tables = 0;
+    uint64_t nib_off = 0;
+    Checkpoint* ck = ck_all;
+    uint8_t* out = enc_pool;
+    const bool have = i < nb && !(meta[i].flags & EF_OVERFLOW);
+    if (have) {
+        const EncMeta& m = meta[i];
+        n_sym = 2 * m.nbytes;  // symbols coded, the pad nibble of an odd count included
+        n_ck = m.n_ck;
+        nib_off = m.nib_off;
+        tables = min((m.sel >> 4) & 15u, n_tables - 1);
+        ck += m.ck_off;
+        out += enc_off[i];
+    }
+    if (lane < 16) B.tab[lane] = rans_entry(model + tables * kModelWords, lane);
+    // the packed nibbles start 16-byte aligned and are padded to 16: a chunk of 32 symbols is 16 bytes
+    const uint4* src = reinterpret_cast<const uint4*>(nib_pool + nib_off);
+    const uint32_t n16 = (n_sym + 31) / 32;
+    auto load_nib = [&](int blk) -> uint4 {
+        const uint32_t q = 32u * (uint32_t)blk + lane;
+        return blk >= 0 && q < n16 ? src[q] : make_uint4(0, 0, 0, 0);
+    };
+    // checkpoints (they have ascending symbols; the chain runs backwards): lane l holds the symbol of
+    // checkpoint ck_base - 1 - l; n_ck are left.  A chunk has at most two (16 ops apart).
+    uint32_t ck_base = n_ck, ck_sym = lane < n_ck ? ck[n_ck - 1 - lane].sym : 0u;
+    const uint32_t lt = (1u << lane) - 1u, le = (2u << lane) - 1u;
+    int chunk = (int)n16 - 1;  // the next chunk to turn into steps
+    uint4 nib_next = load_nib(chunk >> 5);
+    bool fresh = true;         // nib_next is the chunk's block
+    uint32_t made = 0;         // steps so far
+    uint32_t n_batches = have ? 0xFFFFFFFFu : 0u;  // known once every symbol has its steps
+    const uint32_t rel = 31 - lane;  // lane l takes the chunk's symbol 31 - l (a byte's low nibble is the later one)
+    auto produce = [&](uint32_t target) {
+        while (made < target && chunk >= 0) {
+            if (fresh || (chunk & 31) == 31) {
+                __syncwarp();
+                B.nib[lane] = nib_next;
+                nib_next = load_nib((chunk >> 5) - 1);
+                fresh = false;
+                __syncwarp();
+            }
+            const uint32_t sym = 32u * (uint32_t)chunk + rel;
+            const uint32_t byte = reinterpret_cast<const uint8_t*>(B.nib)[16 * (chunk & 31) + (rel >> 1)];
+            const uint4 t = B.tab[(rel & 1u) ? byte & 15u : byte >> 4];
+            const bool valid = sym < n_sym;
+            const bool one = t.x == 0xFFFFFFFFu, few = one || t.y < (16u << 19);  // f = 1, f < 16
+            const uint32_t m0 = __ballot_sync(FULL, valid), m1 = __ballot_sync(FULL, valid && few),
+                           m2 = __ballot_sync(FULL, valid && one);
+            // the chunk's checkpoints, as a mask of its steps' order
+            const uint32_t due = lane >= ck_base - n_ck && lane < ck_base && (ck_sym >> 5) == (uint32_t)chunk
+                                     ? 0x80000000u >> (ck_sym & 31u)
+                                     : 0u;
+            const uint32_t mc = __reduce_or_sync(FULL, due);
+            if (valid) {
+                uint32_t s = made + __popc(m0 & lt) + __popc(m1 & lt) + __popc(m2 & lt);
+                if (few) {
+                    const uint32_t f = one ? 1u : t.y >> 19;
+                    B.ring[s % kRansRing] = make_uint4(0u, f << 27, 0u, 0u);
+                    B.ck[s % kRansRing] = 0;
+                    ++s;
+                }
+                if (one) {
+                    B.ring[s % kRansRing] = make_uint4(0u, 1u << 19, 0u, 0u);
+                    B.ck[s % kRansRing] = 0;
+                    ++s;
+                }
+                B.ring[s % kRansRing] = t;
+                B.ck[s % kRansRing] = (mc >> lane) & 1u ? (uint16_t)(n_ck - __popc(mc & lt)) : (uint16_t)0;
+            }
+            made += __popc(m0) + __popc(m1) + __popc(m2);
+            n_ck -= __popc(mc);
+            if (ck_base - n_ck > 30 && n_ck) {
+                ck_base = n_ck;
+                ck_sym = lane < n_ck ? ck[n_ck - 1 - lane].sym : 0u;
+            }
+            --chunk;
+        }
+        if (chunk < 0 && n_batches == 0xFFFFFFFFu) {  // the last batch is filled up with steps that do nothing
+            n_batches = (made + kRansBatch - 1) / kRansBatch;
+            for (uint32_t s = made + lane; s < n_batches * kRansBatch; s += 32) {
+                B.ring[s % kRansRing] = make_uint4(0u, 0xFFFFFFFFu, 0u, 0u);
+                B.ck[s % kRansRing] = 0;
             }
         }
-        cur = nxt;
+    };
+    if (have) produce(kRansBatch);
+    uint32_t emitted = 0;
+    __syncthreads();
+    for (uint32_t n = 0;; ++n) {
+        if (n >= 1 && n <= n_batches) {  // what batch n - 1 put out
+            const uint32_t d = (n - 1) & 1u;
+#pragma unroll
+            for (uint32_t h = 0; h < kRansBatch / 32; ++h) {
+                const uint32_t j = 32 * h + lane, s = ((n - 1) * kRansBatch + j) % kRansRing;
+                const uint32_t x = B.x[d][j], id = B.ck[s];
+                const uint32_t b = __ballot_sync(FULL, x >= B.ring[s].y);
+                if ((b >> lane) & 1u) out[emitted + __popc(b & lt)] = (uint8_t)x;
+                if (id) {  // a checkpoint's state, the decoder's before its symbol, is the encoder's after it
+                    ck[id - 1].state = j + 1 < kRansBatch ? B.x[d][j + 1] : B.end[d];
+                    ck[id - 1].pos = emitted + __popc(b & le);
+                }
+                emitted += __popc(b);
+            }
+            if (n == n_batches) {
+                const uint32_t x = B.end[d];
+                if (lane < 4) out[emitted + lane] = (uint8_t)(x >> (8 * lane));  // ransFlush, little-endian
+                if (lane == 0) meta[i].E = emitted + 4;
+            }
+            __syncwarp();  // its steps make room for new ones
+        }
+        if (n_batches == 0xFFFFFFFFu) produce((n + 2) * kRansBatch);
+        if (!__syncthreads_or(n < n_batches)) return;
     }
-    for (int b = 0; b < 4; ++b) {  // ransFlush, little-endian
-        out[emitted++] = (uint8_t)(x & 0xFF);
-        x >>= 8;
-    }
-    meta[i].E = emitted;
 }
 
 // ------------------------------------------------------------ K4 serialize
@@ -978,7 +1106,6 @@ static int finish_encode(EncoderState* s, const EncodeSelection* sel, cudaStream
     const uint32_t nb = s->nb, b = s->b;
     const uint32_t n_tables = sel ? sel->n_tables : 0;
     const bool v2 = n_tables > 0;
-    const int device = s->device;
     std::vector<uint32_t> models(kMaxTables * kModelWords, 0);
     if (v2) {  // the caller's shared tables
         for (uint32_t t = 0; t < n_tables; ++t) table_model(sel->freq[t], &models[t * kModelWords]);
@@ -1012,14 +1139,16 @@ static int finish_encode(EncoderState* s, const EncodeSelection* sel, cudaStream
     CK(grow(&s->d_rec_off, &s->rec_cap, std::max<uint32_t>(nb, 1)));
     CK(cudaMemcpyAsync(s->d_enc_off, enc_off.data(), 8ull * nb, cudaMemcpyHostToDevice, st));
     if (nb) {
-        // bricks per warp: the fewest (a power of two) that keeps about 32 warps per SM or fewer
         int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        uint32_t lanes = 1;
-        while (lanes < 32 && (nb + lanes - 1) / lanes > 32ull * (uint64_t)std::max(sms, 1)) lanes <<= 1;
-        const uint32_t per_block = 4 * lanes;  // four warps per block share the tables
-        enc_rans_kernel<<<(nb + per_block - 1) / per_block, 128, 0, st>>>(
-            s->d_meta, nb, s->d_nib, s->d_enc_off, s->d_enc, s->d_model, s->n_tables, s->d_ck, lanes);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+        const uint32_t n_sm = (uint32_t)std::max(sms, 1);
+        auto rans = [&](auto kernel, uint32_t K) {
+            kernel<<<(nb + K - 1) / K, 32 * (K + 1), 0, st>>>(s->d_meta, nb, s->d_nib, s->d_enc_off, s->d_enc,
+                                                             s->d_model, s->n_tables, s->d_ck, n_sm);
+        };
+        if (nb <= 4 * n_sm) rans(enc_rans_kernel<1, 128>, 1);
+        else if (nb <= 16 * n_sm) rans(enc_rans_kernel<4, 64>, 4);
+        else rans(enc_rans_kernel<8, 64>, 8);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(s->h_meta.data(), s->d_meta, sizeof(EncMeta) * nb, cudaMemcpyDeviceToHost, st));
     }
