@@ -34,6 +34,7 @@
 
 #include "block_scan.cuh"
 #include "csv_internal.h"
+#include "majority.cuh"
 
 namespace csv {
 
@@ -109,53 +110,6 @@ void encoder_state_free(EncoderState* s) {
     cudaFree(s->d_model);
     cudaFree(s->d_image);
     delete s;
-}
-
-// ------------------------------------------------------------ majority
-// majorityVote8 (brick.hpp:24-37) under GNU libstdc++: the unordered_map has
-// 13 buckets for <= 8 keys and the identity hash.  Its iteration list holds
-// bucket groups newest-group-first and keys newest-first inside a group, and
-// max_element keeps the first maximal count.  So among the labels with the
-// largest count the winner is the one whose bucket group appeared last and,
-// within the group, the label that appeared last.  Positions of first
-// appearance stand in for insertion order.
-__device__ __forceinline__ uint64_t majority8(const uint64_t v[8]) {
-    bool all = true;
-#pragma unroll
-    for (int i = 1; i < 8; ++i) all &= (v[i] == v[0]);
-    if (all) return v[0];
-    uint32_t bkt[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) bkt[i] = (uint32_t)(v[i] % 13ull);
-    int best = 0, bcnt = -1, bgrp = -1;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        bool first = true;
-        int cnt = 0, grp = i;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            bool eq = v[j] == v[i];
-            if (j < i && eq) first = false;
-            cnt += eq ? 1 : 0;
-        }
-        // first key (by appearance) sharing this bucket
-#pragma unroll
-        for (int j = 7; j >= 0; --j) {
-            if (j < i) {
-                bool key_j = true;
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if (k < j && v[k] == v[j]) key_j = false;
-                if (key_j && bkt[j] == bkt[i]) grp = j;
-            }
-        }
-        if (first && (cnt > bcnt || (cnt == bcnt && (grp > bgrp || (grp == bgrp && i > best))))) {
-            best = i;
-            bcnt = cnt;
-            bgrp = grp;
-        }
-    }
-    return v[best];
 }
 
 __device__ __forceinline__ uint32_t demorton_axis(uint32_t m) {
@@ -311,10 +265,8 @@ __device__ void build_pyramid(const BrickCtx& B) {
             uint64_t v[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c) v[c] = voxel(B, 2 * x + (c & 1), 2 * y + ((c >> 1) & 1), 2 * z + (c >> 2));
-            uint64_t maj = majority8(v);
-            bool same = true;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) same &= (v[c] == maj);
+            bool same;
+            uint64_t maj = majority8(v, same);
             uint32_t m = morton3(x, y, z);
             if (lvl < kEncSmemLevels) {
                 S.lab[((1u << (3 * lvl)) - 1) / 7 + m] = maj;
@@ -336,10 +288,9 @@ __device__ void build_pyramid(const BrickCtx& B) {
                 v[c] = node_label(B, l + 1, 8 * m + c);
                 cc &= node_const(B, l + 1, 8 * m + c);
             }
-            uint64_t maj = majority8(v);
-            bool same = cc;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) same &= (v[c] == maj);
+            bool same;
+            uint64_t maj = majority8(v, same);
+            same &= cc;
             S.lab[((1u << (3 * l)) - 1) / 7 + m] = maj;
             S.cst[((1u << (3 * l)) - 1) / 7 + m] = same;
         }
