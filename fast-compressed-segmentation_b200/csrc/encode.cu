@@ -12,13 +12,13 @@
 //
 // Pipeline (one launch each):
 //   K1 enc_bricks: one CTA per brick (persistent).  Builds the majority pyramid
-//      straight from the volume (no Morton-ordered copy of the leaves), chooses
-//      Rp/Rx/Ry/Rz for every child of every non-constant parent in parallel,
-//      leaves the palette ops to one warp that walks the ops in stream order
-//      with a 17-entry window of the most recent palette entries (reverse find
-//      only matters up to distance 16: farther or absent means Pa), then lays
-//      out nibbles with a block scan and packs them.  Also records, for the
-//      seek index, the nibble and palette index of every S-th op.
+//      straight from the volume (no Morton-ordered copy of the leaves) and the
+//      list of its non-constant nodes, chooses Rp/Rx/Ry/Rz for each of their
+//      children in parallel, leaves the palette ops to one warp that walks them
+//      in stream order with a 17-entry window of the most recent palette entries
+//      (reverse find only matters up to distance 16: farther or absent means Pa),
+//      then lays out nibbles with a block scan and packs them.  Also records, for
+//      the seek index, the nibble and palette index of every S-th op.
 //   K2 model: buildRansModel on the shared 16-bin histogram.
 //   K3 rans: one chain per brick, symbols in reverse; while encoding it also
 //      records the decoder state at the seek checkpoints (the decoder's state
@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "block_scan.cuh"
@@ -38,9 +39,7 @@
 
 namespace csv {
 
-constexpr int kEncThreads = 512;
 constexpr uint32_t kEncSmemLevels = 5;  // levels 0..4 in shared memory
-constexpr uint32_t kEncSmemNodes = 4681;
 constexpr uint32_t OP_PALNEED = 7;  // placeholder code until the palette walk decides P0 / Pd / Pa
 constexpr uint32_t EF_UNIFORM = 1u, EF_OVERFLOW = 2u;
 // Encoder counters (u64 words): 0 nibble pool head, 1 palette pool head,
@@ -150,40 +149,98 @@ struct EncArgs {
     uint32_t index_base;  // file index of brick 0 in the larger volume (the model's sample rule)
     unsigned long long* misc;
     const uint8_t* sel;  // per brick: mode | table << 4 (null: mode 0, table 0)
+    bool pairs;          // voxels 2k, 2k + 1 of a row are a 16-byte aligned pair
 };
 
-struct EncShared {
-    uint64_t lab[kEncSmemNodes];
-    uint8_t cst[kEncSmemNodes];
-    uint32_t sh32[kEncThreads / 32 + 1];
-    uint32_t hist[16];
-    uint32_t work, P;
+// Nodes and activity words of the levels: level l has 8^l nodes from lvl_off(l) on and
+// one bit per node (set: the node is not constant, so its children have ops) in words
+// from moff(l) on.
+__host__ __device__ constexpr uint32_t lvl_off(uint32_t l) { return ((1u << (3 * l)) - 1) / 7; }
+__host__ __device__ constexpr uint32_t mwords(uint32_t l) { return l < 2 ? 1u : (1u << (3 * l)) / 32; }
+__host__ __device__ constexpr uint32_t moff(uint32_t l) { return l < 2 ? l : 2 + (lvl_off(l) - 9) / 32; }
+static_assert(moff(2) == 2 && moff(3) == 4 && moff(5) == 148 && moff(6) == 1172, "one word below 32 nodes");
+
+// A level's labels lie in raster order (x fastest, l bits an axis), so that neighbours are
+// an addition away; its activity bits and its ops in Morton order, the stream's.
+//
+// A block's shared memory: fixed part, then the labels of levels 0 .. min(L - 2, 4), the
+// activity words of levels 0 .. L - 2, then staging.
+struct EncFixed {
+    uint32_t sh32[33];
+    uint32_t hist[64];
+    uint32_t level_r[8];  // active nodes before level l's, l = 0 .. L - 1
+    uint32_t work, P, n_pd, n_act;
     uint64_t nib_off, pal_off, ck_off;
 };
+__host__ __device__ inline uint32_t enc_lab_nodes(uint32_t L) {
+    return lvl_off(L - 1 < kEncSmemLevels ? L - 1 : kEncSmemLevels);
+}
+template <int T>
+__host__ __device__ inline uint32_t enc_smem(uint32_t L) {
+    const uint32_t lab = (8 * enc_lab_nodes(L) + 15) & ~15u, nw = (moff(L - 1) + 7) & ~7u;
+    return lab + 4 * nw + T * 16 + 32;
+}
+// Active nodes whose palette ops the walk lists at a time (their ops numbered in 16 bits).
+template <int T>
+constexpr uint32_t kWalkParents = T * 16 * 8 <= 65536 ? T * 16 : 8192;
+// A block's scratch in global memory (it stays in L2).
+struct EncScratch {
+    uint64_t lab, ops, need8, act, pal, bytes;  // offsets, and all of it
+};
+template <int T>
+__host__ __device__ inline EncScratch enc_scratch(uint32_t L) {
+    const uint64_t max_ops = ((1ull << (3 * L)) - 8) / 7, max_act = lvl_off(L - 1);
+    auto align = [](uint64_t v) { return (v + 255) & ~255ull; };
+    // the walk's list of a block's worth of parents takes the active nodes' place
+    const uint64_t list = 2 * 8 * (max_act < kWalkParents<T> ? max_act : kWalkParents<T>);
+    EncScratch X;
+    X.lab = 0;
+    X.ops = L >= kEncSmemLevels + 2 ? align(8ull << (3 * (L - 2))) : 0;
+    X.need8 = align(X.ops + max_ops + 16);
+    X.act = align(X.need8 + max_act + 16);
+    X.pal = align(X.act + (4 * max_act > list ? 4 * max_act : list));
+    X.bytes = align(X.pal + 8 * max_ops);
+    return X;
+}
 
 struct BrickCtx {
     const EncArgs* A;
-    EncShared* S;
-    uint64_t x0, y0, z0;
-    uint64_t* lab_g;
-    uint8_t* cst_g;
+    EncFixed* S;
+    uint64_t* lab;   // shared: labels of levels 0 .. 4
+    uint32_t* mask;  // shared: activity words
+    uint8_t* room;   // shared: staging (before: the pyramid's queues)
+    uint64_t* lab_g;  // scratch: labels of level 5
+    uint8_t* ops;     // scratch: code | stop << 3 | delta << 4, in stream order
+    uint8_t* need8;   // scratch: per active node, which of its children take a palette op
+    uint32_t* act;    // scratch: the active nodes in stream order, raster | Morton << 16
+    uint64_t* pal_lab;  // scratch: the labels of the ops that do; the palette from its start on
+    const uint64_t* vol;  // the brick's first voxel
+    uint64_t WH;
+    uint32_t x_lim, y_lim, z_lim;  // voxels of the brick inside the volume
+    bool interior;
 };
 
 __device__ __forceinline__ uint64_t voxel(const BrickCtx& B, uint32_t x, uint32_t y, uint32_t z) {
-    uint64_t gx = B.x0 + x, gy = B.y0 + y, gz = B.z0 + z;
-    const EncArgs& A = *B.A;
-    if (gx < A.W && gy < A.H && gz < A.D) return __ldg(A.vol + gx + A.W * (gy + A.H * gz));
+    if (B.interior || (x < B.x_lim && y < B.y_lim && z < B.z_lim))
+        return __ldg(B.vol + (x + B.A->W * y + B.WH * z));
     return 0;  // padding, brick.hpp:181-183
 }
-__device__ __forceinline__ uint64_t node_label(const BrickCtx& B, uint32_t l, uint32_t m) {
-    if (l == B.A->L - 1) return voxel(B, demorton_axis(m), demorton_axis(m >> 1), demorton_axis(m >> 2));
-    if (l < kEncSmemLevels) return B.S->lab[((1u << (3 * l)) - 1) / 7 + m];
-    return B.lab_g[m];
-}
-__device__ __forceinline__ bool node_const(const BrickCtx& B, uint32_t l, uint32_t m) {
-    if (l == B.A->L - 1) return true;  // leaves are constant (brick.hpp:188)
-    if (l < kEncSmemLevels) return B.S->cst[((1u << (3 * l)) - 1) / 7 + m] != 0;
-    return B.cst_g[m] != 0;
+// The eight voxels of node (x, y, z) of the level above the leaves; as 16-byte pairs
+// along x when the volume's rows hold them aligned.
+__device__ __forceinline__ void voxels8(const BrickCtx& B, uint32_t x, uint32_t y, uint32_t z, uint64_t v[8]) {
+    if (B.interior && B.A->pairs) {
+        const uint64_t* p = B.vol + (2 * x + B.A->W * (2 * y) + B.WH * (2 * z));
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const ulonglong2 t =
+                __ldg(reinterpret_cast<const ulonglong2*>(p + ((r & 1) ? B.A->W : 0) + ((r & 2) ? B.WH : 0)));
+            v[2 * r] = t.x;
+            v[2 * r + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[c] = voxel(B, 2 * x + (c & 1), 2 * y + ((c >> 1) & 1), 2 * z + (c >> 2));
+    }
 }
 
 // Decoder-transparent encoding modes.  Where several ops reproduce a child's
@@ -192,289 +249,577 @@ __device__ __forceinline__ bool node_const(const BrickCtx& B, uint32_t l, uint32
 // mode % 6 picks the order of the three neighbour axes, and modes >= 6 try the
 // neighbours before the parent.  The decoder replays any of them unchanged;
 // mode 0 is the reference's order.
-__constant__ uint8_t kAxisOrder[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
-
-// Rp / Rx / Ry / Rz for child n on level lc (bestOperation, brickEncoding.hpp:198-282),
-// or OP_PALNEED when only a palette op can express it.
-__device__ __forceinline__ uint32_t choose_reuse(const BrickCtx& B, uint32_t lc, uint32_t n, uint64_t Lc,
-                                                 uint64_t parent, uint32_t mode) {
-    const bool nfirst = mode >= 6;
-    if (!nfirst && parent == Lc) return OP_RP;
-    const uint32_t ord = nfirst ? mode - 6 : mode;
-    const uint32_t lvlmask = (1u << (3 * lc)) - 1u;
-#pragma unroll
-    for (uint32_t k = 0; k < 3; ++k) {
-        const uint32_t a = kAxisOrder[ord][k];
-        const uint32_t m = (0x09249249u << a) & lvlmask, bit = 1u << a;
-        if (n & bit) {  // +1 side: later in Morton order -> the neighbour's parent (:265-272)
-            if ((n & m) == m) continue;
-            uint32_t N = (((n | ~m) + bit) & m) | (n & ~m);
-            if (node_label(B, lc - 1, N >> 3) == Lc) return OP_RX + a;
-        } else {  // -1 side: earlier in Morton order -> the neighbour itself (:256-261)
-            if ((n & m) == 0) continue;
-            uint32_t N = (((n & m) - bit) & m) | (n & ~m);
-            if (node_label(B, lc, N) == Lc) return OP_RX + a;
+// mode_codes(m): the op code for each set of matches (bit 0 the parent, bits 1..3 the
+// neighbours along x, y, z), 3 bits per set; none: a palette op.
+__host__ __device__ constexpr uint64_t mode_codes(uint32_t mode) {
+    const uint32_t order[6] = {012, 021, 0102, 0120, 0201, 0210};  // axes, first one on top (octal digits)
+    uint64_t t = 0;
+    for (uint32_t set = 0; set < 16; ++set) {
+        uint32_t code = OP_PALNEED;
+        for (uint32_t k = 0; k < 3 && code == OP_PALNEED; ++k) {
+            const uint32_t a = (order[mode % 6] >> (3 * (2 - k))) & 7u;
+            if ((set >> (a + 1)) & 1u) code = OP_RX + a;
         }
+        if ((set & 1u) && (mode < 6 || code == OP_PALNEED)) code = OP_RP;
+        t |= (uint64_t)code << (3 * set);
     }
-    if (nfirst && parent == Lc) return OP_RP;
-    return OP_PALNEED;
+    return t;
+}
+struct ModeTable {
+    uint64_t t[kModes];
+};
+constexpr ModeTable make_mode_table() {
+    ModeTable m{};
+    for (uint32_t k = 0; k < kModes; ++k) m.t[k] = mode_codes(k);
+    return m;
+}
+__constant__ ModeTable kModeTable = make_mode_table();
+
+// The block's scratch and shared memory.
+template <int T>
+__device__ __forceinline__ BrickCtx enc_ctx(const EncArgs& A, EncFixed& S, uint8_t* smem) {
+    uint8_t* scr = A.scratch + (uint64_t)blockIdx.x * A.scratch_per_cta;
+    const EncScratch X = enc_scratch<T>(A.L);
+    const uint32_t nw = (moff(A.L - 1) + 7) & ~7u;
+    BrickCtx B;
+    B.A = &A;
+    B.S = &S;
+    B.lab = reinterpret_cast<uint64_t*>(smem);
+    smem += (8 * enc_lab_nodes(A.L) + 15) & ~15u;
+    B.mask = reinterpret_cast<uint32_t*>(smem);
+    B.room = smem + 4 * nw;
+    B.lab_g = reinterpret_cast<uint64_t*>(scr + X.lab);
+    B.ops = scr + X.ops;
+    B.need8 = scr + X.need8;
+    B.act = reinterpret_cast<uint32_t*>(scr + X.act);
+    B.pal_lab = reinterpret_cast<uint64_t*>(scr + X.pal);
+    B.WH = A.W * A.H;
+    return B;
 }
 
-// Per-CTA scratch carved from the context's encoder scratch.
-struct EncScratch {
-    uint64_t* lab_g;  // level L-2 labels when that level does not fit in shared memory
-    uint8_t* cst_g;
-    uint8_t* ops;     // code | stop << 3 | delta << 4
-    uint64_t* pal_lab;
-    uint8_t* nib;
-    uint64_t* pal_out;
+// Brick i (split order: bx outer, bz inner, brick.hpp:152-154).
+__device__ __forceinline__ void enc_place(BrickCtx& B, uint32_t bx, uint32_t by, uint32_t bz) {
+    const EncArgs& A = *B.A;
+    const uint64_t x0 = (uint64_t)bx * A.b, y0 = (uint64_t)by * A.b, z0 = (uint64_t)bz * A.b;
+    B.vol = A.vol + (x0 + A.W * (y0 + A.H * z0));
+    B.x_lim = (uint32_t)min(A.W - x0, (uint64_t)A.b);
+    B.y_lim = (uint32_t)min(A.H - y0, (uint64_t)A.b);
+    B.z_lim = (uint32_t)min(A.D - z0, (uint64_t)A.b);
+    B.interior = B.x_lim == A.b && B.y_lim == A.b && B.z_lim == A.b;
+}
+
+// A warp's word of 32 Morton-consecutive nodes of a level: where lane's node is.
+struct WordAt {
+    uint32_t x, y, z;
+    __device__ __forceinline__ WordAt(uint32_t w) {
+        const uint32_t lane = threadIdx.x & 31u, m = 32 * w;
+        x = demorton_axis(m) | (lane & 1u) | ((lane >> 2) & 2u);
+        y = demorton_axis(m >> 1) | ((lane >> 1) & 1u) | ((lane >> 3) & 2u);
+        z = demorton_axis(m >> 2) | ((lane >> 2) & 1u);
+    }
+    __device__ __forceinline__ uint32_t raster(uint32_t l) const { return x | y << l | z << (2 * l); }
 };
 
-__device__ __forceinline__ EncScratch enc_scratch(const EncArgs& A) {
-    const uint64_t max_ops = ((1ull << (3 * A.L)) - 8) / 7;
-    uint8_t* scr = A.scratch + (uint64_t)blockIdx.x * A.scratch_per_cta;
-    auto align = [](uint64_t v) { return (v + 255) & ~255ull; };
-    const uint32_t n_g = A.L >= kEncSmemLevels + 2 ? (1u << (3 * (A.L - 2))) : 0;  // level L-2 when it is big
-    EncScratch X;
-    uint64_t o = 0;
-    X.lab_g = reinterpret_cast<uint64_t*>(scr + o);
-    o = align(o + 8ull * n_g);
-    X.cst_g = scr + o;
-    o = align(o + n_g);
-    X.ops = scr + o;
-    o = align(o + max_ops);
-    X.pal_lab = reinterpret_cast<uint64_t*>(scr + o);
-    o = align(o + 8 * max_ops);
-    X.nib = scr + o;
-    o = align(o + 2 * max_ops + 2);
-    X.pal_out = reinterpret_cast<uint64_t*>(scr + o);
-    return X;
-}
-
-// The majority pyramid of one brick (Brick::build, brick.hpp:78-123): level L-2
-// straight from the voxels (x fastest for coalescing), then the coarser levels.
-__device__ void build_pyramid(const BrickCtx& B) {
-    const EncArgs& A = *B.A;
-    EncShared& S = *B.S;
-    const uint32_t tid = threadIdx.x, T = blockDim.x, L = A.L;
-    {
-        const uint32_t s = A.b >> 1, cnt = s * s * s;
-        const uint32_t lvl = L - 2;
-        for (uint32_t k = tid; k < cnt; k += T) {
-            uint32_t x = k % s, y = (k / s) % s, z = k / (s * s);
-            uint64_t v[8];
+// Position of the k-th set bit of b (k below its number of set bits).
+__device__ __forceinline__ uint32_t nth_bit(uint32_t b, uint32_t k) {
+    uint32_t at = 0;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) v[c] = voxel(B, 2 * x + (c & 1), 2 * y + ((c >> 1) & 1), 2 * z + (c >> 2));
-            bool same;
-            uint64_t maj = majority8(v, same);
-            uint32_t m = morton3(x, y, z);
-            if (lvl < kEncSmemLevels) {
-                S.lab[((1u << (3 * lvl)) - 1) / 7 + m] = maj;
-                S.cst[((1u << (3 * lvl)) - 1) / 7 + m] = same;
-            } else {
-                B.lab_g[m] = maj;
-                B.cst_g[m] = same;
-            }
-        }
-        __syncthreads();
-    }
-    for (int l = (int)L - 3; l >= 0; --l) {  // buildLevel (brick.hpp:92-123)
-        const uint32_t cnt = 1u << (3 * l);
-        for (uint32_t m = tid; m < cnt; m += T) {
-            uint64_t v[8];
-            bool cc = true;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                v[c] = node_label(B, l + 1, 8 * m + c);
-                cc &= node_const(B, l + 1, 8 * m + c);
-            }
-            bool same;
-            uint64_t maj = majority8(v, same);
-            same &= cc;
-            S.lab[((1u << (3 * l)) - 1) / 7 + m] = maj;
-            S.cst[((1u << (3 * l)) - 1) / 7 + m] = same;
-        }
-        __syncthreads();
-    }
-}
-
-// Reuse ops, level by level in stream order (encodeBrick, :372-433); returns the
-// op count and the first op of every level in ls.
-__device__ uint32_t gen_reuse_ops(const BrickCtx& B, uint32_t mode, bool root_const, uint8_t* ops, uint64_t* pal_lab,
-                                  uint32_t ls[8]) {
-    const uint32_t tid = threadIdx.x, T = blockDim.x, L = B.A->L;
-    uint32_t base = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) ls[k] = 0;
-    if (!root_const) {
-        for (uint32_t l = 0; l + 1 < L; ++l) {
-            const uint32_t np = 1u << (3 * l), per = (np + T - 1) / T;
-            const uint32_t p0 = min(np, tid * per), p1 = min(np, p0 + per);
-            uint32_t cnt = 0;
-            for (uint32_t p = p0; p < p1; ++p) cnt += node_const(B, l, p) ? 0u : 1u;
-            uint32_t A_l;
-            uint32_t r = block_exclusive<uint32_t>(cnt, B.S->sh32, &A_l);
-            ls[l] = base;
-            for (uint32_t p = p0; p < p1; ++p) {
-                if (node_const(B, l, p)) continue;
-                const uint64_t plab = node_label(B, l, p);
-#pragma unroll 1
-                for (uint32_t c = 0; c < 8; ++c) {
-                    const uint32_t n = 8 * p + c, j = base + 8 * r + c;
-                    const uint64_t Lc = node_label(B, l + 1, n);
-                    const uint32_t code = choose_reuse(B, l + 1, n, Lc, plab, mode);
-                    ops[j] = (uint8_t)(code | (node_const(B, l + 1, n) ? 8u : 0u));
-                    if (code == OP_PALNEED) pal_lab[j] = Lc;
-                }
-                ++r;
-            }
-            base += 8 * A_l;
-            __syncthreads();
+    for (uint32_t h = 16; h; h >>= 1) {
+        const uint32_t low = __popc((b >> at) & ((1u << h) - 1u));
+        if (k >= low) {
+            k -= low;
+            at += h;
         }
     }
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-        if ((uint32_t)k >= L - 1) ls[k] = base;
-    return base;
+    return at;
 }
 
-// Palette ops: one warp walks the ops in stream order with a 17-entry window of
-// the most recent palette entries (reverse find only matters up to distance 16:
-// farther or absent means Pa).  Leaves the palette size in S.P.
-__device__ void palette_walk(const BrickCtx& B, uint64_t root, uint8_t* ops, const uint64_t* pal_lab, uint64_t* pal_out,
-                             uint32_t n_ops) {
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// The list of the active nodes (B.act) and S.level_r from the activity words; returns
+// their number.  A warp takes 32 words at a time and gives every lane one of their set
+// bits.  Every thread of the block calls it.
+template <int T>
+__device__ uint32_t list_active(const BrickCtx& B) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, L = B.A->L, FULL = 0xFFFFFFFFu;
+    const uint32_t nw = moff(L - 1), n_grp = (nw + 31) / 32;  // at most 37 groups of words
+    uint32_t* sum = B.S->hist;  // per group: active nodes, then those before it
+    for (uint32_t g = warp; g < n_grp; g += T / 32) {
+        const uint32_t w = 32 * g + lane;
+        const uint32_t n = __reduce_add_sync(FULL, w < nw ? __popc(B.mask[w]) : 0u);
+        if (lane == 0) sum[g] = n;
+    }
+    __syncthreads();
     if (warp == 0) {
-        uint64_t w = lane == 0 ? root : 0;
-        uint32_t P = 1;
-        if (lane == 0 && pal_out) pal_out[0] = root;
-        for (uint32_t j0 = 0; j0 < n_ops; j0 += 32) {
-            const uint32_t j = j0 + lane;
-            const uint32_t op = j < n_ops ? ops[j] : 0u;
-            const bool need = j < n_ops && (op & 7u) == OP_PALNEED;
-            uint32_t mask = __ballot_sync(0xffffffffu, need);
-            const uint64_t mine = need ? pal_lab[j] : 0ull;
-            while (mask) {
-                const int src = __ffs(mask) - 1;
-                mask &= mask - 1;
-                const uint64_t Lv = __shfl_sync(0xffffffffu, mine, src);
-                const uint32_t hit = __ballot_sync(0xffffffffu, lane < min(P, 17u) && w == Lv);
-                uint32_t code, delta = 0;
-                if (hit) {
-                    const int k = __ffs(hit) - 1;  // distance from the last entry
-                    code = k == 0 ? OP_P0 : OP_PD;
-                    delta = k == 0 ? 0u : (uint32_t)(k - 1);
-                } else {
-                    code = OP_PA;
-                    const uint64_t up = __shfl_up_sync(0xffffffffu, w, 1);
-                    w = lane == 0 ? Lv : up;
-                    if (lane == 0 && pal_out) pal_out[P] = Lv;
-                    ++P;
-                }
-                if (lane == src) ops[j] = (uint8_t)(code | (op & 8u) | (delta << 4));
+        const uint32_t a = 2 * lane < n_grp ? sum[2 * lane] : 0u, b = 2 * lane + 1 < n_grp ? sum[2 * lane + 1] : 0u;
+        uint32_t inc = a + b;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, inc, d);
+            if (lane >= (uint32_t)d) inc += y;
+        }
+        sum[2 * lane] = inc - a - b;
+        sum[2 * lane + 1] = inc - b;
+        if (lane == 31) B.S->n_act = inc;
+    }
+    __syncthreads();
+    for (uint32_t g = warp; g < n_grp; g += T / 32) {
+        const uint32_t w = 32 * g + lane, bits = w < nw ? B.mask[w] : 0u, cnt = __popc(bits);
+        uint32_t inc = cnt;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, inc, d);
+            if (lane >= (uint32_t)d) inc += y;
+        }
+        const uint32_t base = sum[g], total = __shfl_sync(FULL, inc, 31);
+        uint32_t l = 0;  // the word's level
+#pragma unroll
+        for (uint32_t k = 1; k < 6; ++k) l += w >= moff(k) ? 1u : 0u;
+        if (w < nw && w == moff(l)) B.S->level_r[l] = base + inc - cnt;
+        for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+            const uint32_t t = t0 + lane;
+            uint32_t j = 0;  // the lane whose word has the t-th node: as many as end at or before t
+#pragma unroll
+            for (uint32_t h = 16; h; h >>= 1)
+                if (__shfl_sync(FULL, inc, j + h - 1) <= t) j += h;
+            j = min(j, 31u);
+            const uint32_t wb = __shfl_sync(FULL, bits, j), before = __shfl_sync(FULL, inc - cnt, j),
+                           wl = __shfl_sync(FULL, l, j);
+            if (t < total) {
+                const uint32_t m = 32 * (32 * g + j - moff(wl)) + nth_bit(wb, t - before);
+                B.act[base + t] = demorton_axis(m) | demorton_axis(m >> 1) << wl | demorton_axis(m >> 2) << (2 * wl) |
+                                  m << 16;
             }
         }
-        if (lane == 0) B.S->P = P;
+    }
+    if (tid < 8 && tid >= L - 1) B.S->level_r[tid] = B.S->n_act;
+    __syncthreads();
+    return B.S->n_act;
+}
+
+// The majority pyramid of one brick (Brick::build, brick.hpp:78-123) and its active
+// nodes.  Returns their number.  Most nodes above the leaves hold one label, so a warp
+// first only tells which do (32 nodes in raster order at a time, so that it reads whole
+// rows of the brick: rows of 64 bytes, as 32 Morton-consecutive nodes have them, ran at
+// 0.7 of the rate); the others it queues, and takes the vote over 32 of them at once.
+template <int T>
+__device__ uint32_t build_pyramid(const BrickCtx& B) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, L = B.A->L, lb = L - 2;
+    const uint32_t sm = (1u << lb) - 1u, FULL = 0xFFFFFFFFu;
+    uint64_t* lab = lb < kEncSmemLevels ? B.lab + lvl_off(lb) : B.lab_g;
+    uint16_t* queue = reinterpret_cast<uint16_t*>(B.room) + 64 * warp;
+    for (uint32_t w = tid; w < mwords(lb); w += T) B.mask[moff(lb) + w] = 0;
+    __syncthreads();
+    uint32_t queued = 0;
+    auto vote = [&](uint32_t n) {  // of the first n queued
+        if (lane < n) {
+            const uint32_t p = queue[lane];
+            uint64_t v[8];
+            voxels8(B, p & sm, (p >> lb) & sm, p >> (2 * lb), v);
+            lab[p] = majority8_mixed(v);
+        }
+        __syncwarp();
+    };
+    for (uint32_t w = warp; w < mwords(lb); w += T / 32) {
+        const uint32_t p = 32 * w + lane;
+        bool active = false;
+        if (p < 1u << (3 * lb)) {
+            uint64_t v[8];
+            voxels8(B, p & sm, (p >> lb) & sm, p >> (2 * lb), v);
+            active = !uniform8(v);
+            if (!active) lab[p] = v[0];
+        }
+        const uint32_t bits = __ballot_sync(FULL, active);
+        if (!bits) continue;
+        // the activity bits in Morton order: four consecutive x of one (y, z) are bits 0, 1, 8, 9 from
+        // the row's place in their word on (levels of fewer nodes: the first of them)
+        const uint32_t four = (bits >> (4 * (lane & 7u))) & 15u;
+        if (lane < 8 && four) {
+            const uint32_t q = 32 * w + 4 * lane;
+            if (lb >= 2) {
+                const uint32_t m = morton3(q & sm, (q >> lb) & sm, q >> (2 * lb));
+                atomicOr(B.mask + moff(lb) + (m >> 5), ((four & 3u) | (four & 12u) << 6) << (m & 31u));
+            } else {  // at most 2 x 2 x 2 nodes: both orders are one
+                atomicOr(B.mask + moff(lb), four << (4 * lane));
+            }
+        }
+        if (active) queue[queued + __popc(bits & ((1u << lane) - 1u))] = (uint16_t)p;
+        queued += __popc(bits);
+        __syncwarp();
+        if (queued >= 32) {
+            vote(32);
+            queued -= 32;
+            if (lane < queued) queue[lane] = queue[32 + lane];
+            __syncwarp();
+        }
+    }
+    vote(queued);
+    __syncthreads();
+    for (int l = (int)lb - 1; l >= 0; --l) {  // buildLevel (brick.hpp:92-123)
+        const uint64_t* below = l + 1 < (int)kEncSmemLevels ? B.lab + lvl_off(l + 1) : B.lab_g;
+        for (uint32_t w = warp; w < mwords(l); w += T / 32) {
+            const uint32_t m = 32 * w + lane;
+            bool active = false;
+            if (m < 1u << (3 * l)) {
+                const uint32_t x = demorton_axis(m), y = demorton_axis(m >> 1), z = demorton_axis(m >> 2);
+                const uint32_t first = 2 * x | (2 * y) << (l + 1) | (2 * z) << (2 * l + 2);
+                uint64_t v[8];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {  // (one voxel's level is a single, so 8-byte aligned, label)
+                    const uint64_t* q = below + (first | (r & 1) << (l + 1) | (r >> 1) << (2 * l + 2));
+                    v[2 * r] = q[0];
+                    v[2 * r + 1] = q[1];
+                }
+                bool all;
+                B.lab[lvl_off(l) + (x | y << l | z << (2 * l))] = majority8(v, all);
+                // active when a child is, or when the children differ
+                active = !all || ((B.mask[moff(l + 1) + (m >> 2)] >> (8 * (m & 3u))) & 0xFFu) != 0;
+            }
+            const uint32_t bits = __ballot_sync(FULL, active);
+            if (lane == 0) B.mask[moff(l) + w] = bits;
+        }
+        __syncthreads();
+    }
+    return list_active<T>(B);
+}
+
+// The ops of the children of level l's active nodes (encodeBrick, brickEncoding.hpp:372-433):
+// the r-th active node's (levels in order, Morton order within a level) are ops 8r .. 8r +
+// 7.  A warp takes four active nodes at a time, a child per lane.  f(r, c, set, stop,
+// label): which of the parent (bit 0) and the neighbours outside the sibling block (bits
+// 1 .. 3) have the child's label (bestOperation, :198-282; all of them when `every`, else
+// the neighbours only where the parent has not), for every lane of the warp (stop: 2
+// where the lane has no child).  PG, CG: the level's own labels and its children's are
+// level 5's, in scratch; LEAF: the children are voxels.
+template <int T, bool PG, bool CG, bool LEAF, class F>
+__device__ __forceinline__ void level_children(const BrickCtx& B, uint32_t l, bool every, F& f) {
+    const uint32_t lane = threadIdx.x & 31, c = lane & 7u, g = lane >> 3, lc = l + 1, sm = (1u << l) - 1u;
+    const uint32_t r0 = B.S->level_r[l], n = B.S->level_r[l + 1] - r0;
+    const uint32_t* act = B.act + r0;
+    const uint64_t* lab_p = PG ? B.lab_g : B.lab + lvl_off(l);
+    const uint64_t* lab_c = CG ? B.lab_g : B.lab + lvl_off(lc);  // (not used for leaves)
+    const uint64_t W = B.A->W;
+    auto child = [&](uint32_t p, uint32_t& x, uint32_t& y, uint32_t& z) {
+        x = 2 * (p & sm) | (c & 1u);
+        y = 2 * ((p >> l) & sm) | ((c >> 1) & 1u);
+        z = 2 * (p >> (2 * l)) | (c >> 2);
+    };
+    // the nodes two steps ahead and the labels one step ahead are on their way
+    uint32_t k = 4 * (threadIdx.x >> 5) + g;
+    auto load_e = [&](uint32_t i) { return i < n ? act[i] : 0u; };
+    auto load_labels = [&](uint32_t i, uint32_t e, uint64_t& parent, uint64_t& label) {
+        parent = label = 0;
+        if (i >= n) return;
+        const uint32_t p = e & 0xFFFFu;
+        uint32_t x, y, z;
+        child(p, x, y, z);
+        parent = lab_p[p];
+        if (!LEAF) label = lab_c[x | y << lc | z << (2 * lc)];
+        else if (B.interior || (x < B.x_lim && y < B.y_lim && z < B.z_lim)) label = __ldg(B.vol + (x + W * y + B.WH * z));
+    };
+    uint32_t e_next = load_e(k), e_after = load_e(k + T / 8);
+    uint64_t parent_next, label_next;
+    load_labels(k, e_next, parent_next, label_next);
+    for (uint32_t q = k - g; q < n; q += T / 8, k += T / 8) {
+        const uint32_t e = e_next;
+        const uint64_t parent = parent_next, label = label_next;
+        e_next = e_after;
+        e_after = load_e(k + T / 4);
+        load_labels(k + T / 8, e_next, parent_next, label_next);
+        uint32_t set = 0, stop = 2;
+        if (k < n) {
+            const uint32_t p = e & 0xFFFFu, m = e >> 16;
+            stop = LEAF ? 1u  // leaves are constant (brick.hpp:188)
+                        : ((B.mask[moff(lc) + (m >> 2)] >> (8 * (m & 3u) + c)) & 1u ? 0u : 1u);
+            set = parent == label ? 1u : 0u;
+            if (every || !set) {
+                uint32_t x, y, z;
+                child(p, x, y, z);
+                uint64_t nb[3];
+                bool has[3];
+#pragma unroll
+                for (uint32_t a = 0; a < 3; ++a) {
+                    const uint32_t at = (a == 0 ? x : (a == 1 ? y : z)) >> 1;
+                    const bool up = (c >> a) & 1u;
+                    has[a] = up ? at < sm : at > 0;
+                    nb[a] = 0;
+                    if (!has[a]) continue;
+                    if (up) {  // +1 side: later in Morton order -> the neighbour's parent (:265-272)
+                        nb[a] = lab_p[p + (1u << (a * l))];
+                    } else if (!LEAF) {  // -1 side: earlier in Morton order -> the neighbour itself (:256-261)
+                        nb[a] = lab_c[(x | y << lc | z << (2 * lc)) - (1u << (a * lc))];
+                    } else {
+                        nb[a] = voxel(B, x - (a == 0), y - (a == 1), z - (a == 2));
+                    }
+                }
+#pragma unroll
+                for (uint32_t a = 0; a < 3; ++a) set |= (has[a] && nb[a] == label ? 2u : 0u) << a;
+            }
+        }
+        f(r0 + k, c, set, stop, label);
+    }
+}
+template <int T, class F>
+__device__ __forceinline__ void for_children(const BrickCtx& B, bool every, F f) {
+    const uint32_t lb = B.A->L - 2;
+    // the many first
+    if (lb < kEncSmemLevels) level_children<T, false, false, true>(B, lb, every, f);
+    else level_children<T, true, false, true>(B, lb, every, f);
+    for (int l = (int)lb - 1; l >= 0; --l) {
+        if (l + 1 < (int)kEncSmemLevels) level_children<T, false, false, false>(B, l, every, f);
+        else level_children<T, false, true, false>(B, l, every, f);
+    }
+}
+
+// Palette ops: the ops that need one are listed in stream order (8 or 16 active nodes
+// per thread at a time), then the first warp takes them, 32 at a time, with a 17-entry
+// window of the most recent palette entries (reverse find only matters up to distance 16:
+// farther or absent means Pa).  The entries of a window differ, and only a miss changes
+// it (the missed label enters at distance 0, the others move one on), so all 32 look
+// their labels up at once and what is left to do in order is one step per miss.  put(j,
+// code, delta) for every such op; the palette after the root's label goes to the start of
+// pal_lab (an entry's place is never past that of an op still to come), its size to S.P
+// and the number of Pd ops to S.n_pd.
+template <int T, class F>
+__device__ void palette_walk(const BrickCtx& B, uint64_t root, uint32_t n_act, F put) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, FULL = 0xFFFFFFFFu;
+    uint16_t* list = reinterpret_cast<uint16_t*>(B.act);  // (the active nodes' list is done with)
+    uint64_t win = lane == 0 ? root : 0;
+    uint32_t P = 1, n_pd = 0;
+    constexpr uint32_t kPer = kWalkParents<T> / T;  // nodes per thread, 16 or 8
+    static_assert(kPer * T == kWalkParents<T> && kPer % 4 == 0, "whole words of nodes per thread");
+    for (uint32_t r0 = 0; r0 < n_act; r0 += kWalkParents<T>) {
+        const uint32_t r = r0 + kPer * tid;
+        uint32_t words[kPer / 4], cnt = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kPer / 4; ++q) {
+            const uint32_t at = r + 4 * q;  // bytes below n_act
+            words[q] = at < n_act ? *reinterpret_cast<const uint32_t*>(B.need8 + at) : 0u;
+            if (at < n_act && at + 4 > n_act) words[q] &= (1u << (8 * (n_act - at))) - 1u;
+            cnt += __popc(words[q]);
+        }
+        uint32_t total;
+        uint32_t at = block_exclusive<uint32_t>(cnt, B.S->sh32, &total);
+#pragma unroll
+        for (uint32_t q = 0; q < kPer / 4; ++q)
+            for (uint32_t m = words[q]; m; m &= m - 1)
+                list[at++] = (uint16_t)(8 * kPer * tid + 32 * q + __ffs(m) - 1);
+        __syncthreads();
+        if (tid < 32 && total) {
+            uint32_t j_next = lane < total ? 8 * r0 + list[lane] : 0u;
+            uint64_t label_next = lane < total ? B.pal_lab[j_next] : 0ull;
+            for (uint32_t k0 = 0; k0 < total; k0 += 32) {
+                const bool valid = k0 + lane < total;
+                const uint32_t j = j_next;
+                const uint64_t mine = label_next;
+                if (k0 + 32 + lane < total) {
+                    j_next = 8 * r0 + list[k0 + 32 + lane];
+                    label_next = B.pal_lab[j_next];
+                }
+                int d = -1;  // distance from the last entry
+                const uint32_t depth = min(P, 17u);
+                for (uint32_t k = 0; k < depth; ++k)
+                    if (__shfl_sync(FULL, win, k) == mine) d = (int)k;
+                bool added = false;
+                for (uint32_t miss = __ballot_sync(FULL, valid && d < 0); miss;) {
+                    const uint32_t f = __ffs(miss) - 1;
+                    const uint64_t entry = __shfl_sync(FULL, mine, f), up = __shfl_up_sync(FULL, win, 1);
+                    win = lane == 0 ? entry : up;
+                    if (lane == 0) B.pal_lab[P - 1] = entry;
+                    ++P;
+                    if (lane == f) added = true;
+                    if (lane > f) d = mine == entry ? 0 : (d >= 0 && d < 16 ? d + 1 : -1);
+                    miss = __ballot_sync(FULL, valid && lane > f && d < 0);
+                }
+                const bool pd = valid && !added && d > 0;
+                if (valid) put(j, added ? OP_PA : (d == 0 ? OP_P0 : OP_PD), pd ? (uint32_t)d - 1 : 0u);
+                n_pd += __popc(__ballot_sync(FULL, pd));
+            }
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        B.S->P = P;
+        B.S->n_pd = n_pd;
     }
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kEncThreads, 2) enc_bricks_kernel(EncArgs A) {
-    __shared__ EncShared S;
-    const uint32_t tid = threadIdx.x, T = blockDim.x;
-    const EncScratch X = enc_scratch(A);
-    uint8_t* ops = X.ops;
-    uint8_t* nib = X.nib;
-    uint64_t* pal_out = X.pal_out;
+// Per byte of v whose op code is `code`: bit 0.
+__device__ __forceinline__ uint32_t bytes_with(uint32_t v, uint32_t code) {
+    const uint32_t x = (v & 0x07070707u) ^ (code * 0x01010101u);
+    return ~(x | (x >> 1) | (x >> 2)) & 0x01010101u;
+}
+// Four op bytes as nibbles (op << 1 | stop, brickEncoding.cpp:66-67), the first lowest.
+__device__ __forceinline__ uint32_t nibbles4(uint32_t v) {
+    uint32_t n = ((v & 0x07070707u) << 1) | ((v >> 3) & 0x01010101u);
+    n = (n | (n >> 4)) & 0x00FF00FFu;
+    return (n | (n >> 8)) & 0xFFFFu;
+}
 
+// Bound by the volume's reads and their latency: the pyramid streams it (about two thirds
+// of the HBM rate while every brick does so), the children's second look at the voxels of
+// active nodes comes in pieces of 16 bytes.  Measured (B200) against a thread per run of
+// nodes at every step and a palette walk over every op (two CTAs of 512 threads per SM):
+// 512 bricks of 64^3 4.05 -> 0.76 ms (0.16 ms at the HBM rate), 8192 bricks of 32^3 3.33 ->
+// 0.66 ms (0.32 ms), 60 bricks of 32^3 0.184 -> 0.054 ms.
+template <int T, int PER_SM>
+__global__ void __launch_bounds__(T, PER_SM) enc_bricks_kernel(EncArgs A) {
+    extern __shared__ __align__(16) uint8_t enc_dyn[];
+    __shared__ EncFixed S;
+    const uint32_t tid = threadIdx.x;
+    BrickCtx B = enc_ctx<T>(A, S, enc_dyn);
     for (;;) {
         if (tid == 0) S.work = atomicAdd(reinterpret_cast<unsigned int*>(A.misc + kMiscQueue), 1u);
-        if (tid < 16) S.hist[tid] = 0;
         __syncthreads();
         const uint32_t i = S.work;
         if (i >= A.nb) break;
-        // split order: bx outer, bz inner (brick.hpp:152-154)
         const uint32_t bz = i % A.nbz, by = (i / A.nbz) % A.nby, bx = i / (A.nbz * A.nby);
-        BrickCtx B{&A, &S, (uint64_t)bx * A.b, (uint64_t)by * A.b, (uint64_t)bz * A.b, X.lab_g, X.cst_g};
-        const uint32_t sel = A.sel ? A.sel[i] : 0u;
-        build_pyramid(B);
-        const uint64_t root = node_label(B, 0, 0);
-        const bool root_const = node_const(B, 0, 0);
-        uint32_t ls[8];
-        const uint32_t n_ops = gen_reuse_ops(B, sel & 15u, root_const, ops, X.pal_lab, ls);
-        palette_walk(B, root, ops, X.pal_lab, pal_out, n_ops);
-        const uint32_t P = S.P;
+        enc_place(B, bx, by, bz);
+        const uint32_t sel = A.sel ? A.sel[i] : 0u, mode = min(sel & 15u, kModes - 1);
+        const uint32_t n_act = build_pyramid<T>(B), n_ops = 8 * n_act;
+        const uint64_t root = B.lab[0], codes = kModeTable.t[mode];
+        for_children<T>(B, mode >= 6, [&](uint32_t r, uint32_t c, uint32_t set, uint32_t stop, uint64_t label) {
+            const uint32_t code = (uint32_t)(codes >> (3 * set)) & 7u;
+            const bool need = stop < 2 && code == OP_PALNEED;
+            const uint32_t needs = __ballot_sync(0xFFFFFFFFu, need);
+            if (stop < 2) {
+                B.ops[8 * r + c] = (uint8_t)(code | stop << 3);
+                if (need) B.pal_lab[8 * r + c] = label;
+                if (c == 0) B.need8[r] = (uint8_t)(needs >> (threadIdx.x & 24u));
+            }
+        });
+        __syncthreads();
+        palette_walk<T>(B, root, n_act, [&](uint32_t j, uint32_t code, uint32_t delta) {
+            B.ops[j] = (uint8_t)(code | (B.ops[j] & 8u) | delta << 4);
+        });
 
         // ---- nibble layout (packOperationsToNibbles) and seek checkpoints
-        {
-            const uint32_t per = (n_ops + T - 1) / T;
-            const uint32_t j0 = min(n_ops, tid * per), j1 = min(n_ops, j0 + per);
-            uint32_t nc = 0, pa = 0;
-            for (uint32_t j = j0; j < j1; ++j) {
-                uint32_t c = ops[j] & 7u;
-                nc += c == OP_PD ? 2u : 1u;
-                pa += c == OP_PA ? 1u : 0u;
-            }
-            // the brick's seek checkpoints (one per S ops) are reserved in the pool
-            const uint32_t n_ck = (n_ops + A.S - 1) / A.S;
-            if (tid == 0) S.ck_off = atomicAdd(A.misc + kMiscCk, (unsigned long long)n_ck);
-            uint32_t NC, PA;
-            uint32_t pos = 1 + block_exclusive<uint32_t>(nc, S.sh32, &NC);
-            uint32_t ip = block_exclusive<uint32_t>(pa, S.sh32, &PA);
-            __syncthreads();
-            const uint64_t ck_off = S.ck_off;
-            const bool ck_ok = ck_off + n_ck <= A.ck_cap;
-            Checkpoint* ck = A.ck + ck_off;
-            for (uint32_t j = j0; j < j1; ++j) {
-                const uint32_t op = ops[j], c = op & 7u;
-                if (j % A.S == 0 && ck_ok) ck[j / A.S] = Checkpoint{0, 0, pos, ip};
-                nib[pos++] = (uint8_t)((c << 1) | ((op >> 3) & 1u));
-                if (c == OP_PD) nib[pos++] = (uint8_t)(op >> 4);
-                if (c == OP_PA) ++ip;
-            }
-            if (tid == 0) nib[0] = (uint8_t)((OP_PA << 1) | (root_const ? 1u : 0u));
-            const uint32_t nsym = 1 + NC;
-            const uint32_t nbytes = (nsym + 1) / 2;
-            if (tid == 0) {
-                S.nib_off = atomicAdd(A.misc + 0, (unsigned long long)((nbytes + 15) & ~15u));
-                S.pal_off = atomicAdd(A.misc + 1, (unsigned long long)P);
-            }
-            __syncthreads();
-            const uint64_t nib_off = S.nib_off, pal_off = S.pal_off;
-            // the rANS kernel reads whole 16-byte chunks of the reservation
-            const bool ok = nib_off + ((nbytes + 15) & ~15u) <= A.nib_cap && pal_off + P <= A.pal_cap && ck_ok;
-            const bool sample = ((A.index_base + i) % 512) == 0;  // brickEncoding.hpp:482
-            for (uint32_t q = tid; q < nbytes; q += T) {
-                const uint32_t hi = nib[2 * q], lo = (2 * q + 1 < nsym) ? nib[2 * q + 1] : 0u;
-                if (ok) A.nib_pool[nib_off + q] = (uint8_t)((hi << 4) | lo);
-                if (sample) {  // every nibble of the packed bytes, pad included (brickEncoding.cpp:131-143)
-                    atomicAdd(&S.hist[hi], 1u);
-                    atomicAdd(&S.hist[lo], 1u);
+        const uint32_t P = S.P, nsym = 1 + n_ops + S.n_pd, nbytes = (nsym + 1) / 2;
+        static_assert(kOpsPerCheckpoint == 16, "a thread's 16 ops start at a checkpoint");
+        const uint32_t n_ck = (n_ops + 15) / 16;
+        if (tid == 0) {
+            S.ck_off = atomicAdd(A.misc + kMiscCk, (unsigned long long)n_ck);
+            S.nib_off = atomicAdd(A.misc + 0, (unsigned long long)((nbytes + 15) & ~15u));
+            S.pal_off = atomicAdd(A.misc + 1, (unsigned long long)P);
+        }
+        if (tid < 16) S.hist[tid] = 0;
+        // staging: packed nibbles from position `base` (a multiple of 32) on, nibble k at bit 4 k
+        uint32_t* stage = reinterpret_cast<uint32_t*>(B.room);
+        for (uint32_t k = tid; k < T * 4 + 8; k += T) stage[k] = 0;
+        __syncthreads();
+        const uint64_t nib_off = S.nib_off, pal_off = S.pal_off, ck_off = S.ck_off;
+        const bool ck_ok = ck_off + n_ck <= A.ck_cap;
+        // the rANS kernel reads whole 16-byte chunks of the reservation
+        const bool ok = nib_off + ((nbytes + 15) & ~15u) <= A.nib_cap && pal_off + P <= A.pal_cap && ck_ok;
+        const bool root_const = n_act == 0;
+        const bool sample = ((A.index_base + i) % 512) == 0;  // brickEncoding.hpp:482
+        Checkpoint* ck = A.ck + ck_off;
+        uint4* nib = reinterpret_cast<uint4*>(A.nib_pool + nib_off);
+        if (tid == 0) stage[0] = (OP_PA << 1) | (root_const ? 1u : 0u);
+        uint32_t base = 0, pos = 1, pa = 0;  // the first position staged, the next one's, Pa ops before it
+        // 16-byte chunk q of the staging, as the pool holds it (a byte's high nibble is the earlier one)
+        auto chunk_out = [&](uint32_t q) {
+            uint4 v = reinterpret_cast<const uint4*>(stage)[q];
+            if (sample) {  // every nibble of the packed bytes, pad included (brickEncoding.cpp:131-143)
+                uint64_t c[2] = {0, 0};
+                const uint32_t words[4] = {v.x, v.y, v.z, v.w}, first = base + 32 * q;
+#pragma unroll
+                for (uint32_t k = 0; k < 32; ++k) {
+                    const uint32_t s = (words[k >> 3] >> (4 * (k & 7u))) & 15u;
+                    if (first + k < 2 * nbytes) (s & 8u ? c[1] : c[0]) += 1ull << (8 * (s & 7u));
+                }
+#pragma unroll
+                for (uint32_t s = 0; s < 16; ++s) {
+                    const uint32_t n = (uint32_t)(c[s >> 3] >> (8 * (s & 7u))) & 0xFFu;
+                    if (n) atomicAdd(&S.hist[s], n);
                 }
             }
-            if (ok)
-                for (uint32_t k = tid; k < P; k += T) A.pal_pool[pal_off + k] = pal_out[k];
-            __syncthreads();
-            if (sample && tid < 16 && S.hist[tid]) atomicAdd(A.misc + 2 + tid, (unsigned long long)S.hist[tid]);
-            if (tid == 0) {
-                EncMeta m;
-                m.nib_off = nib_off;
-                m.pal_off = pal_off;
-                m.enc_off = 0;
-                m.P = P;
-                m.nsym = nsym;
-                m.nbytes = nbytes;
-                m.n_ops = n_ops;
-                m.id = morton3(bx + A.bx0, by, bz);
-                m.flags = (root_const ? EF_UNIFORM : 0u) | (ok ? 0u : EF_OVERFLOW);
-                m.n_ck = n_ck;
-                m.E = 0;
-                m.sel = sel;
-                m.ck_off = ck_ok ? (uint32_t)ck_off : 0u;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) m.level_start[k] = ls[k];
-                A.meta[i] = m;
+            auto swap = [](uint32_t x) { return ((x & 0x0F0F0F0Fu) << 4) | ((x >> 4) & 0x0F0F0F0Fu); };
+            if (ok) nib[base / 32 + q] = make_uint4(swap(v.x), swap(v.y), swap(v.z), swap(v.w));
+        };
+        for (uint32_t j0 = 0; j0 < n_ops; j0 += 16 * T) {
+            const uint32_t j = j0 + 16 * tid;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            uint32_t nv = 0;  // 16, or 8 at the end
+            if (j < n_ops) {
+                v = *reinterpret_cast<const uint4*>(B.ops + j);
+                nv = min(16u, n_ops - j);
+                if (nv == 8) v.z = v.w = 0;
             }
+            const uint32_t d0 = bytes_with(v.x, OP_PD), d1 = bytes_with(v.y, OP_PD), d2 = bytes_with(v.z, OP_PD),
+                           d3 = bytes_with(v.w, OP_PD);
+            const uint32_t n_d = __popc(d0 | d1 << 1 | d2 << 2 | d3 << 3);
+            const uint32_t n_a = __popc(bytes_with(v.x, OP_PA) | bytes_with(v.y, OP_PA) << 1 |
+                                        bytes_with(v.z, OP_PA) << 2 | bytes_with(v.w, OP_PA) << 3);
+            uint32_t total;
+            const uint32_t before = block_exclusive<uint32_t>((nv + n_d) | n_a << 16, S.sh32, &total);
+            const uint32_t at = pos + (before & 0xFFFFu);
+            if (nv && ck_ok) ck[j >> 4] = Checkpoint{0, 0, at, pa + (before >> 16)};
+            // the ops' nibbles into the staged words (neighbours share a word)
+            uint32_t s = at - base;
+            auto put = [&](uint64_t n) {  // up to 16 nibbles at s, zero above the last one
+                const uint32_t sh = 4 * (s & 7u), k = s >> 3;
+                const uint32_t lo = (uint32_t)n, hi = (uint32_t)(n >> 32);
+                if (lo << sh) atomicOr(stage + k, lo << sh);
+                const uint32_t mid = __funnelshift_l(lo, hi, sh), top = __funnelshift_l(hi, 0u, sh);
+                if (mid) atomicOr(stage + k + 1, mid);
+                if (top) atomicOr(stage + k + 2, top);
+            };
+            if (n_d == 0) {
+                put((uint64_t)(nibbles4(v.x) | nibbles4(v.y) << 16) |
+                    (uint64_t)(nv > 8 ? nibbles4(v.z) | nibbles4(v.w) << 16 : 0u) << 32);
+            } else {
+                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) {
+                    uint64_t n = 0;
+                    uint32_t len = 0;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) {
+                        const uint32_t op = (words[q] >> (8 * k)) & 0xFFu, c = op & 7u;
+                        if (4 * q + k < nv) {
+                            n |= (uint64_t)((c << 1) | ((op >> 3) & 1u)) << (4 * len++);
+                            if (c == OP_PD) n |= (uint64_t)(op >> 4) << (4 * len++);
+                        }
+                    }
+                    put(n);
+                    s += len;
+                }
+            }
+            __syncthreads();
+            pos += total & 0xFFFFu;
+            pa += total >> 16;
+            // whole chunks leave; what is left of the last one moves to the front
+            const uint32_t full = (pos - base) / 32;
+            for (uint32_t q = tid; q < full; q += T) chunk_out(q);
+            const uint32_t rest = tid < 4 ? stage[4 * full + tid] : 0u;
+            __syncthreads();
+            for (uint32_t k = tid; k < 4 * full + 4; k += T) stage[k] = k < 4 ? rest : 0u;
+            base += 32 * full;
+        }
+        __syncthreads();
+        if (tid == 0 && pos > base) chunk_out(0);
+        if (ok)
+            for (uint32_t k = tid; k < P; k += T) A.pal_pool[pal_off + k] = k ? B.pal_lab[k - 1] : root;
+        __syncthreads();
+        if (sample && tid < 16 && S.hist[tid]) atomicAdd(A.misc + 2 + tid, (unsigned long long)S.hist[tid]);
+        if (tid == 0) {
+            EncMeta m;
+            m.nib_off = nib_off;
+            m.pal_off = pal_off;
+            m.enc_off = 0;
+            m.P = P;
+            m.nsym = nsym;
+            m.nbytes = nbytes;
+            m.n_ops = n_ops;
+            m.id = morton3(bx + A.bx0, by, bz);
+            m.flags = (root_const ? EF_UNIFORM : 0u) | (ok ? 0u : EF_OVERFLOW);
+            m.n_ck = n_ck;
+            m.E = 0;
+            m.sel = sel;
+            m.ck_off = ck_ok ? (uint32_t)ck_off : 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) m.level_start[k] = k + 1 < A.L ? 8u * S.level_r[k] : n_ops;
+            A.meta[i] = m;
         }
         __syncthreads();
     }
@@ -482,43 +827,69 @@ __global__ void __launch_bounds__(kEncThreads, 2) enc_bricks_kernel(EncArgs A) {
 
 // Exhaustive statistics for the mode / table choice: per brick and mode, the
 // histogram of the 16 nibble values the rANS coder would see (root nibble, op
-// nibbles, Pd offsets and the pad nibble of an odd count).
-__global__ void __launch_bounds__(kEncThreads, 2) enc_stats_kernel(EncArgs A, uint32_t* __restrict__ hist_out) {
-    __shared__ EncShared S;
-    const uint32_t tid = threadIdx.x, T = blockDim.x;
-    const EncScratch X = enc_scratch(A);
+// nibbles, Pd offsets and the pad nibble of an odd count).  A mode only changes which
+// of several matches an op names: the ops that match nothing, and so the palette, are
+// every mode's, and a mode's other nibbles follow from how often each set of matches
+// occurs.  So one pass over the children counts the sets (32 with the stop bit, one lane
+// each, by ballots) for all modes: 150 bricks of 64^3 19.4 -> 0.25 ms against an op stream
+// and a walk per mode.
+template <int T, int PER_SM>
+__global__ void __launch_bounds__(T, PER_SM) enc_stats_kernel(EncArgs A, uint32_t* __restrict__ hist_out) {
+    extern __shared__ __align__(16) uint8_t enc_dyn[];
+    __shared__ EncFixed S;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, FULL = 0xFFFFFFFFu;
+    BrickCtx B = enc_ctx<T>(A, S, enc_dyn);
+    uint32_t* sets = S.hist + 16;  // [set << 1 | stop]
     for (;;) {
         if (tid == 0) S.work = atomicAdd(reinterpret_cast<unsigned int*>(A.misc + kMiscQueue), 1u);
         __syncthreads();
         const uint32_t i = S.work;
         if (i >= A.nb) break;
-        const uint32_t bz = i % A.nbz, by = (i / A.nbz) % A.nby, bx = i / (A.nbz * A.nby);
-        BrickCtx B{&A, &S, (uint64_t)bx * A.b, (uint64_t)by * A.b, (uint64_t)bz * A.b, X.lab_g, X.cst_g};
-        build_pyramid(B);
-        const uint64_t root = node_label(B, 0, 0);
-        const bool root_const = node_const(B, 0, 0);
-        for (uint32_t mode = 0; mode < kModes; ++mode) {
-            if (tid < 16) S.hist[tid] = 0;
-            uint32_t ls[8];
-            const uint32_t n_ops = gen_reuse_ops(B, mode, root_const, X.ops, X.pal_lab, ls);
-            palette_walk(B, root, X.ops, X.pal_lab, nullptr, n_ops);
-            uint32_t nc = 0;
-            for (uint32_t j = tid; j < n_ops; j += T) {
-                const uint32_t op = X.ops[j], c = op & 7u;
-                atomicAdd(&S.hist[(c << 1) | ((op >> 3) & 1u)], 1u);
-                if (c == OP_PD) atomicAdd(&S.hist[op >> 4], 1u);
-                nc += c == OP_PD ? 2u : 1u;
+        enc_place(B, i / (A.nbz * A.nby), (i / A.nbz) % A.nby, i % A.nbz);
+        const uint32_t n_act = build_pyramid<T>(B), n_ops = 8 * n_act;
+        if (tid < 64) S.hist[tid] = 0;
+        __syncthreads();
+        const uint64_t root = B.lab[0];
+        uint32_t count = 0;  // of the set and stop bit numbered as this lane
+        for_children<T>(B, true, [&](uint32_t r, uint32_t c, uint32_t set, uint32_t stop, uint64_t label) {
+            const uint32_t key = set << 1 | (stop & 1u);
+            uint32_t m = __ballot_sync(FULL, stop < 2);
+#pragma unroll
+            for (uint32_t k = 0; k < 5; ++k) {
+                const uint32_t b = __ballot_sync(FULL, (key >> k) & 1u);
+                m &= (lane >> k) & 1u ? b : ~b;
             }
-            uint32_t NC;
-            block_exclusive<uint32_t>(nc, S.sh32, &NC);
-            if (tid == 0) {
-                atomicAdd(&S.hist[(OP_PA << 1) | (root_const ? 1u : 0u)], 1u);  // root nibble
-                if (((1 + NC) & 1u) != 0) atomicAdd(&S.hist[0], 1u);             // pad nibble
+            count += __popc(m);
+            const bool need = stop < 2 && set == 0;
+            const uint32_t needs = __ballot_sync(FULL, need);
+            if (stop < 2) {
+                if (need) {
+                    B.ops[8 * r + c] = (uint8_t)(stop << 3);
+                    B.pal_lab[8 * r + c] = label;
+                }
+                if (c == 0) B.need8[r] = (uint8_t)(needs >> (lane & 24u));
             }
-            __syncthreads();
-            if (tid < 16) hist_out[((size_t)i * kModes + mode) * 16 + tid] = S.hist[tid];
-            __syncthreads();
+        });
+        if (count) atomicAdd(sets + lane, count);
+        __syncthreads();
+        palette_walk<T>(B, root, n_act, [&](uint32_t j, uint32_t code, uint32_t delta) {
+            atomicAdd(&S.hist[code << 1 | (B.ops[j] >> 3 & 1u)], 1u);
+            if (code == OP_PD) atomicAdd(&S.hist[delta], 1u);
+        });
+        if (tid == 0) {
+            S.hist[(OP_PA << 1) | (n_act == 0 ? 1u : 0u)] += 1;     // root nibble
+            if ((1 + n_ops + S.n_pd) & 1u) S.hist[0] += 1;          // pad nibble
         }
+        __syncthreads();
+        for (uint32_t k = tid; k < kModes * 16; k += T) {
+            const uint32_t mode = k >> 4, nib = k & 15u;
+            const uint64_t codes = kModeTable.t[mode];
+            uint32_t n = S.hist[nib];
+            for (uint32_t set = 1; set < 16; ++set)
+                if (((uint32_t)(codes >> (3 * set)) & 7u) == nib >> 1) n += sets[set << 1 | (nib & 1u)];
+            hist_out[(size_t)i * kModes * 16 + k] = n;
+        }
+        __syncthreads();
     }
 }
 
@@ -827,23 +1198,43 @@ cudaError_t grow(T** p, size_t* cap, size_t need) {
     return e;
 }
 
-size_t enc_scratch_per_cta(uint32_t b) {
-    uint32_t L = levels_of(b);
-    uint64_t mo = max_ops_of(b);
-    auto al = [](uint64_t v) { return (v + 255) & ~255ull; };
-    uint64_t n_g = L >= kEncSmemLevels + 2 ? (1ull << (3 * (L - 2))) : 0;
-    return al(8 * n_g) + al(n_g) + al(mo) + al(8 * mo) + al(2 * mo + 2) + al(8 * (mo + 1));
+int sm_count(int device) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return std::max(1, sms);
 }
 
-int g_enc_occ[64] = {0};
-uint32_t enc_grid(int device) {
-    int& occ = g_enc_occ[device & 63];
-    if (occ == 0) {
-        int per_sm = 0, sms = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enc_bricks_kernel, kEncThreads, 0);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        occ = std::max(1, per_sm) * std::max(1, sms);
-    }
+// K1's two forms.  64^3 bricks: one CTA of 1024 threads per SM (512 bricks 0.76 ms, 150
+// bricks 0.26 ms; 384 threads, four per SM: 0.85 and 0.42 ms -- a brick in flight takes
+// 2 MB of the L2 that its second look at the voxels wants to find them in).  Smaller
+// bricks, whose phases are short against their barriers: 320 threads, four per SM (8192
+// bricks of 32^3 0.66 ms, against 1.27 ms); 32^3 ones no more than there are SMs take
+// the first form (60 bricks 54 against 69 us).
+bool enc_wide(uint32_t L, uint32_t nb, int device) { return L >= 7 || (L == 6 && nb <= (uint32_t)sm_count(device)); }
+template <class F>
+auto enc_form(bool wide, F f) {
+    return wide ? f(std::integral_constant<int, 1024>(), std::integral_constant<int, 1>())
+                : f(std::integral_constant<int, 320>(), std::integral_constant<int, 4>());
+}
+
+size_t enc_scratch_per_cta(uint32_t L, bool wide) {
+    return enc_form(wide, [&](auto t, auto) -> size_t { return enc_scratch<decltype(t)::value>(L).bytes; });
+}
+
+// CTAs of K1 or the statistics kernel that the device holds.
+int g_enc_occ[64][8][2] = {};
+uint32_t enc_grid(int device, uint32_t L, bool wide) {
+    int& occ = g_enc_occ[device & 63][L & 7][wide];
+    if (occ == 0)
+        occ = enc_form(wide, [&](auto t, auto n) {
+            constexpr int T = decltype(t)::value, N = decltype(n)::value;
+            int a = 0, b = 0;
+            for (const void* k : {(const void*)enc_bricks_kernel<T, N>, (const void*)enc_stats_kernel<T, N>})
+                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)enc_smem<T>(7));
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, enc_bricks_kernel<T, N>, T, enc_smem<T>(L));
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, enc_stats_kernel<T, N>, T, enc_smem<T>(L));
+            return std::max(1, std::min(a, b)) * sm_count(device);
+        });
     return (uint32_t)occ;
 }
 
@@ -904,8 +1295,9 @@ int encode_stats(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W,
         err = cudaGetErrorString(e);
         return CSV_ECUDA;
     }
-    const uint32_t grid = std::min<uint32_t>(enc_grid(device), std::max<uint32_t>(nb, 1));
-    const size_t per_cta = enc_scratch_per_cta(b);
+    const bool wide = enc_wide(levels_of(b), nb, device);
+    const uint32_t grid = std::min<uint32_t>(enc_grid(device, levels_of(b), wide), std::max<uint32_t>(nb, 1));
+    const size_t per_cta = enc_scratch_per_cta(levels_of(b), wide);
     if ((e = grow(&s->d_scratch, &s->scratch_cap, per_cta * grid)) != cudaSuccess ||
         (e = cudaMemsetAsync(s->d_misc, 0, kMiscWords * sizeof(unsigned long long), st)) != cudaSuccess) {
         err = cudaGetErrorString(e);
@@ -922,7 +1314,13 @@ int encode_stats(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W,
     A.scratch = s->d_scratch;
     A.scratch_per_cta = per_cta;
     A.misc = s->d_misc;
-    if (nb) enc_stats_kernel<<<grid, kEncThreads, 0, st>>>(A, d_hist);
+    A.pairs = W % 2 == 0 && (uintptr_t)d_vol % 16 == 0;
+    if (nb)
+        enc_form(wide, [&](auto t, auto n) {
+            constexpr int T = decltype(t)::value;
+            enc_stats_kernel<T, decltype(n)::value><<<grid, T, enc_smem<T>(A.L), st>>>(A, d_hist);
+            return 0;
+        });
     if ((e = cudaGetLastError()) != cudaSuccess) {
         err = cudaGetErrorString(e);
         return CSV_ECUDA;
@@ -975,8 +1373,9 @@ int encode_device(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W
         static_assert(sizeof(unsigned long long) == 8, "");
         if (!s->d_misc) CK(cudaMalloc(&s->d_misc, kMiscWords * sizeof(unsigned long long)));
     }
-    const uint32_t grid = std::min<uint32_t>(enc_grid(device), std::max<uint32_t>(nb, 1));
-    const size_t per_cta = enc_scratch_per_cta(b);
+    const bool wide = enc_wide(levels_of(b), nb, device);
+    const uint32_t grid = std::min<uint32_t>(enc_grid(device, levels_of(b), wide), std::max<uint32_t>(nb, 1));
+    const size_t per_cta = enc_scratch_per_cta(levels_of(b), wide);
     CK(grow(&s->d_scratch, &s->scratch_cap, per_cta * grid));
     size_t nib_need = std::max<size_t>(1 << 20, nvox / 4 + 16ull * nb);
     size_t pal_need = std::max<size_t>(1 << 16, nvox / 256 + 64ull * nb);
@@ -1011,8 +1410,13 @@ int encode_device(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W
         A.sel = sel ? sel->d_sel : nullptr;
         A.bx0 = shard ? shard->bx0 : 0u;
         A.index_base = shard ? shard->index_base : 0u;
+        A.pairs = W % 2 == 0 && (uintptr_t)d_vol % 16 == 0;
         if (nb > 0) {
-            enc_bricks_kernel<<<grid, kEncThreads, 0, st>>>(A);
+            enc_form(wide, [&](auto t, auto n) {
+                constexpr int T = decltype(t)::value;
+                enc_bricks_kernel<T, decltype(n)::value><<<grid, T, enc_smem<T>(A.L), st>>>(A);
+                return 0;
+            });
             CK(cudaGetLastError());
         }
         unsigned long long misc[kMiscWords];
@@ -1090,9 +1494,7 @@ static int finish_encode(EncoderState* s, const EncodeSelection* sel, cudaStream
     CK(grow(&s->d_rec_off, &s->rec_cap, std::max<uint32_t>(nb, 1)));
     CK(cudaMemcpyAsync(s->d_enc_off, enc_off.data(), 8ull * nb, cudaMemcpyHostToDevice, st));
     if (nb) {
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-        const uint32_t n_sm = (uint32_t)std::max(sms, 1);
+        const uint32_t n_sm = (uint32_t)sm_count(s->device);
         auto rans = [&](auto kernel, uint32_t K) {
             kernel<<<(nb + K - 1) / K, 32 * (K + 1), 0, st>>>(s->d_meta, nb, s->d_nib, s->d_enc_off, s->d_enc,
                                                              s->d_model, s->n_tables, s->d_ck, n_sm);

@@ -50,3 +50,39 @@ def test_rans_steps_and_checkpoints(codec, oracle, shape, brick):
     ref, _ = oracle.decode_image(oracle.encode(vol, brick), lod)
     assert np.array_equal(out.cpu().numpy().view(np.uint64), ref.ravel())
     ds.close()
+
+
+def _host_volume(shape, seed, labels, zero=0.0):
+    rng = np.random.default_rng(seed)
+    vol = rng.integers(1, 2 ** 63, labels, dtype=np.uint64)[rng.integers(0, labels, shape)]
+    vol[rng.random(shape) < zero] = 0
+    return vol
+
+
+# every brick edge; odd rows (no 16-byte voxel pairs) and bricks cut by the volume's end; noise, in which every
+# node is active and the palette walk misses most of the time; one brick and more than one per SM; sampled bricks
+@pytest.mark.parametrize("brick", [2, 4, 8, 16, 32, 64])
+@pytest.mark.parametrize("shape", [(64, 64, 64), (37, 70, 65), (5, 3, 1)])
+@pytest.mark.parametrize("labels", [2, 3, 5, 40, 5000])
+def test_bricks_bytes_and_statistics(codec, oracle, shape, brick, labels):
+    import torch
+    vol = _host_volume(shape, labels + brick, labels, zero=0.2) if labels != 40 else _volume(shape, brick)
+    d = torch.from_numpy(vol.view(np.int64)).cuda()
+    n = codec.encode_device(d, brick)
+    img = bytes(codec.encoded_image_tensor().cpu().numpy())
+    assert len(img) == n and img == oracle.encode(vol, brick)
+    if brick >= 8 and labels != 5000:
+        nb = int(np.prod([-(-n // brick) for n in shape]))
+        hist = torch.full((nb, 12, 16), -1, dtype=torch.int32, device="cuda")
+        codec.encode_stats(d, brick, hist)
+        assert np.array_equal(hist.cpu().numpy(), oracle.encode_stats(vol, brick).reshape(nb, 12, 16))
+
+
+# 32^3 bricks: as many as SMs or fewer (one wide CTA per SM), and more of them
+@pytest.mark.parametrize("shape", [(96, 96, 100), (200, 190, 161)])
+def test_bricks_forms(codec, oracle, shape):
+    import torch
+    vol = _volume(shape, 5, 60)
+    n = codec.encode_device(torch.from_numpy(vol.view(np.int64)).cuda(), 32)
+    img = bytes(codec.encoded_image_tensor().cpu().numpy())
+    assert len(img) == n and img == oracle.encode(vol, 32)
