@@ -58,6 +58,8 @@ struct RayArgs {
 
 __device__ __forceinline__ float fsgn(float x) { return x > 0.f ? 1.f : (x < 0.f ? -1.f : 0.f); }
 __device__ __forceinline__ int isgn(float x) { return (x > 0.f ? 1 : 0) + (x < 0.f ? -1 : 0); }
+// v / 2^k, towards zero (brick sizes and LOD strides are powers of two)
+__device__ __forceinline__ int div_pow2(int v, int k) { return (v + ((v >> 31) & ((1 << k) - 1))) >> k; }
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 __device__ __forceinline__ uint32_t spread10(uint32_t v) {
@@ -85,16 +87,18 @@ __device__ __forceinline__ bool is_hidden(const RayArgs& A, uint64_t v) {
 // hashLabel (decode.wgsl:135-172): the transfer function's colour, else a
 // colour mixed from the label's two 32-bit halves with alpha 0x40; label 0 is
 // transparent.  The table's keys are unique, so a binary search finds the entry
-// the shader's linear search finds.
-__device__ __forceinline__ uint32_t label_rgba(const RayArgs& A, uint64_t v) {
+// the shader's linear search finds.  (A call, not inline: looked up only where a ray's
+// label changes, and the colour kernel's code has to stay in the instruction cache.)
+__device__ __noinline__ uint32_t label_rgba(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ rgba,
+                                            uint32_t n, uint64_t v) {
     if (v == 0) return 0u;
-    uint32_t lo = 0, hi = A.n_tf;
+    uint32_t lo = 0, hi = n;
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (A.tf_keys[mid] < v) lo = mid + 1;
+        if (__ldg(keys + mid) < v) lo = mid + 1;
         else hi = mid;
     }
-    if (lo < A.n_tf && A.tf_keys[lo] == v) return A.tf_rgba[lo];
+    if (lo < n && __ldg(keys + lo) == v) return __ldg(rgba + lo);
     uint32_t sl = (uint32_t)v, sh = (uint32_t)(v >> 32);
     sl = sl ^ sh;
     sl = sl ^ (sl >> 16);
@@ -109,41 +113,63 @@ __device__ __forceinline__ uint32_t label_rgba(const RayArgs& A, uint64_t v) {
 
 __device__ __forceinline__ float chan(uint32_t rgba, int k) { return (float)((rgba >> (8 * k)) & 0xFFu) / 255.0f; }
 
-// getVoxelColor (:159-198) of a resident slot at brick-local voxel (x, y, z), as RGBA8
-__device__ __forceinline__ uint32_t slot_rgba(const RayArgs& A, const csv_brick_slot& sl, int x, int y, int z) {
-    const int sh = A.lb - (int)sl.lod;
-    const uint64_t lab = sl.lod == 0 ? __ldg(A.labels + sl.offset)
-                                     : __ldg(A.labels + sl.offset + mort((uint32_t)x >> sh, (uint32_t)y >> sh,
-                                                                          (uint32_t)z >> sh));
-    return label_rgba(A, lab);
+// Morton code of a brick-local voxel: bricks up to 64^3 take each axis from a table in
+// shared memory (the shader's bit spreading is ten operations an axis, and a shadow ray
+// needs it at every step).
+constexpr int kSpreadTab = 64;
+__device__ __forceinline__ uint32_t mort_local(const RayArgs& A, const uint32_t* spread, int x, int y, int z) {
+    if (A.bs <= kSpreadTab) return spread[x] | (spread[y] << 1) | (spread[z] << 2);
+    return mort((uint32_t)x, (uint32_t)y, (uint32_t)z);
 }
 
-// sampleAlpha (:272-299): alpha at a world voxel through its brick's slot (0 outside
-// the volume, for empty bricks, and for bricks not resident in the cache)
-__device__ float sample_alpha(const RayArgs& A, int wx, int wy, int wz) {
+// A ray's memory of its last alpha sample: the label it looked up and its alpha, and the
+// brick it was in with its slot.  Successive samples mostly share both.
+struct AlphaMemo {
+    uint64_t lab = 0;
+    float alpha = 0.0f;  // label 0 is transparent
+    uint32_t brick = 0xFFFFFFFFu;  // x | y << 10 | z << 20 of the brick
+    uint32_t sh3 = 0;              // 3 (log2(brick size) - LOD)
+    bool none = true;              // no such brick, empty, or not resident: alpha 0
+    uint64_t offset = 0;
+    const uint32_t* spread = nullptr;
+};
+__device__ __forceinline__ float label_alpha(const RayArgs& A, AlphaMemo& M, uint64_t lab) {
+    if (lab != M.lab) {
+        M.lab = lab;
+        M.alpha = chan(label_rgba(A.tf_keys, A.tf_rgba, A.n_tf, lab), 3);
+    }
+    return M.alpha;
+}
+
+// sampleAlpha (:272-299) with getVoxelColor (:159-198): alpha at a world voxel through
+// its brick's slot (0 outside the volume, for empty bricks, and for bricks not resident in
+// the cache).  sampleAlphaInBrick (:301-318) is the same for voxels of the ray's brick.
+__device__ __forceinline__ float sample_alpha(const RayArgs& A, AlphaMemo& M, int wx, int wy, int wz) {
     const int g = (int)A.grid;
     if (wx < 0 || wy < 0 || wz < 0 || wx >= g || wy >= g || wz >= g) return 0.0f;
-    const int bx = wx / A.bs, by = wy / A.bs, bz = wz / A.bs;
+    const int bx = wx >> A.lb, by = wy >> A.lb, bz = wz >> A.lb;  // (the brick size is a power of two)
     if (bx >= A.num_bricks || by >= A.num_bricks || bz >= A.num_bricks) return 0.0f;
-    const uint32_t m = mort((uint32_t)bx, (uint32_t)by, (uint32_t)bz);
-    if (m >= A.n_slots) return 0.0f;
-    const csv_brick_slot sl = A.slots[m];
-    if (sl.flags & (CSV_SLOT_EMPTY | CSV_SLOT_MISSING)) return 0.0f;
-    return chan(slot_rgba(A, sl, wx - bx * A.bs, wy - by * A.bs, wz - bz * A.bs), 3);
-}
-
-// sampleAlphaInBrick (:301-318)
-__device__ __forceinline__ float sample_alpha_in(const RayArgs& A, const csv_brick_slot& sl, const int* bmin, int wx,
-                                                 int wy, int wz) {
-    const int g = (int)A.grid;
-    if (wx < 0 || wy < 0 || wz < 0 || wx >= g || wy >= g || wz >= g) return 0.0f;
-    const int lx = wx - bmin[0], ly = wy - bmin[1], lz = wz - bmin[2];
-    if (lx < 0 || ly < 0 || lz < 0 || lx >= A.bs || ly >= A.bs || lz >= A.bs) return sample_alpha(A, wx, wy, wz);
-    return chan(slot_rgba(A, sl, lx, ly, lz), 3);
+    const uint32_t brick = (uint32_t)bx | (uint32_t)by << 10 | (uint32_t)bz << 20;
+    if (brick != M.brick) {
+        M.brick = brick;
+        const uint32_t m = mort((uint32_t)bx, (uint32_t)by, (uint32_t)bz);
+        M.none = true;
+        if (m < A.n_slots) {
+            const csv_brick_slot sl = A.slots[m];
+            M.none = (sl.flags & (CSV_SLOT_EMPTY | CSV_SLOT_MISSING)) != 0;
+            M.offset = sl.offset;
+            M.sh3 = 3 * (uint32_t)(A.lb - (int)sl.lod);
+        }
+    }
+    if (M.none) return 0.0f;
+    const int lm = A.bs - 1;
+    // dropping sh bits of every axis drops 3 sh bits of the Morton code
+    return label_alpha(A, M, __ldg(A.labels + M.offset + (mort_local(A, M.spread, wx & lm, wy & lm, wz & lm) >> M.sh3)));
 }
 
 // traceShadowRay (:329-397): 1 = lit, 0 = occluded
-__device__ float shadow_ray(const RayArgs& A, const float* start, const float* nrm, float acc_alpha, float trans) {
+__device__ __forceinline__ float shadow_ray(const RayArgs& A, AlphaMemo& M, const float* start, const float* nrm, float acc_alpha,
+                            float trans) {
     if (trans < 0.1f || acc_alpha < 0.2f) return 1.0f;
     const uint32_t steps = max(24u, (uint32_t)(64.0f * trans));
     const float ll = sqrtf((A.light[0] * A.light[0] + A.light[1] * A.light[1]) + A.light[2] * A.light[2]);
@@ -154,12 +180,13 @@ __device__ float shadow_ray(const RayArgs& A, const float* start, const float* n
         rs[a] = start[a] + nrm[a] * 0.6f;
     }
     float t = 0.5f, occ = 0.0f;
+#pragma unroll 1
     for (uint32_t i = 0; i < steps; ++i) {
         float p[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) p[a] = rs[a] + dir[a] * t;
         if (p[0] < 0.0f || p[1] < 0.0f || p[2] < 0.0f || p[0] >= A.grid || p[1] >= A.grid || p[2] >= A.grid) break;
-        occ = occ + sample_alpha(A, (int)floorf(p[0]), (int)floorf(p[1]), (int)floorf(p[2])) * 1.0f;
+        occ = occ + sample_alpha(A, M, (int)floorf(p[0]), (int)floorf(p[1]), (int)floorf(p[2])) * 1.0f;
         if (occ > 0.8f) return 0.0f;
         t = t + 1.0f;
     }
@@ -167,14 +194,50 @@ __device__ float shadow_ray(const RayArgs& A, const float* start, const float* n
     return 1.0f * (1.0f - trans) + vis * trans;  // mix(1, vis, trans)
 }
 
-template <bool RGBA>
-__global__ void __launch_bounds__(128) render_kernel(RayArgs A) {
-    const uint32_t px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y * blockDim.y + threadIdx.y;
+// One axis of a Morton code: x is bits 0, 3, .., y 1, 4, .., z 2, 5, .. (10 of each, and
+// one more where the word has room).  A voxel forward along it is m - axis in these bits
+// ((m | ~axis) + 1), one back m - 1.
+constexpr uint32_t kAxisX = 0x49249249u, kAxisY = 0x92492492u, kAxisZ = 0x24924924u;
+__device__ __forceinline__ uint32_t axis_move(uint32_t axis, int d) { return d > 0 ? 0u - axis : (d < 0 ? ~0u : 0u); }
+__device__ __forceinline__ int unspread10(uint32_t m) {
+    m &= 0x09249249u;
+    m = (m ^ (m >> 2)) & 0x030c30c3u;
+    m = (m ^ (m >> 4)) & 0x0300f00fu;
+    m = (m ^ (m >> 8)) & 0x030000ffu;
+    m = (m ^ (m >> 16)) & 0x000003ffu;
+    return (int)m;
+}
+
+// Latency bound: a ray is one chain of cells.  What a step does is kept small (the cell's
+// Morton code moves by one addition and also tells when the brick ends, the next label is
+// read while this one is looked at, the divisions by brick size and stride are shifts),
+// and colour rays remember the last label and brick they looked up; their code is kept in
+// the instruction cache by one copy of each lookup.  Measured (B200, 1080p, a 512^3
+// volume in colour, a 768^3 one in labels): RGBA 2.05 -> 0.92 ms, labels 0.138 -> 0.124 ms.
+// Eight blocks per SM (six: 0.97 and 0.125 ms).
+// HUGE: bricks of 1024^3, whose last voxel's neighbour has no Morton code of its own (the word has
+// 10 bits for z): the voxel is kept beside its code to tell when it leaves the brick.
+template <bool RGBA, bool HUGE>
+__global__ void __launch_bounds__(128, 8) render_kernel(RayArgs A) {
+    __shared__ uint32_t s_spread[RGBA ? kSpreadTab : 1];
+    if (RGBA) {
+        if (threadIdx.x < kSpreadTab) s_spread[threadIdx.x] = spread10(threadIdx.x);
+        __syncthreads();
+    }
+    // a warp's pixels are an 8 x 4 tile, a block's 16 x 8
+    const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
+    const uint32_t px = blockIdx.x * 16 + 8 * (wp & 1u) + (lane & 7u), py = blockIdx.y * 8 + 4 * (wp >> 1) + (lane >> 3);
     if (px >= A.W || py >= A.H) return;
     const size_t pix = (size_t)py * A.W + px;
     uint64_t out_lab = 0;
     float out_t = INFINITY;
     float hc[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // RGBA mode: front-to-back accumulated colour
+    // and the last sample's label with its colour and its opacity corrected for the LOD stride
+    uint64_t c_lab = 0;
+    float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, ca = 0.0f;
+    int c_stride = 0;
+    AlphaMemo memo;
+    memo.spread = s_spread;
     const float fw = (float)A.W, fh = (float)A.H, aspect = fw / fh;
     const float ndc_x = (((float)px + 0.5f) / fw) * 2.0f - 1.0f;
     const float ndc_y = 1.0f - (((float)py + 0.5f) / fh) * 2.0f;
@@ -210,7 +273,7 @@ __global__ void __launch_bounds__(128) render_kernel(RayArgs A) {
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 float pos = A.o[a] + d[a] * ts;
-                brick[a] = (int)floorf(pos) / bs;
+                brick[a] = div_pow2((int)floorf(pos), A.lb);
                 step[a] = isgn(d[a]);
                 float bf = (float)brick[a] * (float)bs;
                 float nb = d[a] > 0.0f ? bf + (float)bs : bf;
@@ -221,8 +284,8 @@ __global__ void __launch_bounds__(128) render_kernel(RayArgs A) {
         int be[3], bx[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            be[a] = (int)(A.o[a] + d[a] * tEnter) / bs;
-            bx[a] = (int)(A.o[a] + d[a] * tExit) / bs;
+            be[a] = div_pow2((int)(A.o[a] + d[a] * tEnter), A.lb);
+            bx[a] = div_pow2((int)(A.o[a] + d[a] * tExit), A.lb);
         }
         const uint32_t maxCross = (uint32_t)(abs(bx[0] - be[0]) + abs(bx[1] - be[1]) + abs(bx[2] - be[2])) + 6u;
         float brickEntryT = tEnter;
@@ -266,14 +329,13 @@ __global__ void __launch_bounds__(128) render_kernel(RayArgs A) {
                     vtMax[a] = (nb - A.o[a]) * inv[a];
                     vtDelta[a] = fabsf(inv[a]);
                 }
-                const int lodSize = 1 << sl.lod;
-                const int stride = bs / lodSize;
+                const int stride = bs >> sl.lod;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) vox[a] -= bmin[a];
                 if (stride > 1) {  // LOD quantisation (:706-731)
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
-                        int lv = (vox[a] / stride) * stride;
+                        int lv = div_pow2(vox[a], A.lb - (int)sl.lod) * stride;
                         vox[a] = clampi(lv, 0, bs - 1);
                         vtDelta[a] = fabsf(inv[a]) * (float)stride;
                         float lw = (float)bmin[a] + (float)vox[a];
@@ -285,101 +347,137 @@ __global__ void __launch_bounds__(128) render_kernel(RayArgs A) {
                     for (int a = 0; a < 3; ++a) vox[a] = clampi(vox[a], 0, bs - 1);
                 }
                 int le[3], lx[3];
+                const float inv_stride = 1.0f / (float)stride;  // a power of two: multiplying by it is the division
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     float ve = A.o[a] + d[a] * tEnterBrick, vx = A.o[a] + d[a] * tExitBrick;
-                    le[a] = (int)floorf((ve - (float)bmin[a]) / (float)stride);
-                    lx[a] = (int)ceilf((vx - (float)bmin[a]) / (float)stride);
+                    le[a] = (int)floorf((ve - (float)bmin[a]) * inv_stride);
+                    lx[a] = (int)ceilf((vx - (float)bmin[a]) * inv_stride);
                 }
                 const uint32_t maxSteps =
                     (uint32_t)(abs(lx[0] - le[0]) + abs(lx[1] - le[1]) + abs(lx[2] - le[2])) + 128u;
-                const int sh = A.lb - (int)sl.lod;
+                // the voxel's Morton code, an axis at a time; at a coarser LOD a cell is its code without
+                // the low 3 (log2(brick size) - LOD) bits (LOD 0: the brick's one label)
+                const uint32_t sh3 = 3 * (uint32_t)(A.lb - (int)sl.lod), end = HUGE ? 0u : 1u << (3 * A.lb);
+                uint32_t mx = spread10((uint32_t)vox[0]), my = spread10((uint32_t)vox[1]) << 1,
+                         mz = spread10((uint32_t)vox[2]) << 2;
+                const uint32_t dx = axis_move(kAxisX, step[0]), dy = axis_move(kAxisY, step[1]),
+                               dz = axis_move(kAxisZ, step[2]);
+                const uint64_t* labels = A.labels + sl.offset;
                 float tcell = tEnterBrick;
-                for (uint32_t vi = 0; vi < maxSteps; ++vi) {
-                    if (RGBA && vox[0] >= 0 && vox[1] >= 0 && vox[2] >= 0 && vox[0] < bs && vox[1] < bs &&
-                        vox[2] < bs) {
-                        const uint32_t rgba = slot_rgba(A, sl, vox[0], vox[1], vox[2]);
-                        float c[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) c[k] = chan(rgba, k);
-                        if (c[3] > 0.05f) {
-                            float sc[3] = {c[0], c[1], c[2]};
-                            if (c[3] > 0.35f) {  // shading (:803-826)
-                                float wp[3];
-                                int vp[3];
-#pragma unroll
-                                for (int a = 0; a < 3; ++a) {
-                                    wp[a] = (float)(bmin[a] + vox[a]) + 0.5f;
-                                    vp[a] = (int)wp[a];
-                                }
-                                float gr[3];  // computeGradientLOD (:428-455)
-#pragma unroll
-                                for (int a = 0; a < 3; ++a) {
-                                    int qp[3] = {vp[0], vp[1], vp[2]}, qn[3] = {vp[0], vp[1], vp[2]};
-                                    qp[a] += stride;
-                                    qn[a] -= stride;
-                                    float ap = sample_alpha_in(A, sl, bmin, qp[0], qp[1], qp[2]);
-                                    float an = sample_alpha_in(A, sl, bmin, qn[0], qn[1], qn[2]);
-                                    ap = ap > 0.05f ? ap : c[3];
-                                    an = an > 0.05f ? an : c[3];
-                                    gr[a] = (ap - an) * 0.5f;
-                                }
-                                const float gl = sqrtf((gr[0] * gr[0] + gr[1] * gr[1]) + gr[2] * gr[2]);
-                                float nrm[3];
-#pragma unroll
-                                for (int a = 0; a < 3; ++a) nrm[a] = -gr[a] / fmaxf(gl, 0.001f);
-                                float shadow = 1.0f;
-                                if (c[3] > 0.4f) shadow = shadow_ray(A, wp, nrm, hc[3], 1.0f - hc[3]);
-                                const float ll = sqrtf((A.light[0] * A.light[0] + A.light[1] * A.light[1]) +
-                                                       A.light[2] * A.light[2]);
-                                const float ld = fmaxf(0.0f, (nrm[0] * (A.light[0] / ll) + nrm[1] * (A.light[1] / ll)) +
-                                                                 nrm[2] * (A.light[2] / ll));
-                                const float ds = A.diffuse * shadow;
-                                const float min_amb = ld > 0.01f ? 0.3f : 0.1f;
-                                const float sf = fminf(fmaxf(A.ambient + ld * ds, min_amb), 1.0f);
-                                const float lum = (c[0] * 0.299f + c[1] * 0.587f) + c[2] * 0.114f;
-                                const float smix = fminf(fmaxf(1.0f - shadow, 0.0f), 1.0f) * 0.5f;
-#pragma unroll
-                                for (int k = 0; k < 3; ++k) {
-                                    const float gray = lum * 0.8f + c[k] * 0.2f;
-                                    sc[k] = (c[k] * (1.0f - smix) + gray * smix) * sf;  // mix(c, gray, smix)
-                                }
-                            }
-                            // compositing (:828-836): opacity corrected for the LOD stride
-                            const float ca = fminf(fmaxf(1.0f - powf(1.0f - c[3], (float)stride), 0.0f), 1.0f);
-                            const float sa = ca * (1.0f - hc[3]);
-#pragma unroll
-                            for (int k = 0; k < 3; ++k) hc[k] = hc[k] + sc[k] * sa;
-                            hc[3] = hc[3] + sa;
-                            if (hc[3] > 0.95f) {
-                                done = true;
-                                break;
-                            }
-                        }
-                    } else if (!RGBA && vox[0] >= 0 && vox[1] >= 0 && vox[2] >= 0 && vox[0] < bs && vox[1] < bs &&
-                               vox[2] < bs) {
-                        uint64_t lab;
-                        if (sl.lod == 0) lab = __ldg(A.labels + sl.offset);
-                        else
-                            lab = __ldg(A.labels + sl.offset +
-                                        mort((uint32_t)vox[0] >> sh, (uint32_t)vox[1] >> sh, (uint32_t)vox[2] >> sh));
-                        if (lab != 0 && !(A.n_hidden && is_hidden(A, lab))) {
-                            out_lab = lab;
-                            out_t = tcell;
-                            done = true;
-                            break;
-                        }
+                // advanceDDA (:501-517); returns the t at which the next cell is entered
+                auto advance = [&]() -> float {
+                    const bool p0 = vtMax[0] < vtMax[1] && vtMax[0] < vtMax[2], p1 = !p0 && vtMax[1] < vtMax[2];
+                    const float t = p0 ? vtMax[0] : (p1 ? vtMax[1] : vtMax[2]);
+                    if (p0) {
+                        vtMax[0] += vtDelta[0];
+                        mx = (mx + dx) & kAxisX;
+                        if (HUGE) vox[0] += step[0];
                     }
-                    float t;  // advanceDDA (:501-517)
-                    if (vtMax[0] < vtMax[1] && vtMax[0] < vtMax[2]) {
-                        t = vtMax[0]; vtMax[0] += vtDelta[0]; vox[0] += step[0];
-                    } else if (vtMax[1] < vtMax[2]) {
-                        t = vtMax[1]; vtMax[1] += vtDelta[1]; vox[1] += step[1];
-                    } else {
-                        t = vtMax[2]; vtMax[2] += vtDelta[2]; vox[2] += step[2];
+                    if (p1) {
+                        vtMax[1] += vtDelta[1];
+                        my = (my + dy) & kAxisY;
+                        if (HUGE) vox[1] += step[1];
+                    }
+                    if (!p0 && !p1) {
+                        vtMax[2] += vtDelta[2];
+                        mz = (mz + dz) & kAxisZ;
+                        if (HUGE) vox[2] += step[2];
+                    }
+                    return t;
+                };
+                // 0, the invisible label, outside the brick (whose codes end at 8^log2(brick size))
+                auto load = [&]() -> uint64_t {
+                    const uint32_t m = mx | my | mz;
+                    if (HUGE ? ((uint32_t)vox[0] | (uint32_t)vox[1] | (uint32_t)vox[2]) >= (uint32_t)bs : m >= end)
+                        return 0ull;
+                    return __ldg(labels + (m >> sh3));
+                };
+                // the next cell's label is on its way while this one's is looked at
+                uint64_t lab = load();
+                for (uint32_t vi = 0; vi < maxSteps; ++vi) {
+                    const uint64_t here = lab;
+                    const uint32_t m_here = mx | my | mz;
+                    const float t = advance();
+                    const bool leave = t > tExitBrick;
+                    if (!leave) lab = load();
+                    if (RGBA) {
+                        if (here != 0) {
+                            if (here != c_lab || stride != c_stride) {
+                                const uint32_t rgba = label_rgba(A.tf_keys, A.tf_rgba, A.n_tf, here);
+                                c_lab = here;
+                                c_stride = stride;
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) c[k] = chan(rgba, k);
+                                // compositing (:828-836): opacity corrected for the LOD stride
+                                ca = fminf(fmaxf(1.0f - powf(1.0f - c[3], (float)stride), 0.0f), 1.0f);
+                            }
+                            if (c[3] > 0.05f) {
+                                float sc[3] = {c[0], c[1], c[2]};
+                                if (c[3] > 0.35f) {  // shading (:803-826)
+                                    float wp[3];
+                                    int vp[3];
+                                    const int at[3] = {unspread10(m_here), unspread10(m_here >> 1),
+                                                       unspread10(m_here >> 2)};
+#pragma unroll
+                                    for (int a = 0; a < 3; ++a) {
+                                        wp[a] = (float)(bmin[a] + at[a]) + 0.5f;
+                                        vp[a] = (int)wp[a];
+                                    }
+                                    // computeGradientLOD (:428-455): per axis the sample ahead, then the one behind
+                                    float gr[3] = {0.0f, 0.0f, 0.0f}, ahead = 0.0f;
+#pragma unroll 1
+                                    for (int k = 0; k < 6; ++k) {
+                                        const int a = k >> 1, d = (k & 1) ? -stride : stride;
+                                        float al = sample_alpha(A, memo, vp[0] + (a == 0 ? d : 0),
+                                                                vp[1] + (a == 1 ? d : 0), vp[2] + (a == 2 ? d : 0));
+                                        al = al > 0.05f ? al : c[3];
+                                        const float g = (ahead - al) * 0.5f;
+                                        if (k == 1) gr[0] = g;
+                                        if (k == 3) gr[1] = g;
+                                        if (k == 5) gr[2] = g;
+                                        ahead = al;
+                                    }
+                                    const float gl = sqrtf((gr[0] * gr[0] + gr[1] * gr[1]) + gr[2] * gr[2]);
+                                    float nrm[3];
+#pragma unroll
+                                    for (int a = 0; a < 3; ++a) nrm[a] = -gr[a] / fmaxf(gl, 0.001f);
+                                    float shadow = 1.0f;
+                                    if (c[3] > 0.4f) shadow = shadow_ray(A, memo, wp, nrm, hc[3], 1.0f - hc[3]);
+                                    const float ll = sqrtf((A.light[0] * A.light[0] + A.light[1] * A.light[1]) +
+                                                           A.light[2] * A.light[2]);
+                                    const float ld =
+                                        fmaxf(0.0f, (nrm[0] * (A.light[0] / ll) + nrm[1] * (A.light[1] / ll)) +
+                                                        nrm[2] * (A.light[2] / ll));
+                                    const float ds = A.diffuse * shadow;
+                                    const float min_amb = ld > 0.01f ? 0.3f : 0.1f;
+                                    const float sf = fminf(fmaxf(A.ambient + ld * ds, min_amb), 1.0f);
+                                    const float lum = (c[0] * 0.299f + c[1] * 0.587f) + c[2] * 0.114f;
+                                    const float smix = fminf(fmaxf(1.0f - shadow, 0.0f), 1.0f) * 0.5f;
+#pragma unroll
+                                    for (int k = 0; k < 3; ++k) {
+                                        const float gray = lum * 0.8f + c[k] * 0.2f;
+                                        sc[k] = (c[k] * (1.0f - smix) + gray * smix) * sf;  // mix(c, gray, smix)
+                                    }
+                                }
+                                const float sa = ca * (1.0f - hc[3]);
+#pragma unroll
+                                for (int k = 0; k < 3; ++k) hc[k] = hc[k] + sc[k] * sa;
+                                hc[3] = hc[3] + sa;
+                                if (hc[3] > 0.95f) {
+                                    done = true;
+                                    break;
+                                }
+                            }
+                        }
+                    } else if (here != 0 && !(A.n_hidden && is_hidden(A, here))) {
+                        out_lab = here;
+                        out_t = tcell;
+                        done = true;
+                        break;
                     }
                     tcell = t;
-                    if (t > tExitBrick) break;
+                    if (leave) break;
                 }
                 if (done) break;
             }
@@ -436,8 +534,9 @@ cudaError_t launch_render(const csv_camera& cam, uint32_t W, uint32_t H, float g
     A.tf_rgba = nullptr;
     A.n_tf = 0;
     A.out_rgba = nullptr;
-    dim3 block(16, 8), grid2((W + 15) / 16, (H + 7) / 8);
-    render_kernel<false><<<grid2, block, 0, st>>>(A);
+    const dim3 grid2((W + 15) / 16, (H + 7) / 8);
+    if (A.lb < 10) render_kernel<false, false><<<grid2, 128, 0, st>>>(A);
+    else render_kernel<false, true><<<grid2, 128, 0, st>>>(A);
     return cudaGetLastError();
 }
 
@@ -476,8 +575,9 @@ cudaError_t launch_render_rgba(const csv_camera& cam, uint32_t W, uint32_t H, fl
     A.ambient = ambient;
     A.diffuse = diffuse;
     A.out_rgba = out_rgba;
-    dim3 block(16, 8), grid2((W + 15) / 16, (H + 7) / 8);
-    render_kernel<true><<<grid2, block, 0, st>>>(A);
+    const dim3 grid2((W + 15) / 16, (H + 7) / 8);
+    if (A.lb < 10) render_kernel<true, false><<<grid2, 128, 0, st>>>(A);
+    else render_kernel<true, true><<<grid2, 128, 0, st>>>(A);
     return cudaGetLastError();
 }
 
