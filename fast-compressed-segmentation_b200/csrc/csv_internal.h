@@ -201,17 +201,34 @@ cudaError_t launch_render_rgba(const csv_camera& cam, uint32_t W, uint32_t H, fl
                                const uint64_t* tf_keys, const uint32_t* tf_rgba, uint32_t n_tf, const float* light,
                                float ambient, float diffuse, uint32_t* out_rgba, uint32_t* requests, cudaStream_t st);
 
-size_t gemm_smem_bytes();
-// B [N][K] bf16 -> the tensor cores' no-swizzle K-major core-matrix tiling (K-chunks of 64).
-cudaError_t launch_tile_b(const __nv_bfloat16* B, uint32_t N, uint32_t K, __nv_bfloat16* T, cudaStream_t st);
 // The selector network's forward pass fused in one persistent kernel (mlp.cu): features [count][32]
 // -> logits [count][32] and/or sel (argmax of logits 0..11 | argmax of logits 12..27 << 4).
 cudaError_t launch_mlp_infer(const float* feat, uint32_t count, const __nv_bfloat16* W1t, const __nv_bfloat16* W2t,
                              const __nv_bfloat16* W3t, const float* b1, const float* b2, const float* b3, float* logits,
                              uint8_t* sel, uint32_t* err, int device, cudaStream_t st);
-cudaError_t launch_gemm_bf16(const __nv_bfloat16* A, const __nv_bfloat16* B, uint32_t M, uint32_t N, uint32_t K,
-                             const float* bias, const __nv_bfloat16* mask, uint32_t relu, float* C,
-                             __nv_bfloat16* Cb, __nv_bfloat16* CbT, float* CT, uint32_t* err, cudaStream_t st);
+// C = epilogue(A . B^T) on the tensor cores (csv_gemm_bf16), or with `label` the loss of 32 logits.
+struct GemmArgs {
+    const __nv_bfloat16* A = nullptr;  // [M][K]
+    const __nv_bfloat16* B = nullptr;  // [N][K]
+    uint32_t M = 0, N = 0, K = 0;      // M % 128 == 0, N % 16 == 0, K % 64 == 0
+    // K per CTA (a multiple of 64): below K, split s writes its partial product at C or CT + s M N,
+    // and no other output is set
+    uint32_t k_split = 0;
+    const float* bias = nullptr;          // [N] or null
+    const __nv_bfloat16* mask = nullptr;  // [M][N] or null: multiply by (mask > 0), the ReLU gradient
+    uint32_t relu = 0;                    // max(0, .) after the bias
+    float* C = nullptr;                   // [M][N] or null
+    __nv_bfloat16* Cb = nullptr;          // [M][N] or null
+    __nv_bfloat16* CbT = nullptr;         // [N][M] or null
+    float* CT = nullptr;                  // [N][M] or null
+    uint32_t* err = nullptr;              // set to 1 when a wait gives up
+    // not null (N = 32): Cb [M][64] and CbT [32][M] get the gradient of the mean cross-entropy of the first
+    // n_rows rows against these labels (mode | table << 4), *loss the loss added to it
+    const uint8_t* label = nullptr;
+    uint32_t n_rows = 0;
+    float* loss = nullptr;
+};
+cudaError_t launch_gemm_bf16(const GemmArgs& g, cudaStream_t st, const GemmArgs* second = nullptr);
 
 cudaError_t synth_volume(uint64_t* d_vol, uint32_t W, uint32_t H, uint32_t D, int kind, uint32_t n_cells,
                          uint32_t n_tubes, float r_min, float r_max, float zero_frac, uint64_t seed,

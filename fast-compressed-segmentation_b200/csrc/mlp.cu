@@ -6,15 +6,18 @@
 // in tensor memory, and an epilogue that adds a bias, applies ReLU or the ReLU
 // gradient mask, and writes fp32 and/or bf16, plain or transposed.
 //
-// Per CTA: one 128 x N tile (N <= 256, a multiple of 16), 128 threads.  K runs
-// in chunks of 64: the four warps copy the A and B chunks into shared memory in
-// the canonical no-swizzle K-major layout (8-row x 16-byte core matrices; core
-// matrix (row group g, column group c) at (g * 8 + c) * 128 bytes, so the
-// K-adjacent core matrices are 128 bytes apart and the row-adjacent ones 1024),
-// one thread issues four tcgen05.mma (M=128, N, K=16) with the accumulator in
-// tensor memory and commits them to an mbarrier, and all threads wait for it
-// (bounded) before the next chunk.  The epilogue reads the accumulator with
-// tcgen05.ld (warp w owns lanes 32w..32w+31 = rows) and applies the fused ops.
+// Per CTA: one 128 x N tile (N <= 64, a multiple of 16), 128 threads.  The selector's
+// layers are small (2048 x 256 x 256 at the training batch), so tiles are narrow, to
+// spread over the SMs, and a CTA has up to 256 of K in flight at once: the four warps
+// copy the A and B chunks of 64 into shared memory with cp.async, in the canonical
+// no-swizzle K-major layout (8-row x 16-byte core matrices; core matrix (row group g,
+// column group c) at (g * 8 + c) * 128 bytes, so the K-adjacent core matrices are 128
+// bytes apart and the row-adjacent ones 1024), one thread issues four tcgen05.mma (M=128,
+// N, K=16) per chunk with the accumulator in tensor memory and commits them to an
+// mbarrier, and all threads wait for it (bounded) before the next 256.  The epilogue
+// reads the accumulator with tcgen05.ld (warp w owns lanes 32w..32w+31 = rows) and
+// applies the fused ops.  A product whose K is the batch is split along K over CTAs;
+// their fp32 partial products are summed in order by the caller's reduction.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -28,23 +31,11 @@ namespace {
 
 constexpr uint32_t kGemmThreads = 128;
 constexpr uint32_t kKChunk = 64;               // bf16 elements per row per chunk (128 bytes)
+constexpr uint32_t kTileN = 64;                // columns per CTA
+constexpr uint32_t kKBlock = 256;              // K in flight
 constexpr uint32_t kTileA = 128 * kKChunk * 2; // 16 KB
-constexpr uint32_t kTileBMax = 256 * kKChunk * 2;  // 32 KB
+constexpr uint32_t kTileB = kTileN * kKChunk * 2;  // 8 KB
 constexpr uint32_t kWaitLimit = 1u << 24;
-
-struct GemmArgs {
-    const __nv_bfloat16* A;
-    const __nv_bfloat16* B;
-    uint32_t M, N, K;
-    const float* bias;            // [N] or null
-    const __nv_bfloat16* mask;    // [M][N] or null: multiply by (mask > 0), the ReLU gradient
-    uint32_t relu;                // max(0, .) after the bias
-    float* C;                     // [M][N] or null
-    __nv_bfloat16* Cb;            // [M][N] or null
-    __nv_bfloat16* CbT;           // [N][M] or null
-    float* CT;                    // [N][M] or null
-    uint32_t* err;                // set to 1 when a wait gives up
-};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -74,21 +65,91 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return false;
 }
 
-__global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rn(a));
+    const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16_rn(b));
+    return lo | (hi << 16);
+}
+
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Rows [r0, r0 + n) of a K-major operand, K elements [k0, k0 + 64 chunks), into core
+// matrices (n a multiple of 8).  Eight lanes read 32 bytes of four rows each.
+__device__ __forceinline__ void load_operand(uint32_t dst, uint32_t tile, const __nv_bfloat16* src, uint32_t K,
+                                             uint32_t r0, uint32_t n, uint32_t k0, uint32_t chunks) {
+    for (uint32_t c = 0; c < chunks; ++c)
+        for (uint32_t u = threadIdx.x; u < n * 8u; u += kGemmThreads) {
+            const uint32_t r = ((u >> 1) & 7u) + 8 * (u >> 6), kb = (u & 1u) | ((u >> 3) & 6u);
+            cp_async16(dst + c * tile + ((r >> 3) * 8 + kb) * 128 + (r & 7u) * 16,
+                       src + (size_t)(r0 + r) * K + k0 + c * kKChunk + kb * 8);
+        }
+}
+
+// Softmax cross-entropy of the mode head (logits 0..11) and the table head (12..27) of one
+// row against its label: g = (softmax - onehot) / n; returns the row's loss / n.
+__device__ __forceinline__ float loss_grad_row(const float (&z)[32], uint32_t label, uint32_t n, float (&g)[32]) {
+    float l = 0.0f;
+#pragma unroll
+    for (int head = 0; head < 2; ++head) {
+        constexpr int first[2] = {0, 12}, cnt[2] = {12, 16};
+        const int y = head ? label >> 4 : label & 15u;
+        float mx = -INFINITY;
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (k < cnt[head]) mx = fmaxf(mx, z[first[head] + k]);
+        float se = 0.0f, zy = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            if (k < cnt[head]) {
+                g[first[head] + k] = expf(z[first[head] + k] - mx);
+                se += g[first[head] + k];
+            }
+            if (k == y) zy = z[first[head] + k];
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (k < cnt[head]) g[first[head] + k] = (g[first[head] + k] / se - (k == y ? 1.0f : 0.0f)) / (float)n;
+        l += logf(se) + mx - zy;
+    }
+    return l / (float)n;
+}
+
+// Up to two products in one launch: the first n_first blocks are the first one's.
+// Bound by latency: a layer of the training batch is a few tiles of work.  Measured (B200,
+// a gradient step of 2048 rows; 128 x 256 tiles whose 64-wide chunks were loaded and
+// multiplied in turn, products over the rows on 2 CTAs, bias sums by one block each): 0.87
+// -> 0.072 ms of kernels (0.7 us at the bf16 rate); a 2048 x 256 x 256 layer 74 -> 11 us,
+// the 256 x 256 product over the rows 171 -> 12 us beside the next layer's.
+__global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, GemmArgs G1, uint32_t n_first) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sA = smem;                  // 16 KB
-    uint8_t* sB = smem + kTileA;         // up to 32 KB
+    uint8_t* sA = smem;                                // 4 x 16 KB
+    uint8_t* sB = smem + kTileA * (kKBlock / kKChunk);  // 4 x 8 KB
     __shared__ uint64_t bar;
     __shared__ uint32_t tmem_base;
-    __shared__ uint32_t failed;
+    const bool second = blockIdx.x >= n_first;
+    const GemmArgs& G = second ? G1 : G0;
+    const uint32_t blk = second ? blockIdx.x - n_first : blockIdx.x;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t m0 = blockIdx.x * 128u, n0 = blockIdx.y * 256u;
-    const uint32_t N = min(256u, G.N - n0);
-    uint32_t ncols = 32;
-    while (ncols < N) ncols <<= 1;
+    const uint32_t mt = G.M / 128u, nt = (G.N + kTileN - 1) / kTileN;
+    const uint32_t m0 = (blk % mt) * 128u, n0 = (blk / mt % nt) * kTileN, split = blk / (mt * nt);
+    const uint32_t N = min(kTileN, G.N - n0);
+    const uint32_t ncols = N <= 32 ? 32u : 64u;
+    const uint32_t ka = split * G.k_split, ke = min(G.K, ka + G.k_split);
     if (tid == 0) {
         mbar_init(smem_u32(&bar), 1);
-        failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -103,77 +164,123 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G) {
     const uint32_t tmem = tmem_base;
     // M = 128, N, bf16 x bf16 -> f32, both operands K-major
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
-    const uint32_t nchunks = G.K / kKChunk;
     uint32_t parity = 0;
-    for (uint32_t c = 0; c < nchunks; ++c) {
-        const uint32_t k0 = c * kKChunk;
-        // A: 128 rows x 8 units of 16 bytes
-        for (uint32_t u = tid; u < 128u * 8u; u += kGemmThreads) {
-            const uint32_t r = u >> 3, kb = u & 7u;
-            const uint4 v = *reinterpret_cast<const uint4*>(G.A + (size_t)(m0 + r) * G.K + k0 + kb * 8);
-            *reinterpret_cast<uint4*>(sA + ((r >> 3) * 8 + kb) * 128 + (r & 7u) * 16) = v;
-        }
-        for (uint32_t u = tid; u < N * 8u; u += kGemmThreads) {
-            const uint32_t r = u >> 3, kb = u & 7u;
-            const uint4 v = *reinterpret_cast<const uint4*>(G.B + (size_t)(n0 + r) * G.K + k0 + kb * 8);
-            *reinterpret_cast<uint4*>(sB + ((r >> 3) * 8 + kb) * 128 + (r & 7u) * 16) = v;
-        }
+    bool ok = true;
+    for (uint32_t k0 = ka; k0 < ke && ok; k0 += kKBlock) {
+        const uint32_t chunks = min(kKBlock, ke - k0) / kKChunk;
+        load_operand(smem_u32(sA), kTileA, G.A, G.K, m0, 128u, k0, chunks);
+        load_operand(smem_u32(sB), kTileB, G.B, G.K, n0, N, k0, chunks);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (tid == 0 && !failed) {
+        if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (uint32_t c = 0; c < chunks; ++c)
 #pragma unroll
-            for (uint32_t s = 0; s < kKChunk / 16; ++s) {
-                const uint64_t ad = smem_desc(smem_u32(sA) + s * 256u);
-                const uint64_t bd = smem_desc(smem_u32(sB) + s * 256u);
-                const uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-                    : "memory");
-            }
+                for (uint32_t s = 0; s < kKChunk / 16; ++s) {
+                    const uint64_t ad = smem_desc(smem_u32(sA) + c * kTileA + s * 256u);
+                    const uint64_t bd = smem_desc(smem_u32(sB) + c * kTileB + s * 256u);
+                    const uint32_t acc = (k0 > ka || c > 0 || s > 0) ? 1u : 0u;
+                    asm volatile(
+                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+                        "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+                        : "memory");
+                }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                              smem_u32(&bar))
                          : "memory");
         }
-        if (!failed) {
-            if (!mbar_wait(smem_u32(&bar), parity)) {
-                failed = 1;
-                if (G.err) atomicExch(G.err, 1u);
-            }
-        }
+        // one decision for the whole block; the operands' shared memory is free again
+        ok = __syncthreads_and(mbar_wait(smem_u32(&bar), parity)) != 0;
         parity ^= 1u;
-        __syncthreads();  // the chunk's shared memory is free again
     }
+    if (!ok && tid == 0 && G.err) atomicExch(G.err, 1u);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!failed) {
-        const uint32_t row = m0 + warp * 32u + lane;
+    const uint32_t row = m0 + warp * 32u + lane, taddr = tmem + ((warp * 32u) << 16);
+    if (ok && G.label) {  // the logits (N = 32): the loss and its gradient
+        float z[32], g[32];
+        uint32_t v[32];
+        tmem_ld16(taddr, v);
+        tmem_ld16(taddr + 16, v + 16);
+#pragma unroll
+        for (uint32_t j = 0; j < 32; ++j) {
+            z[j] = __uint_as_float(v[j]) + G.bias[j];
+            g[j] = 0.0f;
+        }
+        float l = 0.0f;
+        if (row < G.n_rows) l = loss_grad_row(z, G.label[row], G.n_rows, g);
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+        if (lane == 0) atomicAdd(G.loss, l);
+        // dZ [rows][64], zero beyond the logits, and its transpose [32][rows]
+        uint4* dst = reinterpret_cast<uint4*>(G.Cb + (size_t)row * 64);
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+            dst[q] = make_uint4(pack_bf16(g[8 * q], g[8 * q + 1]), pack_bf16(g[8 * q + 2], g[8 * q + 3]),
+                                pack_bf16(g[8 * q + 4], g[8 * q + 5]), pack_bf16(g[8 * q + 6], g[8 * q + 7]));
+#pragma unroll
+        for (uint32_t q = 4; q < 8; ++q) dst[q] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (uint32_t j = 0; j < 32; ++j) G.CbT[(size_t)j * G.M + row] = __float2bfloat16_rn(g[j]);
+    } else if (ok) {
+        float* C = G.C ? G.C + (size_t)split * G.M * G.N : nullptr;
+        float* CT = G.CT ? G.CT + (size_t)split * G.M * G.N : nullptr;
+        // (rows of N = 16 k values: 16-byte pieces when the arrays start on one)
+        const bool vec_c = aligned16(C), vec_cb = aligned16(G.Cb), vec_mask = aligned16(G.mask);
         for (uint32_t j0 = 0; j0 < N; j0 += 16) {
             uint32_t v[16];
-            const uint32_t taddr = tmem + ((warp * 32u) << 16) + j0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                "[%16];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                  "=r"(v[15])
-                : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row < G.M) {
+            tmem_ld16(taddr + j0, v);
+            const size_t at = (size_t)row * G.N + n0 + j0;
+            float x[16];
 #pragma unroll
-                for (uint32_t j = 0; j < 16; ++j) {
-                    const uint32_t n = n0 + j0 + j;
-                    float x = __uint_as_float(v[j]);
-                    if (G.bias) x += G.bias[n];
-                    if (G.relu) x = fmaxf(x, 0.0f);
-                    if (G.mask && !(__bfloat162float(G.mask[(size_t)row * G.N + n]) > 0.0f)) x = 0.0f;
-                    if (G.C) G.C[(size_t)row * G.N + n] = x;
-                    if (G.Cb) G.Cb[(size_t)row * G.N + n] = __float2bfloat16_rn(x);
-                    if (G.CbT) G.CbT[(size_t)n * G.M + row] = __float2bfloat16_rn(x);
-                    if (G.CT) G.CT[(size_t)n * G.M + row] = x;
+            for (uint32_t j = 0; j < 16; ++j) {
+                x[j] = __uint_as_float(v[j]);
+                if (G.bias) x[j] += G.bias[n0 + j0 + j];
+                if (G.relu) x[j] = fmaxf(x[j], 0.0f);
+            }
+            if (G.mask) {
+                __nv_bfloat16 m[16];
+                if (vec_mask) {
+                    reinterpret_cast<uint4*>(m)[0] = reinterpret_cast<const uint4*>(G.mask + at)[0];
+                    reinterpret_cast<uint4*>(m)[1] = reinterpret_cast<const uint4*>(G.mask + at)[1];
+                } else {
+#pragma unroll
+                    for (uint32_t j = 0; j < 16; ++j) m[j] = G.mask[at + j];
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j)
+                    if (!(__bfloat162float(m[j]) > 0.0f)) x[j] = 0.0f;
+            }
+            if (C) {
+                if (vec_c) {
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q)
+                        reinterpret_cast<float4*>(C + at)[q] =
+                            make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+                } else {
+#pragma unroll
+                    for (uint32_t j = 0; j < 16; ++j) C[at + j] = x[j];
                 }
             }
+            if (G.Cb) {
+                if (vec_cb) {
+#pragma unroll
+                    for (uint32_t q = 0; q < 2; ++q)
+                        reinterpret_cast<uint4*>(G.Cb + at)[q] =
+                            make_uint4(pack_bf16(x[8 * q], x[8 * q + 1]), pack_bf16(x[8 * q + 2], x[8 * q + 3]),
+                                       pack_bf16(x[8 * q + 4], x[8 * q + 5]), pack_bf16(x[8 * q + 6], x[8 * q + 7]));
+                } else {
+#pragma unroll
+                    for (uint32_t j = 0; j < 16; ++j) G.Cb[at + j] = __float2bfloat16_rn(x[j]);
+                }
+            }
+            if (G.CbT)
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j)
+                    G.CbT[(size_t)(n0 + j0 + j) * G.M + row] = __float2bfloat16_rn(x[j]);
+            if (CT)
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j) CT[(size_t)(n0 + j0 + j) * G.M + row] = x[j];
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -194,7 +301,8 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G) {
 // The MMAs are the ones the layer-by-layer GEMMs issue (same shapes, same K
 // order), so the logits are those of gemm_bf16_kernel's three launches.
 // Weights come pre-tiled in the no-swizzle K-major core-matrix layout, so that
-// each K-chunk is one contiguous bulk copy (tile_b_kernel).
+// each K-chunk is one contiguous bulk copy: K-chunks of 64, each N/8 x 8 core matrices
+// of 8 rows x 16 bytes, core (g, c) at (g * 8 + c) * 128 bytes.
 constexpr uint32_t kInferThreads = 128;
 constexpr uint32_t kHidN = 256, kInN = 64, kOutN = 32;
 constexpr uint32_t kSelModes = 12, kSelTables = 16;  // the two heads: logits 0..11 and 12..27
@@ -239,24 +347,9 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 // (row r, K element k) of a 128-row A operand held as 64-wide K-chunks of core matrices
 __device__ __forceinline__ uint32_t a_off(uint32_t r, uint32_t k) {
     return (k >> 6) * kChunkH + (((r >> 3) * 8 + ((k & 63) >> 3)) * 128) + (r & 7) * 16 + (k & 7) * 2;
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-    const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rn(a));
-    const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16_rn(b));
-    return lo | (hi << 16);
 }
 
 // acc (TMEM, this warp's 32 rows, 256 columns from col0) + bias, ReLU, bf16 -> the A operand in shared memory
@@ -476,24 +569,8 @@ __global__ void __launch_bounds__(kInferThreads, 1) mlp_infer_kernel(InferArgs G
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
-// B [N][K] row-major bf16 -> the tiled layout: K-chunks of 64, each N/8 x 8 core
-// matrices of 8 rows x 16 bytes, core (g, c) at (g * 8 + c) * 128 bytes.
-__global__ void tile_b_kernel(const __nv_bfloat16* __restrict__ B, uint32_t N, uint32_t K, __nv_bfloat16* __restrict__ T) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N * K) return;
-    const uint32_t n = i / K, k = i % K;
-    T[(size_t)(k >> 6) * N * 64 + ((n >> 3) * 8 + ((k & 63) >> 3)) * 64 + (n & 7) * 8 + (k & 7)] = B[i];
-}
-
 }  // namespace
 
-size_t gemm_smem_bytes() { return kTileA + kTileBMax; }
-
-cudaError_t launch_tile_b(const __nv_bfloat16* B, uint32_t N, uint32_t K, __nv_bfloat16* T, cudaStream_t st) {
-    if (N % 8 || K % 64) return cudaErrorInvalidValue;
-    tile_b_kernel<<<(N * K + 255) / 256, 256, 0, st>>>(B, N, K, T);
-    return cudaGetLastError();
-}
 
 cudaError_t launch_mlp_infer(const float* feat, uint32_t count, const __nv_bfloat16* W1t, const __nv_bfloat16* W2t,
                              const __nv_bfloat16* W3t, const float* b1, const float* b2, const float* b3, float* logits,
@@ -526,34 +603,24 @@ cudaError_t launch_mlp_infer(const float* feat, uint32_t count, const __nv_bfloa
     return cudaGetLastError();
 }
 
-cudaError_t launch_gemm_bf16(const __nv_bfloat16* A, const __nv_bfloat16* B, uint32_t M, uint32_t N, uint32_t K,
-                             const float* bias, const __nv_bfloat16* mask, uint32_t relu, float* C,
-                             __nv_bfloat16* Cb, __nv_bfloat16* CbT, float* CT, uint32_t* err, cudaStream_t st) {
-    if (M == 0 || N == 0 || K == 0) return cudaSuccess;
-    if (M % 128 || N % 16 || K % kKChunk) return cudaErrorInvalidValue;
+static uint32_t gemm_blocks(const GemmArgs& g) {
+    return g.M / 128 * ((g.N + kTileN - 1) / kTileN) * ((g.K + g.k_split - 1) / g.k_split);
+}
+
+cudaError_t launch_gemm_bf16(const GemmArgs& g, cudaStream_t st, const GemmArgs* second) {
+    if (g.M == 0 || g.N == 0 || g.K == 0) return cudaSuccess;
+    for (const GemmArgs* p : {&g, second})
+        if (p && (p->M % 128 || p->N % 16 || p->K % kKChunk || p->k_split == 0 || p->k_split % kKChunk))
+            return cudaErrorInvalidValue;
+    constexpr int smem = (int)((kTileA + kTileB) * (kKBlock / kKChunk));
     static bool attr = false;
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)gemm_smem_bytes());
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    GemmArgs G;
-    G.A = A;
-    G.B = B;
-    G.M = M;
-    G.N = N;
-    G.K = K;
-    G.bias = bias;
-    G.mask = mask;
-    G.relu = relu;
-    G.C = C;
-    G.Cb = Cb;
-    G.CbT = CbT;
-    G.CT = CT;
-    G.err = err;
-    dim3 grid(M / 128, (N + 255) / 256);
-    gemm_bf16_kernel<<<grid, kGemmThreads, gemm_smem_bytes(), st>>>(G);
+    const uint32_t n = gemm_blocks(g);
+    gemm_bf16_kernel<<<n + (second ? gemm_blocks(*second) : 0u), kGemmThreads, smem, st>>>(g, second ? *second : g, n);
     return cudaGetLastError();
 }
 
@@ -569,9 +636,21 @@ extern "C" int csv_gemm_bf16(csv_ctx* ctx, const void* d_A, const void* d_B, uin
     if (!ctx || !d_A || !d_B) return CSV_EINVAL;
     if (M % 128 || N % 16 || K % 64) return abi_fail(ctx, CSV_EINVAL, "gemm: M % 128, N % 16 and K % 64 must be 0");
     DeviceGuard g(ctx->device);
-    cudaError_t e = launch_gemm_bf16((const __nv_bfloat16*)d_A, (const __nv_bfloat16*)d_B, M, N, K, d_bias,
-                                     (const __nv_bfloat16*)d_mask, relu, d_C, (__nv_bfloat16*)d_Cb,
-                                     (__nv_bfloat16*)d_CbT, d_CT, d_err, (cudaStream_t)stream);
+    GemmArgs G;
+    G.A = (const __nv_bfloat16*)d_A;
+    G.B = (const __nv_bfloat16*)d_B;
+    G.M = M;
+    G.N = N;
+    G.K = G.k_split = K;
+    G.bias = d_bias;
+    G.mask = (const __nv_bfloat16*)d_mask;
+    G.relu = relu;
+    G.C = d_C;
+    G.Cb = (__nv_bfloat16*)d_Cb;
+    G.CbT = (__nv_bfloat16*)d_CbT;
+    G.CT = d_CT;
+    G.err = d_err;
+    cudaError_t e = launch_gemm_bf16(G, (cudaStream_t)stream);
     if (e != cudaSuccess) return abi_cuda_fail(ctx, e, "gemm");
     return CSV_OK;
 }

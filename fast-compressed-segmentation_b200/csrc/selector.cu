@@ -377,82 +377,100 @@ __global__ void pack_input_kernel(const float* __restrict__ feat, uint32_t n, ui
     XT[(size_t)c * rows + r] = b;
 }
 
-// Softmax cross-entropy of the mode head (logits 0..11) and the table head
-// (12..27) against the labels; dZ = (softmax - onehot) / n as bf16 (rows x 64,
-// zero beyond column 27 and row n) and its transpose (32 x rows).
-__global__ void loss_grad_kernel(const float* __restrict__ Z, const uint8_t* __restrict__ label, uint32_t n,
-                                 uint32_t rows, __nv_bfloat16* __restrict__ dZ, __nv_bfloat16* __restrict__ dZT,
-                                 float* __restrict__ loss) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    float g[kOut];
-    for (uint32_t k = 0; k < kOut; ++k) g[k] = 0.0f;
-    if (r < n) {
-        const float* z = Z + (size_t)r * kOut;
-        const uint32_t lm = label[r] & 15u, lt = label[r] >> 4;
-        float l = 0.0f;
-        for (int head = 0; head < 2; ++head) {
-            const uint32_t b0 = head ? kModesN : 0, cnt = head ? kTablesN : kModesN, y = head ? lt : lm;
-            float mx = -INFINITY;
-            for (uint32_t k = 0; k < cnt; ++k) mx = fmaxf(mx, z[b0 + k]);
-            float se = 0.0f;
-            for (uint32_t k = 0; k < cnt; ++k) se += expf(z[b0 + k] - mx);
-            for (uint32_t k = 0; k < cnt; ++k)
-                g[b0 + k] = (expf(z[b0 + k] - mx) / se - (k == y ? 1.0f : 0.0f)) / (float)n;
-            l += logf(se) + mx - z[b0 + y];
-        }
-        atomicAdd(loss, l / (float)n);
-    }
-    for (uint32_t k = 0; k < kOutPad; ++k) {
-        const __nv_bfloat16 v = __float2bfloat16_rn(k < kOut ? g[k] : 0.0f);
-        dZ[(size_t)r * kOutPad + k] = v;
-        if (k < kOut) dZT[(size_t)k * rows + r] = v;
-    }
-}
-
-// Column sums of a bf16 [rows][N] matrix (row stride ld) into out[N] (fp32): the bias gradients.
-__global__ void colsum_kernel(const __nv_bfloat16* __restrict__ M, uint32_t rows, uint32_t N, uint32_t ld,
-                              float* __restrict__ out) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
+// Partial column sums of dZ (32 columns of 64), dH2 and dH1 (256), the bias gradients:
+// block (part, matrix), a thread per column, over `per` rows each.
+__global__ void __launch_bounds__(256) colsum_kernel(const __nv_bfloat16* __restrict__ dZ,
+                                                     const __nv_bfloat16* __restrict__ dH2,
+                                                     const __nv_bfloat16* __restrict__ dH1, uint32_t rows, uint32_t per,
+                                                     float* __restrict__ out) {
+    const uint32_t c = threadIdx.x, which = blockIdx.y;
+    if (which == 0 && c >= kOut) return;
+    const __nv_bfloat16* m = which == 0 ? dZ : (which == 1 ? dH2 : dH1);
+    const uint32_t ld = which == 0 ? kOutPad : kHid, r1 = min(rows, (blockIdx.x + 1) * per);
     float s = 0.0f;
-    for (uint32_t r = 0; r < rows; ++r) s += __bfloat162float(M[(size_t)r * ld + c]);
-    out[c] = s;
+#pragma unroll 8
+    for (uint32_t r = blockIdx.x * per; r < r1; ++r) s += __bfloat162float(m[(size_t)r * ld + c]);
+    out[((size_t)which * gridDim.x + blockIdx.x) * kHid + c] = s;
 }
 
-// Adam (Kingma & Ba 2015) on the fp32 parameters.
+// The gradients from their partial sums, in order.  part: `splits` products dW1 [256][64],
+// then dW2 [256][256], then dW3^T stored as W3 lies [32][256]; bias: colsum_kernel's.
+__global__ void __launch_bounds__(256) grad_sum_kernel(const float* __restrict__ part, uint32_t splits,
+                                                       const float* __restrict__ bias, uint32_t bias_parts,
+                                                       float* __restrict__ G) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= N_PARAMS) return;
+    const float* p;
+    uint32_t n = splits, stride;
+    if (k < OFF_B1) {
+        p = part + k;
+        stride = kHid * kFeatPad;
+    } else if (k >= OFF_W2 && k < OFF_B2) {
+        p = part + (size_t)splits * (kHid * kFeatPad) + (k - OFF_W2);
+        stride = kHid * kHid;
+    } else if (k >= OFF_W3 && k < OFF_B3) {
+        p = part + (size_t)splits * (kHid * kFeatPad + kHid * kHid) + (k - OFF_W3);
+        stride = kOut * kHid;
+    } else {
+        const uint32_t which = k >= OFF_B3 ? 0u : (k >= OFF_B2 ? 1u : 2u);
+        p = bias + (size_t)which * bias_parts * kHid + (k - (which == 0 ? OFF_B3 : (which == 1 ? OFF_B2 : OFF_B1)));
+        stride = kHid;
+        n = bias_parts;
+    }
+    float s = 0.0f;
+#pragma unroll 8
+    for (uint32_t i = 0; i < n; ++i) s += p[(size_t)i * stride];
+    G[k] = s;
+}
+
+// A weight's bf16 copies: W1b [256][64], W2b [256][256] and its transpose, W3b [32][256] and its
+// transpose [256][64] (columns >= 32 zero), and each layer tiled for the fused forward.
+struct WeightCopies {
+    __nv_bfloat16 *W1b, *W2b, *W2bT, *W3b, *W3bT, *W1t, *W2t, *W3t;
+};
+__device__ __forceinline__ uint32_t tiled_at(uint32_t N, uint32_t n, uint32_t k) {  // the fused forward's layout
+    return (k >> 6) * N * 64 + ((n >> 3) * 8 + ((k & 63u) >> 3)) * 64 + (n & 7u) * 8 + (k & 7u);
+}
+__device__ __forceinline__ void put_weight(const WeightCopies& C, uint32_t k, float v) {
+    const __nv_bfloat16 w = __float2bfloat16_rn(v);
+    if (k < OFF_B1) {
+        C.W1b[k] = w;
+        C.W1t[tiled_at(kHid, k / kFeatPad, k % kFeatPad)] = w;
+    } else if (k >= OFF_W2 && k < OFF_B2) {
+        const uint32_t i = k - OFF_W2, o = i / kHid, in = i % kHid;
+        C.W2b[i] = w;
+        C.W2bT[(size_t)in * kHid + o] = w;
+        C.W2t[tiled_at(kHid, o, in)] = w;
+    } else if (k >= OFF_W3 && k < OFF_B3) {
+        const uint32_t i = k - OFF_W3, o = i / kHid, in = i % kHid;
+        C.W3b[i] = w;
+        C.W3bT[(size_t)in * kOutPad + o] = w;
+        C.W3t[tiled_at(kOut, o, in)] = w;
+    }
+}
+
+// Adam (Kingma & Ba 2015) on the fp32 parameters, and the weights' bf16 copies.
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                             float* __restrict__ v, uint32_t n, float lr, float b1, float b2, float eps, float c1,
-                            float c2) {
+                            float c2, WeightCopies C) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const float gk = g[k];
     const float mk = b1 * m[k] + (1.0f - b1) * gk, vk = b2 * v[k] + (1.0f - b2) * gk * gk;
     m[k] = mk;
     v[k] = vk;
-    p[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+    const float pk = p[k] - lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+    p[k] = pk;
+    put_weight(C, k, pk);
 }
 
-// bf16 weight copies: W1b [256][64], W2b [256][256], W2bT, W3b [32][256], W3bT [256][64] (columns >= 32 zero)
-__global__ void refresh_kernel(const float* __restrict__ P, __nv_bfloat16* W1b, __nv_bfloat16* W2b,
-                               __nv_bfloat16* W2bT, __nv_bfloat16* W3b, __nv_bfloat16* W3bT) {
+// The copies of given parameters.
+__global__ void refresh_kernel(const float* __restrict__ P, WeightCopies C) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < kHid * kFeatPad) W1b[k] = __float2bfloat16_rn(P[OFF_W1 + k]);
-    if (k < kHid * kHid) {
-        const uint32_t o = k / kHid, in = k % kHid;
-        const __nv_bfloat16 w = __float2bfloat16_rn(P[OFF_W2 + k]);
-        W2b[k] = w;
-        W2bT[(size_t)in * kHid + o] = w;
-    }
-    if (k < kOut * kHid) {
-        const uint32_t o = k / kHid, in = k % kHid;
-        const __nv_bfloat16 w = __float2bfloat16_rn(P[OFF_W3 + k]);
-        W3b[k] = w;
-        W3bT[(size_t)in * kOutPad + o] = w;
-    }
+    if (k < N_PARAMS) put_weight(C, k, P[k]);
     if (k < kHid * (kOutPad - kOut)) {
         const uint32_t in = k / (kOutPad - kOut), o = kOut + k % (kOutPad - kOut);
-        W3bT[(size_t)in * kOutPad + o] = __float2bfloat16_rn(0.0f);
+        C.W3bT[(size_t)in * kOutPad + o] = __float2bfloat16_rn(0.0f);
     }
 }
 
@@ -474,7 +492,8 @@ struct csv_mlp {
     __nv_bfloat16 *W1t = nullptr, *W2t = nullptr, *W3t = nullptr;  // tiled for the fused forward
     __nv_bfloat16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *H2 = nullptr, *H2T = nullptr;
     __nv_bfloat16 *dZ = nullptr, *dZT = nullptr, *dH2 = nullptr, *dH2T = nullptr, *dH1 = nullptr, *dH1T = nullptr;
-    float* Z = nullptr;
+    float* part = nullptr;       // the weight gradients' partial products
+    float* bias_part = nullptr;  // and the bias gradients' partial sums
     float* loss = nullptr;
     uint32_t* err = nullptr;
 };
@@ -484,12 +503,19 @@ namespace {
 void mlp_free_acts(csv_mlp* n) {
     for (void* p : {(void*)n->X, (void*)n->XT, (void*)n->H1, (void*)n->H1T, (void*)n->H2, (void*)n->H2T,
                     (void*)n->dZ, (void*)n->dZT, (void*)n->dH2, (void*)n->dH2T, (void*)n->dH1, (void*)n->dH1T,
-                    (void*)n->Z})
+                    (void*)n->part, (void*)n->bias_part})
         cudaFree(p);
     n->X = n->XT = n->H1 = n->H1T = n->H2 = n->H2T = n->dZ = n->dZT = n->dH2 = n->dH2T = n->dH1 = n->dH1T = nullptr;
-    n->Z = nullptr;
+    n->part = n->bias_part = nullptr;
     n->cap = 0;
 }
+
+// The weight gradients are products over the rows: split so that a CTA has 256 rows of
+// them (its operands in flight at once), and into no more than 32 partial products.
+uint32_t mlp_k_split(uint32_t rows) { return std::max(256u, (rows / 32 + 63) / 64 * 64); }
+uint32_t mlp_splits(uint32_t rows) { return (rows + mlp_k_split(rows) - 1) / mlp_k_split(rows); }
+uint32_t mlp_bias_rows(uint32_t rows) { return std::max(64u, (rows + 63) / 64); }  // per partial sum
+uint32_t mlp_bias_parts(uint32_t rows) { return (rows + mlp_bias_rows(rows) - 1) / mlp_bias_rows(rows); }
 
 cudaError_t mlp_reserve(csv_mlp* n, uint32_t rows) {
     if (rows <= n->cap) return cudaSuccess;
@@ -511,33 +537,54 @@ cudaError_t mlp_reserve(csv_mlp* n, uint32_t rows) {
     al((void**)&n->dH2T, r * kHid * 2);
     al((void**)&n->dH1, r * kHid * 2);
     al((void**)&n->dH1T, r * kHid * 2);
-    al((void**)&n->Z, r * kOut * 4);
+    // (as many partial results as any batch up to this one has)
+    al((void**)&n->part, std::min<size_t>(32, (rows + 255) / 256) * (kHid * kFeatPad + kHid * kHid + kOut * kHid) * 4);
+    al((void**)&n->bias_part, 3 * std::min<size_t>(64, (rows + 63) / 64) * kHid * 4);
     if (e == cudaSuccess) n->cap = rows;
     return e;
 }
 
-cudaError_t mlp_refresh(csv_mlp* n, cudaStream_t st) {
-    refresh_kernel<<<(kHid * kHid + 255) / 256, 256, 0, st>>>(n->P, n->W1b, n->W2b, n->W2bT, n->W3b, n->W3bT);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = launch_tile_b(n->W1b, kHid, kFeatPad, n->W1t, st);
-    if (e == cudaSuccess) e = launch_tile_b(n->W2b, kHid, kHid, n->W2t, st);
-    if (e == cudaSuccess) e = launch_tile_b(n->W3b, kOut, kHid, n->W3t, st);
-    return e;
+WeightCopies mlp_copies(const csv_mlp* n) {
+    return WeightCopies{n->W1b, n->W2b, n->W2bT, n->W3b, n->W3bT, n->W1t, n->W2t, n->W3t};
 }
 
-// Forward pass on `rows` (padded) rows of which `cnt` hold features; Z holds the logits.
-cudaError_t mlp_forward(csv_mlp* n, const float* feat, uint32_t cnt, uint32_t rows, cudaStream_t st) {
-    cudaError_t e;
+GemmArgs mlp_gemm(const csv_mlp* n, const __nv_bfloat16* A, const __nv_bfloat16* B, uint32_t M, uint32_t N, uint32_t K) {
+    GemmArgs g;
+    g.A = A;
+    g.B = B;
+    g.M = M;
+    g.N = N;
+    g.K = g.k_split = K;
+    g.err = n->err;
+    return g;
+}
+
+// Forward pass on `rows` (padded) rows of which `cnt` hold features, the loss, and dZ.
+cudaError_t mlp_forward(csv_mlp* n, const float* feat, const uint8_t* label, uint32_t cnt, uint32_t rows, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(n->loss, 0, 4, st);
+    if (e != cudaSuccess) return e;
     pack_input_kernel<<<(rows * kFeatPad + 255) / 256, 256, 0, st>>>(feat, cnt, rows, n->X, n->XT);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = launch_gemm_bf16(n->X, n->W1b, rows, kHid, kFeatPad, n->P + OFF_B1, nullptr, 1, nullptr, n->H1, n->H1T,
-                              nullptr, n->err, st)) != cudaSuccess)
-        return e;
-    if ((e = launch_gemm_bf16(n->H1, n->W2b, rows, kHid, kHid, n->P + OFF_B2, nullptr, 1, nullptr, n->H2, n->H2T,
-                              nullptr, n->err, st)) != cudaSuccess)
-        return e;
-    return launch_gemm_bf16(n->H2, n->W3b, rows, kOut, kHid, n->P + OFF_B3, nullptr, 0, n->Z, nullptr, nullptr,
-                            nullptr, n->err, st);
+    GemmArgs g = mlp_gemm(n, n->X, n->W1b, rows, kHid, kFeatPad);
+    g.bias = n->P + OFF_B1;
+    g.relu = 1;
+    g.Cb = n->H1;
+    g.CbT = n->H1T;
+    if ((e = launch_gemm_bf16(g, st)) != cudaSuccess) return e;
+    g = mlp_gemm(n, n->H1, n->W2b, rows, kHid, kHid);
+    g.bias = n->P + OFF_B2;
+    g.relu = 1;
+    g.Cb = n->H2;
+    g.CbT = n->H2T;
+    if ((e = launch_gemm_bf16(g, st)) != cudaSuccess) return e;
+    g = mlp_gemm(n, n->H2, n->W3b, rows, kOut, kHid);
+    g.bias = n->P + OFF_B3;
+    g.Cb = n->dZ;
+    g.CbT = n->dZT;
+    g.label = label;
+    g.n_rows = cnt;
+    g.loss = n->loss;
+    return launch_gemm_bf16(g, st);
 }
 
 }  // namespace
@@ -585,7 +632,10 @@ int csv_mlp_create(csv_ctx* ctx, const float* params, csv_mlp** out) {
     if (e == cudaSuccess) e = cudaMemset(n->Vm, 0, N_PARAMS * 4);
     if (e == cudaSuccess) e = cudaMemset(n->G, 0, N_PARAMS * 4);
     if (e == cudaSuccess) e = cudaMemset(n->err, 0, 4);
-    if (e == cudaSuccess) e = mlp_refresh(n, 0);
+    if (e == cudaSuccess) {
+        refresh_kernel<<<(N_PARAMS + 255) / 256, 256>>>(n->P, mlp_copies(n));
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         csv_mlp_destroy(n);
@@ -625,37 +675,43 @@ int csv_mlp_grad(csv_mlp* n, const float* d_feat, const uint8_t* d_label, uint32
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t rows = (count + 127) / 128 * 128;
     cudaError_t e = mlp_reserve(n, rows);
-    if (e == cudaSuccess) e = mlp_forward(n, d_feat, count, rows, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(n->loss, 0, 4, st);
+    if (e == cudaSuccess) e = mlp_forward(n, d_feat, d_label, count, rows, st);
+    const uint32_t ks = mlp_k_split(rows), splits = mlp_splits(rows), parts = mlp_bias_parts(rows);
+    float* p1 = n->part;
+    float* p2 = p1 + (size_t)splits * (kHid * kFeatPad);
+    float* p3 = p2 + (size_t)splits * (kHid * kHid);
+    // a product over the rows beside one over the units where both have their operands
+    auto over_rows = [&](const __nv_bfloat16* A, const __nv_bfloat16* B, uint32_t N) {
+        GemmArgs g = mlp_gemm(n, A, B, kHid, N, rows);
+        g.k_split = ks;
+        return g;
+    };
     if (e == cudaSuccess) {
-        loss_grad_kernel<<<(rows + 127) / 128, 128, 0, st>>>(n->Z, d_label, count, rows, n->dZ, n->dZT, n->loss);
-        e = cudaGetLastError();
+        GemmArgs w = over_rows(n->H2T, n->dZT, kOut);  // dW3^T = H2^T dZ, written as W3 lies
+        w.CT = p3;
+        GemmArgs h = mlp_gemm(n, n->dZ, n->W3bT, rows, kHid, kOutPad);  // dH2 = (dZ W3) * (H2 > 0)
+        h.mask = n->H2;
+        h.Cb = n->dH2;
+        h.CbT = n->dH2T;
+        e = launch_gemm_bf16(h, st, &w);
     }
-    float* G = n->G;
-    // dW3^T = H2^T dZ (M 256, N 32, K rows), written transposed into W3's slot
-    if (e == cudaSuccess)
-        e = launch_gemm_bf16(n->H2T, n->dZT, kHid, kOut, rows, nullptr, nullptr, 0, nullptr, nullptr, nullptr,
-                             G + OFF_W3, n->err, st);
-    // dH2 = (dZ W3) * (H2 > 0)
-    if (e == cudaSuccess)
-        e = launch_gemm_bf16(n->dZ, n->W3bT, rows, kHid, kOutPad, nullptr, n->H2, 0, nullptr, n->dH2, n->dH2T,
-                             nullptr, n->err, st);
-    // dW2 = dH2^T H1
-    if (e == cudaSuccess)
-        e = launch_gemm_bf16(n->dH2T, n->H1T, kHid, kHid, rows, nullptr, nullptr, 0, G + OFF_W2, nullptr, nullptr,
-                             nullptr, n->err, st);
-    // dH1 = (dH2 W2) * (H1 > 0)
-    if (e == cudaSuccess)
-        e = launch_gemm_bf16(n->dH2, n->W2bT, rows, kHid, kHid, nullptr, n->H1, 0, nullptr, n->dH1, n->dH1T,
-                             nullptr, n->err, st);
-    // dW1 = dH1^T X
-    if (e == cudaSuccess)
-        e = launch_gemm_bf16(n->dH1T, n->XT, kHid, kFeatPad, rows, nullptr, nullptr, 0, G + OFF_W1, nullptr,
-                             nullptr, nullptr, n->err, st);
     if (e == cudaSuccess) {
-        colsum_kernel<<<1, 256, 0, st>>>(n->dZ, rows, kOut, kOutPad, G + OFF_B3);
-        colsum_kernel<<<1, 256, 0, st>>>(n->dH2, rows, kHid, kHid, G + OFF_B2);
-        colsum_kernel<<<1, 256, 0, st>>>(n->dH1, rows, kHid, kHid, G + OFF_B1);
+        GemmArgs w = over_rows(n->dH2T, n->H1T, kHid);  // dW2 = dH2^T H1
+        w.C = p2;
+        GemmArgs h = mlp_gemm(n, n->dH2, n->W2bT, rows, kHid, kHid);  // dH1 = (dH2 W2) * (H1 > 0)
+        h.mask = n->H1;
+        h.Cb = n->dH1;
+        h.CbT = n->dH1T;
+        e = launch_gemm_bf16(h, st, &w);
+    }
+    if (e == cudaSuccess) {
+        GemmArgs w = over_rows(n->dH1T, n->XT, kFeatPad);  // dW1 = dH1^T X
+        w.C = p1;
+        e = launch_gemm_bf16(w, st);
+    }
+    if (e == cudaSuccess) {
+        colsum_kernel<<<dim3(parts, 3), 256, 0, st>>>(n->dZ, n->dH2, n->dH1, rows, mlp_bias_rows(rows), n->bias_part);
+        grad_sum_kernel<<<(N_PARAMS + 255) / 256, 256, 0, st>>>(n->part, splits, n->bias_part, parts, n->G);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && loss) {
@@ -673,9 +729,8 @@ int csv_mlp_adam(csv_mlp* n, float lr, float beta1, float beta2, float eps, void
     n->t += 1;
     const float c1 = 1.0f - powf(beta1, (float)n->t), c2 = 1.0f - powf(beta2, (float)n->t);
     adam_kernel<<<(N_PARAMS + 255) / 256, 256, 0, st>>>(n->P, n->G, n->Mm, n->Vm, N_PARAMS, lr, beta1, beta2, eps, c1,
-                                                         c2);
+                                                         c2, mlp_copies(n));
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = mlp_refresh(n, st);
     if (e != cudaSuccess) return abi_cuda_fail(n->ctx, e, "mlp adam");
     return CSV_OK;
 }
