@@ -206,14 +206,19 @@ cudaError_t launch_render_rgba(const csv_camera& cam, uint32_t W, uint32_t H, fl
 cudaError_t launch_mlp_infer(const float* feat, uint32_t count, const __nv_bfloat16* W1t, const __nv_bfloat16* W2t,
                              const __nv_bfloat16* W3t, const float* b1, const float* b2, const float* b3, float* logits,
                              uint8_t* sel, uint32_t* err, int device, cudaStream_t st);
+// Element (r, k) of an R x K bf16 operand in the tensor cores' no-swizzle K-major layout, as the
+// network's operands lie in global memory: K-chunks of 64, each of R / 8 x 8 core matrices of 8
+// rows x 16 bytes, so that consecutive rows of a chunk are one contiguous bulk copy.
+__host__ __device__ inline size_t tiled_at(uint32_t R, uint32_t r, uint32_t k) {
+    return (size_t)(k >> 6) * R * 64 + ((r >> 3) * 8 + ((k & 63u) >> 3)) * 64 + (r & 7u) * 8 + (k & 7u);
+}
 // C = epilogue(A . B^T) on the tensor cores (csv_gemm_bf16), or with `label` the loss of 32 logits.
 struct GemmArgs {
     const __nv_bfloat16* A = nullptr;  // [M][K]
     const __nv_bfloat16* B = nullptr;  // [N][K]
     uint32_t M = 0, N = 0, K = 0;      // M % 128 == 0, N % 16 == 0, K % 64 == 0
-    // K per CTA (a multiple of 64): below K, split s writes its partial product at C or CT + s M N,
-    // and no other output is set
-    uint32_t k_split = 0;
+    uint32_t tile_n = 64;              // columns per CTA, a multiple of 16 up to 64
+    bool tiled = false;                // A, B, mask, Cb and CbT are tiled (tiled_at), not row-major
     const float* bias = nullptr;          // [N] or null
     const __nv_bfloat16* mask = nullptr;  // [M][N] or null: multiply by (mask > 0), the ReLU gradient
     uint32_t relu = 0;                    // max(0, .) after the bias
@@ -222,7 +227,7 @@ struct GemmArgs {
     __nv_bfloat16* CbT = nullptr;         // [N][M] or null
     float* CT = nullptr;                  // [N][M] or null
     uint32_t* err = nullptr;              // set to 1 when a wait gives up
-    // not null (N = 32): Cb [M][64] and CbT [32][M] get the gradient of the mean cross-entropy of the first
+    // not null (N = 32, tiled): Cb [M][64] and CbT [32][M] get the gradient of the mean cross-entropy of the first
     // n_rows rows against these labels (mode | table << 4), *loss the loss added to it
     const uint8_t* label = nullptr;
     uint32_t n_rows = 0;

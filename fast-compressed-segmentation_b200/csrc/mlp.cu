@@ -8,16 +8,19 @@
 //
 // Per CTA: one 128 x N tile (N <= 64, a multiple of 16), 128 threads.  The selector's
 // layers are small (2048 x 256 x 256 at the training batch), so tiles are narrow, to
-// spread over the SMs, and a CTA has up to 256 of K in flight at once: the four warps
-// copy the A and B chunks of 64 into shared memory with cp.async, in the canonical
-// no-swizzle K-major layout (8-row x 16-byte core matrices; core matrix (row group g,
-// column group c) at (g * 8 + c) * 128 bytes, so the K-adjacent core matrices are 128
-// bytes apart and the row-adjacent ones 1024), one thread issues four tcgen05.mma (M=128,
-// N, K=16) per chunk with the accumulator in tensor memory and commits them to an
-// mbarrier, and all threads wait for it (bounded) before the next 256.  The epilogue
-// reads the accumulator with tcgen05.ld (warp w owns lanes 32w..32w+31 = rows) and
-// applies the fused ops.  A product whose K is the batch is split along K over CTAs;
-// their fp32 partial products are summed in order by the caller's reduction.
+// spread over the SMs.  K runs in chunks of 64 through four stages of shared memory in the
+// canonical no-swizzle K-major layout (8-row x 16-byte core matrices; core matrix (row
+// group g, column group c) at (g * 8 + c) * 128 bytes, so the K-adjacent core matrices are
+// 128 bytes apart and the row-adjacent ones 1024).  One thread issues four tcgen05.mma
+// (M=128, N, K=16) per chunk with the accumulator in tensor memory and commits them to the
+// stage's mbarrier.  The network's own operands lie in global memory in that layout, chunk
+// after chunk (tiled_at), so that the same thread fills a stage with one bulk copy per
+// operand and nothing else of the block takes part; row-major operands (csv_gemm_bf16) are
+// copied by all threads with cp.async, a block barrier per chunk.  (A product
+// over 2048 rows: 30 us row-major, 20 us tiled.)  The epilogue reads the accumulator
+// with tcgen05.ld (warp w owns lanes 32w..32w+31 = rows) and applies the fused ops.  An
+// output's products are added in the order of K whatever the tile, so results do not
+// depend on it.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -31,8 +34,8 @@ namespace {
 
 constexpr uint32_t kGemmThreads = 128;
 constexpr uint32_t kKChunk = 64;               // bf16 elements per row per chunk (128 bytes)
-constexpr uint32_t kTileN = 64;                // columns per CTA
-constexpr uint32_t kKBlock = 256;              // K in flight
+constexpr uint32_t kTileN = 64;                // columns per CTA at most
+constexpr uint32_t kStages = 4;
 constexpr uint32_t kTileA = 128 * kKChunk * 2; // 16 KB
 constexpr uint32_t kTileB = kTileN * kKChunk * 2;  // 8 KB
 constexpr uint32_t kWaitLimit = 1u << 24;
@@ -50,6 +53,27 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+
+__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void expect_bytes(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+        "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
@@ -86,16 +110,14 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// Rows [r0, r0 + n) of a K-major operand, K elements [k0, k0 + 64 chunks), into core
-// matrices (n a multiple of 8).  Eight lanes read 32 bytes of four rows each.
-__device__ __forceinline__ void load_operand(uint32_t dst, uint32_t tile, const __nv_bfloat16* src, uint32_t K,
-                                             uint32_t r0, uint32_t n, uint32_t k0, uint32_t chunks) {
-    for (uint32_t c = 0; c < chunks; ++c)
-        for (uint32_t u = threadIdx.x; u < n * 8u; u += kGemmThreads) {
-            const uint32_t r = ((u >> 1) & 7u) + 8 * (u >> 6), kb = (u & 1u) | ((u >> 3) & 6u);
-            cp_async16(dst + c * tile + ((r >> 3) * 8 + kb) * 128 + (r & 7u) * 16,
-                       src + (size_t)(r0 + r) * K + k0 + c * kKChunk + kb * 8);
-        }
+// Rows [r0, r0 + n) of a K-major operand, 64 K elements from k0 on, into core matrices (n
+// a multiple of 8).  Eight lanes read 32 bytes of four rows each.
+__device__ __forceinline__ void load_operand(uint32_t dst, const __nv_bfloat16* src, uint32_t K, uint32_t r0, uint32_t n,
+                                             uint32_t k0) {
+    for (uint32_t u = threadIdx.x; u < n * 8u; u += kGemmThreads) {
+        const uint32_t r = ((u >> 1) & 7u) + 8 * (u >> 6), kb = (u & 1u) | ((u >> 3) & 6u);
+        cp_async16(dst + ((r >> 3) * 8 + kb) * 128 + (r & 7u) * 16, src + (size_t)(r0 + r) * K + k0 + kb * 8);
+    }
 }
 
 // Softmax cross-entropy of the mode head (logits 0..11) and the table head (12..27) of one
@@ -128,28 +150,34 @@ __device__ __forceinline__ float loss_grad_row(const float (&z)[32], uint32_t la
 }
 
 // Up to two products in one launch: the first n_first blocks are the first one's.
-// Bound by latency: a layer of the training batch is a few tiles of work.  Measured (B200,
-// a gradient step of 2048 rows; 128 x 256 tiles whose 64-wide chunks were loaded and
-// multiplied in turn, products over the rows on 2 CTAs, bias sums by one block each): 0.87
-// -> 0.072 ms of kernels (0.7 us at the bf16 rate); a 2048 x 256 x 256 layer 74 -> 11 us,
-// the 256 x 256 product over the rows 171 -> 12 us beside the next layer's.
+// Bound by latency: a layer of the training batch is a few tiles of work, and a product
+// over the rows one chain of chunks per output.  Tiles of 16 columns for the latter spread
+// it over four times the SMs; a split of the chain would be shorter yet, but its partial
+// sums round apart from the single accumulation's (3.6e-5 of the gradient at 14,826 rows).
+// Measured (B200, a gradient step of 2048 rows; 128 x 256 tiles whose 64-wide chunks were
+// loaded and multiplied in turn, products over the rows on 2 CTAs, bias sums by one block
+// each): 0.87 -> 0.105 ms of kernels (0.7 us at the bf16 rate); a 2048 x 256 x 256 layer
+// 74 -> 9.5 us, the 256 x 256 product over the rows 171 -> 20 us beside the next layer's.
+template <bool TILED>
 __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, GemmArgs G1, uint32_t n_first) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sA = smem;                                // 4 x 16 KB
-    uint8_t* sB = smem + kTileA * (kKBlock / kKChunk);  // 4 x 8 KB
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bars[kStages], full[kStages];  // a stage's products done; its copies landed (TILED)
+    __shared__ uint32_t s_ok;
     __shared__ uint32_t tmem_base;
     const bool second = blockIdx.x >= n_first;
     const GemmArgs& G = second ? G1 : G0;
     const uint32_t blk = second ? blockIdx.x - n_first : blockIdx.x;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t mt = G.M / 128u, nt = (G.N + kTileN - 1) / kTileN;
-    const uint32_t m0 = (blk % mt) * 128u, n0 = (blk / mt % nt) * kTileN, split = blk / (mt * nt);
-    const uint32_t N = min(kTileN, G.N - n0);
+    const uint32_t mt = G.M / 128u;
+    const uint32_t m0 = (blk % mt) * 128u, n0 = (blk / mt) * G.tile_n;
+    const uint32_t N = min(G.tile_n, G.N - n0);
     const uint32_t ncols = N <= 32 ? 32u : 64u;
-    const uint32_t ka = split * G.k_split, ke = min(G.K, ka + G.k_split);
+    const uint32_t sA = smem_u32(smem), sB = sA + kStages * kTileA;
     if (tid == 0) {
-        mbar_init(smem_u32(&bar), 1);
+        for (uint32_t s = 0; s < kStages; ++s) {
+            mbar_init(smem_u32(&bars[s]), 1);
+            mbar_init(smem_u32(&full[s]), 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -164,36 +192,66 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
     const uint32_t tmem = tmem_base;
     // M = 128, N, bf16 x bf16 -> f32, both operands K-major
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
-    uint32_t parity = 0;
-    bool ok = true;
-    for (uint32_t k0 = ka; k0 < ke && ok; k0 += kKBlock) {
-        const uint32_t chunks = min(kKBlock, ke - k0) / kKChunk;
-        load_operand(smem_u32(sA), kTileA, G.A, G.K, m0, 128u, k0, chunks);
-        load_operand(smem_u32(sB), kTileB, G.B, G.K, n0, N, k0, chunks);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (uint32_t c = 0; c < chunks; ++c)
+    const uint32_t chunks = G.K / kKChunk;
+    auto done = [&](uint32_t c) { return mbar_wait(smem_u32(&bars[c % kStages]), (c / kStages) & 1u); };
+    auto multiply = [&](uint32_t c) {
 #pragma unroll
-                for (uint32_t s = 0; s < kKChunk / 16; ++s) {
-                    const uint64_t ad = smem_desc(smem_u32(sA) + c * kTileA + s * 256u);
-                    const uint64_t bd = smem_desc(smem_u32(sB) + c * kTileB + s * 256u);
-                    const uint32_t acc = (k0 > ka || c > 0 || s > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                        "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-                        : "memory");
+        for (uint32_t s = 0; s < kKChunk / 16; ++s)
+            mma_bf16(tmem, smem_desc(sA + (c % kStages) * kTileA + s * 256u),
+                     smem_desc(sB + (c % kStages) * kTileB + s * 256u), idesc, (c > 0 || s > 0) ? 1u : 0u);
+        mma_commit(smem_u32(&bars[c % kStages]));
+    };
+    bool ok = true;
+    if (TILED) {
+        if (tid == 0) {
+            auto landed = [&](uint32_t c) { return mbar_wait(smem_u32(&full[c % kStages]), (c / kStages) & 1u); };
+            auto load = [&](uint32_t c) {
+                const uint32_t s = c % kStages, bar = smem_u32(&full[s]);
+                expect_bytes(bar, kTileA + N * kKChunk * 2);
+                bulk_g2s(sA + s * kTileA, G.A + tiled_at(G.M, m0, c * kKChunk), kTileA, bar);
+                bulk_g2s(sB + s * kTileB, G.B + tiled_at(G.N, n0, c * kKChunk), N * kKChunk * 2, bar);
+            };
+            uint32_t issued = 0, waited = 0;
+            for (; issued < min(kStages, chunks); ++issued) load(issued);
+            for (uint32_t c = 0; c < chunks && ok; ++c) {
+                ok = landed(c);
+                waited = c + 1;
+                if (!ok) break;
+                multiply(c);
+                // the stage before this one is filled again once its products are done
+                if (c > 0 && issued < chunks) {
+                    ok = done(c - 1);
+                    if (ok) load(issued++);
                 }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&bar))
-                         : "memory");
+            }
+            if (ok) ok = done(chunks - 1);
+            for (; waited < issued; ++waited) landed(waited);  // (after a failure: no copy in flight at the exit)
+            s_ok = ok ? 1u : 0u;
         }
-        // one decision for the whole block; the operands' shared memory is free again
-        ok = __syncthreads_and(mbar_wait(smem_u32(&bar), parity)) != 0;
-        parity ^= 1u;
+        __syncthreads();
+        ok = s_ok != 0;
+    } else {
+        auto load = [&](uint32_t c) {  // chunk c into its stage; a group of copies either way
+            if (c < chunks) {
+                load_operand(sA + (c % kStages) * kTileA, G.A, G.K, m0, 128u, c * kKChunk);
+                load_operand(sB + (c % kStages) * kTileB, G.B, G.K, n0, N, c * kKChunk);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        for (uint32_t c = 0; c + 1 < kStages; ++c) load(c);
+        for (uint32_t c = 0; c < chunks; ++c) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (!(ok = __syncthreads_and(ok))) break;  // one decision for the whole block
+            if (tid == 0) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                multiply(c);
+            }
+            if (c > 0) ok = done(c - 1);
+            if (ok) load(c + kStages - 1);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        ok = __syncthreads_and(ok && done(chunks - 1)) != 0;
     }
     if (!ok && tid == 0 && G.err) atomicExch(G.err, 1u);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -212,25 +270,25 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
         if (row < G.n_rows) l = loss_grad_row(z, G.label[row], G.n_rows, g);
         for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
         if (lane == 0) atomicAdd(G.loss, l);
-        // dZ [rows][64], zero beyond the logits, and its transpose [32][rows]
-        uint4* dst = reinterpret_cast<uint4*>(G.Cb + (size_t)row * 64);
+        // dZ [rows][64], zero beyond the logits, and its transpose [32][rows], tiled
 #pragma unroll
-        for (uint32_t q = 0; q < 4; ++q)
-            dst[q] = make_uint4(pack_bf16(g[8 * q], g[8 * q + 1]), pack_bf16(g[8 * q + 2], g[8 * q + 3]),
-                                pack_bf16(g[8 * q + 4], g[8 * q + 5]), pack_bf16(g[8 * q + 6], g[8 * q + 7]));
+        for (uint32_t q = 0; q < 8; ++q)
+            *reinterpret_cast<uint4*>(G.Cb + tiled_at(G.M, row, 8 * q)) =
+                q < 4 ? make_uint4(pack_bf16(g[8 * q], g[8 * q + 1]), pack_bf16(g[8 * q + 2], g[8 * q + 3]),
+                                   pack_bf16(g[8 * q + 4], g[8 * q + 5]), pack_bf16(g[8 * q + 6], g[8 * q + 7]))
+                      : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (uint32_t q = 4; q < 8; ++q) dst[q] = make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (uint32_t j = 0; j < 32; ++j) G.CbT[(size_t)j * G.M + row] = __float2bfloat16_rn(g[j]);
+        for (uint32_t j = 0; j < 32; ++j) G.CbT[tiled_at(32, j, row)] = __float2bfloat16_rn(g[j]);
     } else if (ok) {
-        float* C = G.C ? G.C + (size_t)split * G.M * G.N : nullptr;
-        float* CT = G.CT ? G.CT + (size_t)split * G.M * G.N : nullptr;
+        float *C = G.C, *CT = G.CT;
         // (rows of N = 16 k values: 16-byte pieces when the arrays start on one)
         const bool vec_c = aligned16(C), vec_cb = aligned16(G.Cb), vec_mask = aligned16(G.mask);
         for (uint32_t j0 = 0; j0 < N; j0 += 16) {
             uint32_t v[16];
             tmem_ld16(taddr + j0, v);
-            const size_t at = (size_t)row * G.N + n0 + j0;
+            // two runs of eight columns, 16 bytes each: side by side, or in two core matrices
+            const size_t at = TILED ? tiled_at(G.M, row, n0 + j0) : (size_t)row * G.N + n0 + j0;
+            const uint32_t next8 = TILED ? 64u : 8u;
             float x[16];
 #pragma unroll
             for (uint32_t j = 0; j < 16; ++j) {
@@ -240,9 +298,9 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
             }
             if (G.mask) {
                 __nv_bfloat16 m[16];
-                if (vec_mask) {
-                    reinterpret_cast<uint4*>(m)[0] = reinterpret_cast<const uint4*>(G.mask + at)[0];
-                    reinterpret_cast<uint4*>(m)[1] = reinterpret_cast<const uint4*>(G.mask + at)[1];
+                if (TILED || vec_mask) {
+                    reinterpret_cast<uint4*>(m)[0] = *reinterpret_cast<const uint4*>(G.mask + at);
+                    reinterpret_cast<uint4*>(m)[1] = *reinterpret_cast<const uint4*>(G.mask + at + next8);
                 } else {
 #pragma unroll
                     for (uint32_t j = 0; j < 16; ++j) m[j] = G.mask[at + j];
@@ -251,22 +309,23 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
                 for (uint32_t j = 0; j < 16; ++j)
                     if (!(__bfloat162float(m[j]) > 0.0f)) x[j] = 0.0f;
             }
-            if (C) {
+            if (C) {  // (row-major either way)
+                float* o = C + (size_t)row * G.N + n0 + j0;
                 if (vec_c) {
 #pragma unroll
                     for (uint32_t q = 0; q < 4; ++q)
-                        reinterpret_cast<float4*>(C + at)[q] =
+                        reinterpret_cast<float4*>(o)[q] =
                             make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
                 } else {
 #pragma unroll
-                    for (uint32_t j = 0; j < 16; ++j) C[at + j] = x[j];
+                    for (uint32_t j = 0; j < 16; ++j) o[j] = x[j];
                 }
             }
             if (G.Cb) {
-                if (vec_cb) {
+                if (TILED || vec_cb) {
 #pragma unroll
                     for (uint32_t q = 0; q < 2; ++q)
-                        reinterpret_cast<uint4*>(G.Cb + at)[q] =
+                        *reinterpret_cast<uint4*>(G.Cb + at + q * next8) =
                             make_uint4(pack_bf16(x[8 * q], x[8 * q + 1]), pack_bf16(x[8 * q + 2], x[8 * q + 3]),
                                        pack_bf16(x[8 * q + 4], x[8 * q + 5]), pack_bf16(x[8 * q + 6], x[8 * q + 7]));
                 } else {
@@ -277,7 +336,8 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
             if (G.CbT)
 #pragma unroll
                 for (uint32_t j = 0; j < 16; ++j)
-                    G.CbT[(size_t)(n0 + j0 + j) * G.M + row] = __float2bfloat16_rn(x[j]);
+                    G.CbT[TILED ? tiled_at(G.N, n0 + j0 + j, row) : (size_t)(n0 + j0 + j) * G.M + row] =
+                        __float2bfloat16_rn(x[j]);
             if (CT)
 #pragma unroll
                 for (uint32_t j = 0; j < 16; ++j) CT[(size_t)(n0 + j0 + j) * G.M + row] = x[j];
@@ -327,25 +387,6 @@ struct InferArgs {
     uint8_t* sel;               // [count] or null: argmax(0..11) | argmax(12..27) << 4
     uint32_t* err;
 };
-
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-        "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 
 // (row r, K element k) of a 128-row A operand held as 64-wide K-chunks of core matrices
 __device__ __forceinline__ uint32_t a_off(uint32_t r, uint32_t k) {
@@ -414,7 +455,9 @@ __global__ void __launch_bounds__(kInferThreads, 1) mlp_infer_kernel(InferArgs G
                          sbase + kOffW3),
                      "l"(G.W3t), "r"(4 * kChunkW3), "r"(b_w)
                      : "memory");
+        expect_bytes(b_full(0), kChunkW2);
         bulk_g2s(sbase + kOffRing, G.W2t, kChunkW2, b_full(0));
+        expect_bytes(b_full(1), kChunkW2);
         bulk_g2s(sbase + kOffRing + kChunkW2, reinterpret_cast<const uint8_t*>(G.W2t) + kChunkW2, kChunkW2, b_full(1));
     }
     const uint32_t idesc256 = (1u << 4) | (1u << 7) | (1u << 10) | ((kHidN >> 3) << 17) | ((128u >> 4) << 24);
@@ -492,6 +535,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) mlp_infer_kernel(InferArgs G
                     w = mbar_wait(b_free(ps), ph_free[ps]);
                     ph_free[ps] ^= 1u;
                     if (w) {
+                        expect_bytes(b_full(ps), kChunkW2);
                         bulk_g2s(sbase + kOffRing + ps * kChunkW2, reinterpret_cast<const uint8_t*>(G.W2t) + nq * kChunkW2,
                                  kChunkW2, b_full(ps));
                         pending[ps] = true;
@@ -502,6 +546,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) mlp_infer_kernel(InferArgs G
                 w = mbar_wait(b_free(1), ph_free[1]);
                 ph_free[1] ^= 1u;
                 if (w) {
+                    expect_bytes(b_full(1), kChunkW2);
                     bulk_g2s(sbase + kOffRing + kChunkW2, reinterpret_cast<const uint8_t*>(G.W2t) + kChunkW2, kChunkW2,
                              b_full(1));
                     pending[1] = true;
@@ -603,24 +648,24 @@ cudaError_t launch_mlp_infer(const float* feat, uint32_t count, const __nv_bfloa
     return cudaGetLastError();
 }
 
-static uint32_t gemm_blocks(const GemmArgs& g) {
-    return g.M / 128 * ((g.N + kTileN - 1) / kTileN) * ((g.K + g.k_split - 1) / g.k_split);
-}
+static uint32_t gemm_blocks(const GemmArgs& g) { return g.M / 128 * ((g.N + g.tile_n - 1) / g.tile_n); }
 
 cudaError_t launch_gemm_bf16(const GemmArgs& g, cudaStream_t st, const GemmArgs* second) {
     if (g.M == 0 || g.N == 0 || g.K == 0) return cudaSuccess;
     for (const GemmArgs* p : {&g, second})
-        if (p && (p->M % 128 || p->N % 16 || p->K % kKChunk || p->k_split == 0 || p->k_split % kKChunk))
+        if (p && (p->M % 128 || p->N % 16 || p->K % kKChunk || p->tile_n == 0 || p->tile_n % 16 || p->tile_n > kTileN))
             return cudaErrorInvalidValue;
-    constexpr int smem = (int)((kTileA + kTileB) * (kKBlock / kKChunk));
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (second && second->tiled != g.tiled) return cudaErrorInvalidValue;
+    constexpr int smem = (int)((kTileA + kTileB) * kStages);
+    const auto kernel = g.tiled ? gemm_bf16_kernel<true> : gemm_bf16_kernel<false>;
+    static bool attr[2] = {false, false};
+    if (!attr[g.tiled]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
-        attr = true;
+        attr[g.tiled] = true;
     }
     const uint32_t n = gemm_blocks(g);
-    gemm_bf16_kernel<<<n + (second ? gemm_blocks(*second) : 0u), kGemmThreads, smem, st>>>(g, second ? *second : g, n);
+    kernel<<<n + (second ? gemm_blocks(*second) : 0u), kGemmThreads, smem, st>>>(g, second ? *second : g, n);
     return cudaGetLastError();
 }
 
@@ -641,7 +686,7 @@ extern "C" int csv_gemm_bf16(csv_ctx* ctx, const void* d_A, const void* d_B, uin
     G.B = (const __nv_bfloat16*)d_B;
     G.M = M;
     G.N = N;
-    G.K = G.k_split = K;
+    G.K = K;
     G.bias = d_bias;
     G.mask = (const __nv_bfloat16*)d_mask;
     G.relu = relu;

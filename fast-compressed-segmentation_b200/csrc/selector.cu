@@ -365,7 +365,7 @@ constexpr uint32_t OFF_W1 = 0, OFF_B1 = OFF_W1 + kHid * kFeatPad, OFF_W2 = OFF_B
                    N_PARAMS = OFF_B3 + kOut;
 static_assert(N_PARAMS == CSV_MLP_PARAMS, "parameter layout");
 
-// features (n x 32, fp32) -> X (rows x 64, bf16, zero padded) and X^T (64 x rows)
+// features (n x 32, fp32) -> X (rows x 64, bf16, zero padded) and X^T (64 x rows), tiled
 __global__ void pack_input_kernel(const float* __restrict__ feat, uint32_t n, uint32_t rows,
                                   __nv_bfloat16* __restrict__ X, __nv_bfloat16* __restrict__ XT) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -373,79 +373,63 @@ __global__ void pack_input_kernel(const float* __restrict__ feat, uint32_t n, ui
     const uint32_t r = k / kFeatPad, c = k % kFeatPad;
     const float v = (r < n && c < kFeat) ? feat[(size_t)r * kFeat + c] : 0.0f;
     const __nv_bfloat16 b = __float2bfloat16_rn(v);
-    X[k] = b;
-    XT[(size_t)c * rows + r] = b;
+    X[tiled_at(rows, r, c)] = b;
+    XT[tiled_at(kFeatPad, c, r)] = b;
 }
 
-// Partial column sums of dZ (32 columns of 64), dH2 and dH1 (256), the bias gradients:
-// block (part, matrix), a thread per column, over `per` rows each.
-__global__ void __launch_bounds__(256) colsum_kernel(const __nv_bfloat16* __restrict__ dZ,
-                                                     const __nv_bfloat16* __restrict__ dH2,
-                                                     const __nv_bfloat16* __restrict__ dH1, uint32_t rows, uint32_t per,
+// Partial sums over the rows of dZ (32 columns), dH2 and dH1 (256), the bias gradients, from
+// their tiled transposes (eight rows of a column are 16 bytes): block (part, matrix), a
+// thread per column, over `per` rows each (a multiple of 8, as the batch's).
+__global__ void __launch_bounds__(256) colsum_kernel(const __nv_bfloat16* __restrict__ dZT,
+                                                     const __nv_bfloat16* __restrict__ dH2T,
+                                                     const __nv_bfloat16* __restrict__ dH1T, uint32_t rows, uint32_t per,
                                                      float* __restrict__ out) {
-    const uint32_t c = threadIdx.x, which = blockIdx.y;
-    if (which == 0 && c >= kOut) return;
-    const __nv_bfloat16* m = which == 0 ? dZ : (which == 1 ? dH2 : dH1);
-    const uint32_t ld = which == 0 ? kOutPad : kHid, r1 = min(rows, (blockIdx.x + 1) * per);
+    const uint32_t c = threadIdx.x, which = blockIdx.y, cols = which == 0 ? kOut : kHid;
+    if (c >= cols) return;
+    const __nv_bfloat16* m = which == 0 ? dZT : (which == 1 ? dH2T : dH1T);
+    const uint32_t r1 = min(rows, (blockIdx.x + 1) * per);
     float s = 0.0f;
-#pragma unroll 8
-    for (uint32_t r = blockIdx.x * per; r < r1; ++r) s += __bfloat162float(m[(size_t)r * ld + c]);
+#pragma unroll 4
+    for (uint32_t r = blockIdx.x * per; r < r1; r += 8) {
+        const uint4 v = *reinterpret_cast<const uint4*>(m + tiled_at(cols, c, r));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {  // (bf16 is the upper half of fp32)
+            s += __uint_as_float(w[k] << 16);
+            s += __uint_as_float(w[k] & 0xFFFF0000u);
+        }
+    }
     out[((size_t)which * gridDim.x + blockIdx.x) * kHid + c] = s;
 }
 
-// The gradients from their partial sums, in order.  part: `splits` products dW1 [256][64],
-// then dW2 [256][256], then dW3^T stored as W3 lies [32][256]; bias: colsum_kernel's.
-__global__ void __launch_bounds__(256) grad_sum_kernel(const float* __restrict__ part, uint32_t splits,
-                                                       const float* __restrict__ bias, uint32_t bias_parts,
+// The bias gradients from colsum_kernel's partial sums, in order.
+__global__ void __launch_bounds__(256) bias_sum_kernel(const float* __restrict__ part, uint32_t parts,
                                                        float* __restrict__ G) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N_PARAMS) return;
-    const float* p;
-    uint32_t n = splits, stride;
-    if (k < OFF_B1) {
-        p = part + k;
-        stride = kHid * kFeatPad;
-    } else if (k >= OFF_W2 && k < OFF_B2) {
-        p = part + (size_t)splits * (kHid * kFeatPad) + (k - OFF_W2);
-        stride = kHid * kHid;
-    } else if (k >= OFF_W3 && k < OFF_B3) {
-        p = part + (size_t)splits * (kHid * kFeatPad + kHid * kHid) + (k - OFF_W3);
-        stride = kOut * kHid;
-    } else {
-        const uint32_t which = k >= OFF_B3 ? 0u : (k >= OFF_B2 ? 1u : 2u);
-        p = bias + (size_t)which * bias_parts * kHid + (k - (which == 0 ? OFF_B3 : (which == 1 ? OFF_B2 : OFF_B1)));
-        stride = kHid;
-        n = bias_parts;
-    }
+    const uint32_t c = threadIdx.x, which = blockIdx.x;
+    if (which == 0 && c >= kOut) return;
     float s = 0.0f;
 #pragma unroll 8
-    for (uint32_t i = 0; i < n; ++i) s += p[(size_t)i * stride];
-    G[k] = s;
+    for (uint32_t i = 0; i < parts; ++i) s += part[((size_t)which * parts + i) * kHid + c];
+    G[(which == 0 ? OFF_B3 : (which == 1 ? OFF_B2 : OFF_B1)) + c] = s;
 }
 
-// A weight's bf16 copies: W1b [256][64], W2b [256][256] and its transpose, W3b [32][256] and its
-// transpose [256][64] (columns >= 32 zero), and each layer tiled for the fused forward.
+// A weight's bf16 copies, tiled as the layers read them: W1 [256][64], W2 [256][256] and its
+// transpose, W3 [32][256] and its transpose [256][64] (columns >= 32 zero).
 struct WeightCopies {
-    __nv_bfloat16 *W1b, *W2b, *W2bT, *W3b, *W3bT, *W1t, *W2t, *W3t;
+    __nv_bfloat16 *W1t, *W2t, *W2Tt, *W3t, *W3Tt;
 };
-__device__ __forceinline__ uint32_t tiled_at(uint32_t N, uint32_t n, uint32_t k) {  // the fused forward's layout
-    return (k >> 6) * N * 64 + ((n >> 3) * 8 + ((k & 63u) >> 3)) * 64 + (n & 7u) * 8 + (k & 7u);
-}
 __device__ __forceinline__ void put_weight(const WeightCopies& C, uint32_t k, float v) {
     const __nv_bfloat16 w = __float2bfloat16_rn(v);
     if (k < OFF_B1) {
-        C.W1b[k] = w;
         C.W1t[tiled_at(kHid, k / kFeatPad, k % kFeatPad)] = w;
     } else if (k >= OFF_W2 && k < OFF_B2) {
         const uint32_t i = k - OFF_W2, o = i / kHid, in = i % kHid;
-        C.W2b[i] = w;
-        C.W2bT[(size_t)in * kHid + o] = w;
         C.W2t[tiled_at(kHid, o, in)] = w;
+        C.W2Tt[tiled_at(kHid, in, o)] = w;
     } else if (k >= OFF_W3 && k < OFF_B3) {
         const uint32_t i = k - OFF_W3, o = i / kHid, in = i % kHid;
-        C.W3b[i] = w;
-        C.W3bT[(size_t)in * kOutPad + o] = w;
         C.W3t[tiled_at(kOut, o, in)] = w;
+        C.W3Tt[tiled_at(kHid, in, o)] = w;
     }
 }
 
@@ -470,7 +454,7 @@ __global__ void refresh_kernel(const float* __restrict__ P, WeightCopies C) {
     if (k < N_PARAMS) put_weight(C, k, P[k]);
     if (k < kHid * (kOutPad - kOut)) {
         const uint32_t in = k / (kOutPad - kOut), o = kOut + k % (kOutPad - kOut);
-        C.W3bT[(size_t)in * kOutPad + o] = __float2bfloat16_rn(0.0f);
+        C.W3Tt[tiled_at(kHid, in, o)] = __float2bfloat16_rn(0.0f);
     }
 }
 
@@ -488,12 +472,11 @@ struct csv_mlp {
     float* G = nullptr;
     float* Mm = nullptr;
     float* Vm = nullptr;
-    __nv_bfloat16 *W1b = nullptr, *W2b = nullptr, *W2bT = nullptr, *W3b = nullptr, *W3bT = nullptr;
-    __nv_bfloat16 *W1t = nullptr, *W2t = nullptr, *W3t = nullptr;  // tiled for the fused forward
+    __nv_bfloat16 *W1t = nullptr, *W2t = nullptr, *W2Tt = nullptr, *W3t = nullptr, *W3Tt = nullptr;  // WeightCopies
+    // tiled operands of the gradient step, with their transposes
     __nv_bfloat16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *H2 = nullptr, *H2T = nullptr;
-    __nv_bfloat16 *dZ = nullptr, *dZT = nullptr, *dH2 = nullptr, *dH2T = nullptr, *dH1 = nullptr, *dH1T = nullptr;
-    float* part = nullptr;       // the weight gradients' partial products
-    float* bias_part = nullptr;  // and the bias gradients' partial sums
+    __nv_bfloat16 *dZ = nullptr, *dZT = nullptr, *dH2 = nullptr, *dH2T = nullptr, *dH1T = nullptr;
+    float* bias_part = nullptr;  // the bias gradients' partial sums
     float* loss = nullptr;
     uint32_t* err = nullptr;
 };
@@ -502,19 +485,15 @@ namespace {
 
 void mlp_free_acts(csv_mlp* n) {
     for (void* p : {(void*)n->X, (void*)n->XT, (void*)n->H1, (void*)n->H1T, (void*)n->H2, (void*)n->H2T,
-                    (void*)n->dZ, (void*)n->dZT, (void*)n->dH2, (void*)n->dH2T, (void*)n->dH1, (void*)n->dH1T,
-                    (void*)n->part, (void*)n->bias_part})
+                    (void*)n->dZ, (void*)n->dZT, (void*)n->dH2, (void*)n->dH2T, (void*)n->dH1T,
+                    (void*)n->bias_part})
         cudaFree(p);
-    n->X = n->XT = n->H1 = n->H1T = n->H2 = n->H2T = n->dZ = n->dZT = n->dH2 = n->dH2T = n->dH1 = n->dH1T = nullptr;
-    n->part = n->bias_part = nullptr;
+    n->X = n->XT = n->H1 = n->H1T = n->H2 = n->H2T = n->dZ = n->dZT = n->dH2 = n->dH2T = n->dH1T = nullptr;
+    n->bias_part = nullptr;
     n->cap = 0;
 }
 
-// The weight gradients are products over the rows: split so that a CTA has 256 rows of
-// them (its operands in flight at once), and into no more than 32 partial products.
-uint32_t mlp_k_split(uint32_t rows) { return std::max(256u, (rows / 32 + 63) / 64 * 64); }
-uint32_t mlp_splits(uint32_t rows) { return (rows + mlp_k_split(rows) - 1) / mlp_k_split(rows); }
-uint32_t mlp_bias_rows(uint32_t rows) { return std::max(64u, (rows + 63) / 64); }  // per partial sum
+uint32_t mlp_bias_rows(uint32_t rows) { return std::max(64u, (rows / 64 + 7) / 8 * 8); }  // per partial sum
 uint32_t mlp_bias_parts(uint32_t rows) { return (rows + mlp_bias_rows(rows) - 1) / mlp_bias_rows(rows); }
 
 cudaError_t mlp_reserve(csv_mlp* n, uint32_t rows) {
@@ -535,17 +514,14 @@ cudaError_t mlp_reserve(csv_mlp* n, uint32_t rows) {
     al((void**)&n->dZT, r * kOut * 2);
     al((void**)&n->dH2, r * kHid * 2);
     al((void**)&n->dH2T, r * kHid * 2);
-    al((void**)&n->dH1, r * kHid * 2);
     al((void**)&n->dH1T, r * kHid * 2);
-    // (as many partial results as any batch up to this one has)
-    al((void**)&n->part, std::min<size_t>(32, (rows + 255) / 256) * (kHid * kFeatPad + kHid * kHid + kOut * kHid) * 4);
     al((void**)&n->bias_part, 3 * std::min<size_t>(64, (rows + 63) / 64) * kHid * 4);
     if (e == cudaSuccess) n->cap = rows;
     return e;
 }
 
 WeightCopies mlp_copies(const csv_mlp* n) {
-    return WeightCopies{n->W1b, n->W2b, n->W2bT, n->W3b, n->W3bT, n->W1t, n->W2t, n->W3t};
+    return WeightCopies{n->W1t, n->W2t, n->W2Tt, n->W3t, n->W3Tt};
 }
 
 GemmArgs mlp_gemm(const csv_mlp* n, const __nv_bfloat16* A, const __nv_bfloat16* B, uint32_t M, uint32_t N, uint32_t K) {
@@ -554,7 +530,8 @@ GemmArgs mlp_gemm(const csv_mlp* n, const __nv_bfloat16* A, const __nv_bfloat16*
     g.B = B;
     g.M = M;
     g.N = N;
-    g.K = g.k_split = K;
+    g.K = K;
+    g.tiled = true;
     g.err = n->err;
     return g;
 }
@@ -565,19 +542,19 @@ cudaError_t mlp_forward(csv_mlp* n, const float* feat, const uint8_t* label, uin
     if (e != cudaSuccess) return e;
     pack_input_kernel<<<(rows * kFeatPad + 255) / 256, 256, 0, st>>>(feat, cnt, rows, n->X, n->XT);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    GemmArgs g = mlp_gemm(n, n->X, n->W1b, rows, kHid, kFeatPad);
+    GemmArgs g = mlp_gemm(n, n->X, n->W1t, rows, kHid, kFeatPad);
     g.bias = n->P + OFF_B1;
     g.relu = 1;
     g.Cb = n->H1;
     g.CbT = n->H1T;
     if ((e = launch_gemm_bf16(g, st)) != cudaSuccess) return e;
-    g = mlp_gemm(n, n->H1, n->W2b, rows, kHid, kHid);
+    g = mlp_gemm(n, n->H1, n->W2t, rows, kHid, kHid);
     g.bias = n->P + OFF_B2;
     g.relu = 1;
     g.Cb = n->H2;
     g.CbT = n->H2T;
     if ((e = launch_gemm_bf16(g, st)) != cudaSuccess) return e;
-    g = mlp_gemm(n, n->H2, n->W3b, rows, kOut, kHid);
+    g = mlp_gemm(n, n->H2, n->W3t, rows, kOut, kHid);
     g.bias = n->P + OFF_B3;
     g.Cb = n->dZ;
     g.CbT = n->dZT;
@@ -595,9 +572,8 @@ void csv_mlp_destroy(csv_mlp* n) {
     if (!n) return;
     DeviceGuard g(n->ctx->device);
     mlp_free_acts(n);
-    for (void* p : {(void*)n->P, (void*)n->G, (void*)n->Mm, (void*)n->Vm, (void*)n->W1b, (void*)n->W2b,
-                    (void*)n->W2bT, (void*)n->W3b, (void*)n->W3bT, (void*)n->W1t, (void*)n->W2t, (void*)n->W3t,
-                    (void*)n->loss, (void*)n->err})
+    for (void* p : {(void*)n->P, (void*)n->G, (void*)n->Mm, (void*)n->Vm, (void*)n->W1t, (void*)n->W2t, (void*)n->W2Tt,
+                    (void*)n->W3t, (void*)n->W3Tt, (void*)n->loss, (void*)n->err})
         cudaFree(p);
     delete n;
 }
@@ -617,11 +593,8 @@ int csv_mlp_create(csv_ctx* ctx, const float* params, csv_mlp** out) {
     al((void**)&n->G, N_PARAMS * 4);
     al((void**)&n->Mm, N_PARAMS * 4);
     al((void**)&n->Vm, N_PARAMS * 4);
-    al((void**)&n->W1b, kHid * kFeatPad * 2);
-    al((void**)&n->W2b, kHid * kHid * 2);
-    al((void**)&n->W2bT, kHid * kHid * 2);
-    al((void**)&n->W3b, kOut * kHid * 2);
-    al((void**)&n->W3bT, kHid * kOutPad * 2);
+    al((void**)&n->W2Tt, kHid * kHid * 2);
+    al((void**)&n->W3Tt, kHid * kOutPad * 2);
     al((void**)&n->W1t, kHid * kFeatPad * 2);
     al((void**)&n->W2t, kHid * kHid * 2);
     al((void**)&n->W3t, kOut * kHid * 2);
@@ -676,42 +649,39 @@ int csv_mlp_grad(csv_mlp* n, const float* d_feat, const uint8_t* d_label, uint32
     const uint32_t rows = (count + 127) / 128 * 128;
     cudaError_t e = mlp_reserve(n, rows);
     if (e == cudaSuccess) e = mlp_forward(n, d_feat, d_label, count, rows, st);
-    const uint32_t ks = mlp_k_split(rows), splits = mlp_splits(rows), parts = mlp_bias_parts(rows);
-    float* p1 = n->part;
-    float* p2 = p1 + (size_t)splits * (kHid * kFeatPad);
-    float* p3 = p2 + (size_t)splits * (kHid * kHid);
-    // a product over the rows beside one over the units where both have their operands
+    // a product over the rows (few outputs, so narrow tiles) beside one over the units where both have
+    // their operands
     auto over_rows = [&](const __nv_bfloat16* A, const __nv_bfloat16* B, uint32_t N) {
         GemmArgs g = mlp_gemm(n, A, B, kHid, N, rows);
-        g.k_split = ks;
+        g.tile_n = 16;
         return g;
     };
     if (e == cudaSuccess) {
         GemmArgs w = over_rows(n->H2T, n->dZT, kOut);  // dW3^T = H2^T dZ, written as W3 lies
-        w.CT = p3;
-        GemmArgs h = mlp_gemm(n, n->dZ, n->W3bT, rows, kHid, kOutPad);  // dH2 = (dZ W3) * (H2 > 0)
+        w.CT = n->G + OFF_W3;
+        GemmArgs h = mlp_gemm(n, n->dZ, n->W3Tt, rows, kHid, kOutPad);  // dH2 = (dZ W3) * (H2 > 0)
         h.mask = n->H2;
         h.Cb = n->dH2;
         h.CbT = n->dH2T;
-        e = launch_gemm_bf16(h, st, &w);
+        e = launch_gemm_bf16(w, st, &h);
     }
     if (e == cudaSuccess) {
         GemmArgs w = over_rows(n->dH2T, n->H1T, kHid);  // dW2 = dH2^T H1
-        w.C = p2;
-        GemmArgs h = mlp_gemm(n, n->dH2, n->W2bT, rows, kHid, kHid);  // dH1 = (dH2 W2) * (H1 > 0)
+        w.C = n->G + OFF_W2;
+        GemmArgs h = mlp_gemm(n, n->dH2, n->W2Tt, rows, kHid, kHid);  // dH1 = (dH2 W2) * (H1 > 0)
         h.mask = n->H1;
-        h.Cb = n->dH1;
         h.CbT = n->dH1T;
-        e = launch_gemm_bf16(h, st, &w);
+        e = launch_gemm_bf16(w, st, &h);
     }
     if (e == cudaSuccess) {
         GemmArgs w = over_rows(n->dH1T, n->XT, kFeatPad);  // dW1 = dH1^T X
-        w.C = p1;
+        w.C = n->G + OFF_W1;
         e = launch_gemm_bf16(w, st);
     }
     if (e == cudaSuccess) {
-        colsum_kernel<<<dim3(parts, 3), 256, 0, st>>>(n->dZ, n->dH2, n->dH1, rows, mlp_bias_rows(rows), n->bias_part);
-        grad_sum_kernel<<<(N_PARAMS + 255) / 256, 256, 0, st>>>(n->part, splits, n->bias_part, parts, n->G);
+        const uint32_t parts = mlp_bias_parts(rows);
+        colsum_kernel<<<dim3(parts, 3), 256, 0, st>>>(n->dZT, n->dH2T, n->dH1T, rows, mlp_bias_rows(rows), n->bias_part);
+        bias_sum_kernel<<<3, 256, 0, st>>>(n->bias_part, parts, n->G);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && loss) {

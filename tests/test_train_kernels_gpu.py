@@ -9,8 +9,7 @@ def _rel(a, b):
     return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-12))
 
 
-# one row; a tile and its remainder; one partial product and several; a batch whose partial products are longer, then a
-# smaller one with more of them in the same buffers
+# one row; a tile and its remainder; one partial bias sum and several; a large batch, then smaller ones in its buffers
 @pytest.mark.parametrize("batches", [(1,), (128, 200), (256, 257), (2048,), (8300, 8192, 100)])
 def test_gradients_by_batch(codec, oracle, batches):
     import torch
@@ -36,9 +35,9 @@ def test_gradients_by_batch(codec, oracle, batches):
     net.close()
 
 
-# column tiles of 64 and their remainders, K below, at and above what a CTA has in flight; outputs that start off a
-# 16-byte boundary
-@pytest.mark.parametrize("M,N,K", [(128, 80, 64), (256, 208, 320), (128, 64, 256), (384, 112, 832)])
+# column tiles of 64 and their remainders, K below, at and above what a CTA has in flight (three and four chunks of 64);
+# outputs that start off a 16-byte boundary
+@pytest.mark.parametrize("M,N,K", [(128, 80, 64), (256, 208, 320), (128, 64, 192), (128, 64, 256), (384, 112, 832)])
 def test_dense_layer_tiles(codec, M, N, K):
     import torch
     rng = np.random.default_rng(M + N + K)
