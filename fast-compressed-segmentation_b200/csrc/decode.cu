@@ -248,7 +248,7 @@ __device__ __forceinline__ uint32_t index_step(uint32_t& x, uint32_t& pos, const
 constexpr uint32_t kSnap = 32;  // symbols between state snapshots
 static_assert(kSeedSymbols % kSnap == 0, "a sidecar's states fall on snapshots");
 
-// Pass 1's chain step in two forms.
+// Pass 1's chain step in three forms (ChainRing, of whole chains, follows them).
 //
 // ChainRef: ransDecodeSymbol and the renormalisation loop as the reference
 // writes them (brickDecoding.cpp:137-151), for any table and start state.  The
@@ -345,6 +345,181 @@ struct ChainFast {
     }
     __device__ __forceinline__ uint32_t where() const { return pos8 >> 3; }
 };
+
+// ChainFast's arithmetic for a brick whose whole chain one lane runs, where the dependent
+// chain itself sets the time.  What is off the chain:
+//   - the choice between taking no byte and one: both successors' table entries are looked
+//     up while the compare runs, and one is selected;
+//   - two bytes: only a symbol of frequency below 16 can want them.  Eight symbols are
+//     decoded as if none did, and again by step() if one did;
+//   - shifts between an entry and the next address: an entry holds 16 freq and 16 (x -
+//     start) + symbol, so that 16 freq (x >> 12) + 16 (x - start) + symbol = 16 x' + symbol
+//     has the next entry's address in its low bits, and a second table with the index's
+//     bytes exchanged takes the one-byte successor's;
+//   - the stream: the eight bytes at the read position are all that eight symbols can take;
+//     they come from 512 bytes of the stream in a shared ring per lane, filled ahead by
+//     asynchronous copies, so that no lane's load holds up the warp.
+// Measured (B200, one warp, a table with 0.6 % of rare symbols): a step of the chain 50
+// cycles, 64 with the windows, the copies and the words done again; all three successors
+// looked up and selected: 80.
+constexpr uint32_t kRing = 512, kRingPitch = kRing + 16, kRingPieces = kRing / 16;
+extern __shared__ __align__(16) uint8_t idx_smem[];  // entries by index (first half of 16 bytes) and by exchanged index
+struct ChainRing {
+    const uint8_t* enc;
+    uint8_t* ring;
+    uint32_t x, pos;
+    uint32_t xh;       // x >> 12
+    uint2 e;           // x's entry
+    uint32_t hi, lo;   // the eight bytes below pos, next one on top
+    int32_t qn;        // the next 16-byte piece of the stream to be copied (below 0: none)
+    __device__ __forceinline__ uint2 entry(uint32_t at) const {
+        return *reinterpret_cast<const uint2*>(idx_smem + at);
+    }
+    __device__ __forceinline__ uint32_t ring_word(uint32_t byte) const {
+        return *reinterpret_cast<const uint32_t*>(ring + (byte & (kRing - 1)));
+    }
+    __device__ __forceinline__ void copy_piece() {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(ring + (((uint32_t)qn << 4) & (kRing - 1)))),
+                     "l"(enc + ((size_t)qn << 4))
+                     : "memory");
+        --qn;
+    }
+    __device__ __forceinline__ void init(const uint8_t* stream, uint32_t x0, uint32_t pos0, uint8_t* lane_ring) {
+        enc = stream;
+        ring = lane_ring;
+        pos = pos0;
+        qn = (int32_t)((pos0 + 15) >> 4) - 1;
+        // what is left is a multiple of four pieces
+        const int32_t last = qn >= (int32_t)kRingPieces - 4 ? (qn - ((int32_t)kRingPieces - 4)) & ~3 : 0;
+        while (qn >= last) copy_piece();
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        window();
+        set(x0);
+    }
+    __device__ __forceinline__ void set(uint32_t v) {
+        x = v;
+        xh = v >> kTotBits;
+        e = entry((v & (kTot - 1)) * 16);
+    }
+    // Before each 32 symbols (64 bytes at most): keeps the ring full, four pieces at a time, when those 512 bytes
+    // above them have been read.  They are first read five groups later or more (four may be in flight).
+    __device__ __forceinline__ void stage() {
+        if (qn >= 0 && (int32_t)(pos >> 4) - qn < (int32_t)kRingPieces - 3) {
+            copy_piece();
+            copy_piece();
+            copy_piece();
+            copy_piece();
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 4;" ::: "memory");
+    }
+    __device__ __forceinline__ void window() {
+        const uint32_t r = 8 * (pos & 3u), a = pos & ~3u, w1 = ring_word(a - 4);
+        hi = __funnelshift_r(w1, ring_word(a), r);
+        lo = __funnelshift_r(ring_word(a - 8), w1, r);
+    }
+    __device__ __forceinline__ uint32_t step() {  // anywhere in the stream
+        const uint32_t sym = e.y & 15u;
+        const uint32_t v = (e.x >> 4) * xh + (e.y >> 4);
+        const uint32_t want = v < (kRansL >> 8) ? 2u : (v < kRansL ? 1u : 0u);
+        const uint32_t n = min(want, pos);
+        set(__funnelshift_l(hi, v, 8 * n));
+        pos -= n;
+        window();
+        return sym;
+    }
+    // Eight symbols, with 16 bytes or more left.
+    __device__ __forceinline__ uint32_t word() {
+        const uint32_t pos0 = pos, xh0 = xh;
+        const uint2 e0 = e;
+        uint32_t low = ~0u, wd = 0, bits = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint64_t p = (uint64_t)e.x * xh + e.y;  // 16 v + symbol
+            const uint2 s0 = entry((uint32_t)p & (16 * (kTot - 1)));
+            const uint2 s1 = entry((((uint32_t)p & 0xF0u) | __byte_perm(hi, 0, 0x4434)) + 8);
+            wd = __funnelshift_r(wd, e.y, 4);
+            const uint32_t h0 = (uint32_t)(p >> 16), h1 = (uint32_t)p >> 8;  // v >> 12, v >> 4 (v < 2^23)
+            const bool n1 = h0 < (kRansL >> kTotBits);
+            low = min(low, h0);
+            if (j == 7) x = n1 ? (uint32_t)(p >> 4) << 8 | hi >> 24 : (uint32_t)(p >> 4);
+            const uint32_t sh = n1 ? 8u : 0u;
+            xh = n1 ? h1 : h0;
+            hi = __funnelshift_l(lo, hi, sh);
+            lo <<= sh;
+            bits += sh;
+            e.x = n1 ? s1.x : s0.x;
+            e.y = n1 ? s1.y : s0.y;
+        }
+        pos -= bits >> 3;
+        window();
+        if (low < (kRansL >> 8 >> kTotBits)) {
+            pos = pos0;
+            xh = xh0;
+            e = e0;
+            window();
+            wd = slow_word();
+        }
+        return wd;
+    }
+    __device__ __forceinline__ uint32_t slow_word() {
+        uint32_t wd = 0;
+#pragma unroll 1
+        for (uint32_t j = 0; j < 8; ++j) wd = __funnelshift_r(wd, step(), 4);
+        return wd;
+    }
+    __device__ __forceinline__ uint32_t where() const { return pos; }
+};
+
+// index_walk over a whole brick's chain (32 symbols at a time: w 16-byte aligned).
+__device__ __forceinline__ bool index_walk_ring(ChainRing& c, uint32_t n, uint32_t* __restrict__ w,
+                                                uint2* __restrict__ sn) {
+    sn[0] = make_uint2(c.x, c.pos);
+    const uint32_t root = c.step();
+    if (root & 1u) {
+        w[0] = root;
+        return false;
+    }
+    uint32_t wd = root << 28;
+    for (uint32_t i = 1; i < 32 && i < n; ++i) {  // symbols 1..31
+        wd = __funnelshift_r(wd, c.step(), 4);
+        if ((i & 7u) == 7) w[i >> 3] = wd;
+    }
+    if (n < 32) {
+        if (n & 7u) w[n >> 3] = wd >> (32 - 4 * (n & 7u));
+        return true;
+    }
+    uint32_t k = 1;  // groups of 32
+    while (32 * k + 32 <= n) {
+        const uint32_t fast = c.pos >> 6;  // each takes 64 bytes at most
+        for (const uint32_t end = min(n >> 5, k + max(fast, 1u)); k < end; ++k) {
+            c.stage();
+            sn[k] = make_uint2(c.x, c.pos);
+            uint4 q;
+            if (fast) {
+                q.x = c.word();
+                q.y = c.word();
+                q.z = c.word();
+                q.w = c.word();
+            } else {
+                q.x = c.slow_word();
+                q.y = c.slow_word();
+                q.z = c.slow_word();
+                q.w = c.slow_word();
+            }
+            reinterpret_cast<uint4*>(w)[k] = q;
+        }
+    }
+    if (32 * k < n) {
+        sn[k] = make_uint2(c.x, c.pos);
+        for (uint32_t i = 32 * k; i < n; ++i) {
+            wd = __funnelshift_r(wd, c.step(), 4);
+            if ((i & 7u) == 7) w[i >> 3] = wd;
+        }
+        if (n & 7u) w[n >> 3] = wd >> (32 - 4 * (n & 7u));
+    }
+    return true;
+}
 
 // Symbols [s0, s1) of one brick's chain (s0 a multiple of kSnap): packed
 // nibbles to w (word s0 / 8 on), the state before every kSnap-th symbol to sn.
@@ -458,26 +633,30 @@ __device__ __forceinline__ void index_finish(BrickDesc* bricks, uint32_t bi, con
     }
 }
 
-__global__ void __launch_bounds__(128) index_symbols_kernel(BrickDesc* __restrict__ bricks, uint32_t nb,
-                                                           const uint8_t* __restrict__ enc_pool,
-                                                           const uint32_t* __restrict__ g_lut,
-                                                           const uint32_t* __restrict__ g_lutf, uint32_t n_models,
-                                                           uint32_t fast_models, uint32_t lanes,
-                                                           const uint32_t* __restrict__ order,
-                                                           const uint64_t* __restrict__ nib_off,
-                                                           const uint64_t* __restrict__ snap_off,
-                                                           uint32_t* __restrict__ nib, uint2* __restrict__ snap,
-                                                           uint8_t* __restrict__ chain, uint32_t L, bool write_desc) {
-    __shared__ uint32_t lut0[kTot];
-    load_fast_lut(lut0, g_lut);
+// One lane per brick, `lanes` bricks of similar length to a warp (`order`: longest first), so
+// that a warp's chains end together.  Bound by the longest brick's dependent chain; model 0's
+// bricks take ChainRing, the others index_run's forms.
+// Measured (B200; every brick in ChainFast's form, four to a warp): 256 bricks of 64^3,
+// longest 78,694 symbols, 4.26 -> 3.03 ms (106 -> 76 cycles a symbol); 2048 bricks of 64^3
+// 5.23 -> 4.51 ms, of 32^3 0.71 -> 0.63 ms; 32,768 bricks of 16^3 0.28 -> 0.17 ms.
+constexpr uint32_t kIndexThreads = 128;
+constexpr uint32_t kIndexTables = 2 * kTot * 8;
+__global__ void __launch_bounds__(kIndexThreads) index_symbols_kernel(
+    BrickDesc* __restrict__ bricks, uint32_t nb, const uint8_t* __restrict__ enc_pool, const uint32_t* __restrict__ g_lut,
+    const uint32_t* __restrict__ g_lutf, uint32_t n_models, uint32_t fast_models, uint32_t lanes,
+    const uint32_t* __restrict__ order, const uint64_t* __restrict__ nib_off, const uint64_t* __restrict__ snap_off,
+    uint32_t* __restrict__ nib, uint2* __restrict__ snap, uint8_t* __restrict__ chain, uint32_t L, bool write_desc) {
+    uint2* t = reinterpret_cast<uint2*>(idx_smem);  // model 0's entries
+    for (uint32_t i = threadIdx.x; i < kTot; i += kIndexThreads) {
+        const uint32_t g = g_lut[i];
+        const uint2 v = make_uint2(((g >> 4) & 0x1FFFu) * 16, ((i - (g >> 17)) & (kTot - 1)) * 16 | (g & 15u));
+        t[2 * i] = v;
+        t[2 * ((i & 255u) << 4 | i >> 8) + 1] = v;
+    }
     __syncthreads();
-    // The lanes of a warp take `lanes` bricks of similar length (order: longest
-    // first), so that a warp's chains end together, and one warp instruction
-    // steps them all: the longest chain then runs at its own latency instead of
-    // sharing a scheduler's issue slots with the other long chains.
     const uint32_t lane = threadIdx.x & 31;
     if (lane >= lanes) return;
-    const uint32_t slot = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lanes + lane;
+    const uint32_t slot = (blockIdx.x * (kIndexThreads >> 5) + (threadIdx.x >> 5)) * lanes + lane;
     if (slot >= nb) return;
     const uint32_t bi = order[slot];
     const BrickDesc br = bricks[bi];
@@ -488,12 +667,21 @@ __global__ void __launch_bounds__(128) index_symbols_kernel(BrickDesc* __restric
         flags = BF_TRUNCATED;
     } else {
         const uint8_t* enc = enc_pool + br.enc_off;
+        uint32_t* w = nib + nib_off[bi];
+        uint2* sn = snap + snap_off[bi];
         uint32_t pos = br.E - 4;
         uint32_t x = ((uint32_t)enc[br.E - 1] << 24) | ((uint32_t)enc[br.E - 2] << 16) |
                      ((uint32_t)enc[br.E - 3] << 8) | enc[br.E - 4];
         const bool fast = x >= kRansL && model < 32 && ((fast_models >> model) & 1u);
-        if (index_run(enc, x, pos, lut0, g_lutf, g_lut, model, fast, 0, br.nsym, nib + nib_off[bi],
-                      snap + snap_off[bi]))
+        bool more;
+        if (fast && model == 0) {
+            ChainRing c;
+            c.init(enc, x, pos, idx_smem + kIndexTables + ((threadIdx.x >> 5) * lanes + lane) * kRingPitch);
+            more = index_walk_ring(c, br.nsym, w, sn);
+        } else {
+            more = index_run(enc, x, pos, g_lutf, g_lutf, g_lut, model, fast, 0, br.nsym, w, sn);
+        }
+        if (more)
             go = L >= 2;
         else
             flags = BF_UNIFORM;  // the whole brick is palette[0]: nothing more to index
@@ -784,7 +972,7 @@ cudaError_t index_alloc(const DeviceDataset& ds, cudaStream_t st, IndexTemps& t)
         const uint64_t ns = ds.h_cost ? ds.h_cost[i] : ds.max_nsym;
         off[i] = words;
         off[nb + i] = snaps;
-        words += ns / 8 + 1;
+        words += (ns / 8 + 4) & ~3ull;  // (a brick's words start 16-byte aligned)
         snaps += ns / kSnap + 1;
     }
     std::vector<uint32_t> order(nb);
@@ -824,19 +1012,28 @@ void index_free(IndexTemps& t, cudaStream_t st) {
     t = IndexTemps();
 }
 
-// pass 1 from the stream headers: four bricks per warp, four warps per block.
-// (Measured on the 2048 bricks of a 1024 x 1024 x 512 volume of 64^3 bricks,
-// longest 126k symbols: one brick per warp 10.4 ms, its warps sharing the
-// schedulers' issue slots; 32 per warp 15.8 ms, each step slowed by 32 lanes'
-// scattered byte loads and table bank conflicts.)
-void index_pass1_serial(const DeviceDataset& ds, const IndexTemps& t, cudaStream_t st, bool write_desc) {
-    const uint32_t nb = ds.nb;
-    constexpr uint32_t lanes = 4;
-    const uint32_t per_block = 4 * lanes;
+// Pass 1 from the stream headers.  Lanes of a warp wait for each other's words done again
+// and for table bank conflicts, warps of an SM share its schedulers, and every block lays
+// out the tables, so bricks spread over warps until there are six per SM, then over lanes
+// (up to 16).  (ms by bricks per warp -- 1, 2, 4, 8, 16, 32: 256 bricks of 64^3 3.03, 3.17,
+// 3.50, 3.99, 4.73, 6.07; 2048 of 64^3 5.56, 4.35, 4.33, 5.03, 6.12, 8.03; 2048 of 32^3
+// 0.64, 0.60, 0.63, 0.72, 0.85, 1.10; 16,384 of 32^3 4.37, 2.39, 1.44, 0.99, 1.06, 1.28;
+// 32,768 of 16^3 1.14, 0.62, 0.35, 0.24, 0.17, 0.19.)
+cudaError_t index_pass1_serial(const DeviceDataset& ds, const IndexTemps& t, cudaStream_t st, bool write_desc) {
+    cudaError_t e = cudaFuncSetAttribute(index_symbols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kIndexTables + kIndexThreads * kRingPitch));
+    if (e != cudaSuccess) return e;
+    const uint32_t nb = ds.nb, warps = kIndexThreads / 32;
+    int sms = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ds.device);
+    if (e != cudaSuccess) return e;
+    const uint32_t in_flight = 6 * (uint32_t)std::max(1, sms), lanes = std::min(16u, (nb + in_flight - 1) / in_flight);
     const uint32_t nm = ds.n_models ? ds.n_models : 1u;
-    index_symbols_kernel<<<(nb + per_block - 1) / per_block, 128, 0, st>>>(
+    index_symbols_kernel<<<(nb + warps * lanes - 1) / (warps * lanes), kIndexThreads,
+                           kIndexTables + warps * lanes * kRingPitch, st>>>(
         ds.d_bricks, nb, ds.d_enc, ds.d_lut, t.lutf, nm, ds.fast_models, lanes, t.order, t.off, t.off + nb, t.nib,
         t.snap, t.chain, ds.L, write_desc);
+    return cudaGetLastError();
 }
 }  // namespace
 
@@ -877,8 +1074,7 @@ cudaError_t launch_build_index(DeviceDataset& ds, cudaStream_t st, const IndexSe
             return cudaSuccess;
         }
     } else if (e == cudaSuccess) {
-        index_pass1_serial(ds, t, st, true);
-        e = cudaGetLastError();
+        e = index_pass1_serial(ds, t, st, true);
     }
     if (e == cudaSuccess) {
         index_book_kernel<<<(nb + 3) / 4, 128, 0, st>>>(ds.d_bricks, nb, t.nib, t.off, t.chain, ds.d_ck, t.nck, ds.L,
@@ -905,10 +1101,7 @@ cudaError_t index_seeds_of(const DeviceDataset& ds, cudaStream_t st, std::vector
     std::vector<uint8_t> chain(nb);
     std::vector<BrickDesc> desc(nb);
     cudaError_t e = index_alloc(ds, st, t);
-    if (e == cudaSuccess) {
-        index_pass1_serial(ds, t, st, false);  // the dataset's descriptors stay as they are
-        e = cudaGetLastError();
-    }
+    if (e == cudaSuccess) e = index_pass1_serial(ds, t, st, false);  // the dataset's descriptors stay as they are
     if (e == cudaSuccess) e = cudaMemcpyAsync(chain.data(), t.chain, nb, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(desc.data(), ds.d_bricks, sizeof(BrickDesc) * nb, cudaMemcpyDeviceToHost, st);

@@ -1,0 +1,60 @@
+"""GPU: the seek index's serial chain pass on streams of every length and end, against the oracle's chain."""
+import struct
+
+import numpy as np
+import pytest
+
+from test_index_sidecar_gpu import SEED, decode_all, parse_sidecar
+
+pytestmark = pytest.mark.gpu
+
+
+def image(freq, brick: int, streams, nsyms) -> bytes:
+    """A version-1 image of bricks with five palette entries around these streams."""
+    cum = np.concatenate([[0], np.cumsum(freq)[:-1]])
+    out = [struct.pack("<6I", 0x43534244, 1, len(streams), brick, 16, 4096), np.asarray(freq, np.uint32).tobytes(),
+           cum.astype(np.uint32).tobytes()]
+    for i, (s, n) in enumerate(zip(streams, nsyms)):
+        out.append(struct.pack("<2I", i, 5) + np.arange(1, 6, dtype=np.uint64).tobytes() + struct.pack("<I", len(s)) + s
+                   + struct.pack("<I", n))
+    return b"".join(out)
+
+
+# symbols of frequency 1 (two bytes at once), none below 16, and almost one symbol only; few bricks (a lane per warp,
+# long streams), and enough that several share a warp
+@pytest.mark.parametrize("nb,brick,longest", [(120, 64, 9000), (3700, 16, 600)])
+@pytest.mark.parametrize("freq", [(4081,) + (1,) * 15, (256,) * 16, (2689, 347, 104, 651, 46, 201, 10, 31, 5, 1, 1, 1, 2, 3, 1, 3),
+                                  (16,) * 13 + (3856, 16, 16)])
+def test_chain_of_every_length(codec, oracle, freq, nb, brick, longest):
+    assert sum(freq) == 4096
+    rng = np.random.default_rng(nb + freq[0])
+    cum = np.concatenate([[0], np.cumsum(freq)[:-1]]).astype(np.uint32)
+    E = np.concatenate([4 + np.arange(90), rng.integers(4, 4 + longest // 3, nb - 90)])
+    ns = np.concatenate([1 + np.arange(70), rng.integers(1, longest, nb - 70)])
+    streams = [rng.integers(0, 256, e, dtype=np.uint8).tobytes() for e in E]
+    for k in range(0, nb, 3):  # a third start below 2^23, the others as an encoder leaves them
+        streams[k] = streams[k][:-1] + b"\0"
+    img = image(freq, brick, streams, ns)
+    ds = codec.open(img)
+    sc = ds.index_sidecar()
+    rows, states = parse_sidecar(sc)
+    at = 0
+    for i in range(nb):
+        want = oracle.rans_states(np.asarray(freq, np.uint32), cum, streams[i], int(ns[i]), SEED)
+        if rows[i, 2] == 0:  # the root's stop bit: no chain
+            x = struct.unpack("<I", streams[i][-4:])[0]
+            sym = int(np.searchsorted(cum, x & 4095, side="right")) - 1
+            assert sym & 1
+            continue
+        got = states[at:at + rows[i, 2]]
+        assert rows[i, 2] == -(-int(ns[i]) // SEED) and np.array_equal(got, want[:len(got)]), i
+        at += rows[i, 2]
+    # the symbols: the pieces of a sidecar's chain, stepped in the general form, index the same ops (labels of a brick
+    # that reports an error are not defined: its missing ops differ from decode to decode)
+    ds2 = codec.open(img, sidecar=sc)
+    lod = brick.bit_length() - 1
+    a, sa = decode_all(codec, ds, lod)
+    b, sb = decode_all(codec, ds2, lod)
+    assert np.array_equal(sa, sb) and np.array_equal(a[sa == 0], b[sa == 0])
+    ds.close()
+    ds2.close()
