@@ -64,6 +64,7 @@ __host__ __device__ constexpr int dec_ctas_per_sm() {
     return KL == 6 ? (sizeof(V) == 1 ? 4 : 2) : (sizeof(V) == 1 ? 9 : 6);
 }
 constexpr uint32_t kDecLevels = 6;       // parent levels 0..5 (a 64^3 brick has 7 levels)
+constexpr uint32_t kTeamLod = 5;        // requests of this LOD and finer are worth several CTAs
 constexpr uint32_t kPalCache = 1024;     // palettes up to this size are copied to shared memory
 template <class V, uint32_t KL>
 __host__ __device__ constexpr uint32_t pal_cache() { return sizeof(V) == 1 ? 256u : (KL == 6 ? kPalCache : 512u); }
@@ -152,6 +153,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if (done) return true;
     }
     return false;
+}
+
+// ---- clusters: a small batch's brick is decoded by several CTAs together
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t v;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t v;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// atomicOr on the same shared variable of the cluster's first CTA
+__device__ __forceinline__ void first_cta_or(uint32_t* p, uint32_t v) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_addr(p)));
+    asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
 // ------------------------------------------------------------------ LUT
@@ -1161,16 +1183,16 @@ __device__ __forceinline__ void st_cs_v4(uint64_t* p, uint64_t a, uint64_t b, ui
     asm volatile("st.global.cs.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
 }
 
-// Writes `cnt` copies of `v` at out[0..cnt) (out 8-byte aligned).
-__device__ void fill_labels(uint64_t* out, uint64_t cnt, uint64_t v) {
+// Writes `cnt` copies of `v` at out[0..cnt) (out 8-byte aligned), as thread `t` of `n`.
+__device__ void fill_labels(uint64_t* out, uint64_t cnt, uint64_t v, uint32_t t, uint32_t n) {
     uint64_t start = 0;
     if (((uintptr_t)out & 15) && cnt) {
-        if (threadIdx.x == 0) out[0] = v;
+        if (t == 0) out[0] = v;
         start = 1;
     }
     uint64_t pairs = (cnt - start) / 2;
-    for (uint64_t i = threadIdx.x; i < pairs; i += blockDim.x) st_cs_v2(out + start + 2 * i, v, v);
-    if (((cnt - start) & 1) && threadIdx.x == 0) out[cnt - 1] = v;
+    for (uint64_t i = t; i < pairs; i += n) st_cs_v2(out + start + 2 * i, v, v);
+    if (((cnt - start) & 1) && t == 0) out[cnt - 1] = v;
 }
 
 // Eight labels of one parent (64 bytes) at o8.
@@ -1299,8 +1321,9 @@ __device__ __forceinline__ uint32_t decode_op(uint32_t& x, uint32_t& pos, uint32
 template <bool GLOBAL, bool CLUT>
 __device__ __forceinline__ void decode_segments(const DecodeArgs& A, const BrickDesc& br, const uint8_t* enc,
                                                 const uint32_t* lut, uint32_t n_need, uint32_t nseg,
-                                                uint32_t* __restrict__ recs, uint32_t& st, uint32_t LABEL0) {
-    for (uint32_t k = threadIdx.x; k < nseg; k += blockDim.x) {
+                                                uint32_t* __restrict__ recs, uint32_t& st, uint32_t LABEL0, uint32_t t,
+                                                uint32_t nt) {
+    for (uint32_t k = t; k < nseg; k += nt) {  // thread t of nt
         const Checkpoint c = A.ck[br.ck_off + k];
         uint32_t x = c.state, pos = c.pos, sym = c.sym, ip = c.ip;
         uint32_t j = k * A.S;  // a multiple of 4 (S is)
@@ -1396,7 +1419,8 @@ __device__ __forceinline__ void load_lut(uint32_t* lut, const uint32_t* __restri
 // V = uint8_t when every requested brick's palette has fewer than 255 entries
 // (value 0xFF stands for "label 0"), uint16_t when every
 // palette of the dataset has fewer than 65535 entries (0xFFFF), else uint32_t.
-template <class V, uint32_t KL>
+// CLUSTERS: launched in clusters, which may decode a request together.
+template <class V, uint32_t KL, bool CLUSTERS>
 __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()) decode_kernel(DecodeArgs A) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     DecShared<V, KL>& S = *reinterpret_cast<DecShared<V, KL>*>(smem_raw);
@@ -1406,6 +1430,27 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
     // grid's CTAs leave; without one this is a no-op.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr uint32_t LABEL0 = sizeof(V) == 1 ? 0xFFu : (sizeof(V) == 2 ? 0xFFFFu : PIDX_LABEL0);
+
+    // the request count: fixed at launch, or produced on the device by an
+    // earlier kernel in the same stream (the serving loop's admission)
+    const uint32_t n_req = A.n_dev ? min(*A.n_dev, A.n) : A.n;
+    // A launch in clusters with no more requests than clusters (joint): request k is cluster
+    // k's.  At LOD 5 and finer its CTAs are a team: each takes a share of the rANS segments
+    // and of the last level's output, and every one of them works out the levels between for
+    // itself -- under a third of a brick's time, and nothing to exchange but the op records.
+    // Below that the first CTA decodes it alone (LOD 4 and coarser took up to 20 us longer
+    // in teams).  With more requests, as without clusters,
+    // each CTA takes whole requests from the queue.
+    const uint32_t cs = CLUSTERS ? cluster_size() : 1u, cr = CLUSTERS ? cluster_rank() : 0u;
+    const bool joint = CLUSTERS && n_req <= gridDim.x / cs;
+    uint32_t next = CLUSTERS ? blockIdx.x / cs : 0u;  // joint: the cluster's request
+    bool team = false;
+    if (joint) {
+        const uint32_t r = next < n_req ? (A.order ? A.order[next] : next) : 0xFFFFFFFFu;
+        team = r < A.n_reqs && A.reqs[r].lod >= kTeamLod;
+        if (cr && !team) return;
+    }
+    const uint32_t jt = team ? cr * T + tid : tid, jT = team ? cs * T : T;  // of the threads of a request
 
     load_lut<V>(S.lut, A.lut, tid, T);
     if (tid == 0) {
@@ -1419,21 +1464,19 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
     uint32_t phase = 0;     // parity of the stream-copy barrier
     bool stage_ok = true;   // cleared if a copy ever fails to land in time
 
-    // per-CTA scratch: op records | active-node lists of every parent level
+    // per-CTA scratch: op records (a team's: the first CTA's) | active-node lists of every parent level
     uint8_t* scr = A.scratch + (uint64_t)blockIdx.x * A.scratch_per_cta;
-    uint32_t* recs = reinterpret_cast<uint32_t*>(scr);
+    uint32_t* recs = reinterpret_cast<uint32_t*>(team ? scr - (uint64_t)cr * A.scratch_per_cta : scr);
     const uint64_t max_ops = ((1ull << (3 * A.L)) - 8) / 7;
     uint32_t* act = reinterpret_cast<uint32_t*>(scr + ((max_ops * 4 + 255) & ~255ull));
     // parent level KL (if the launch's bricks have one) in scratch, after the active lists
     V* spill = reinterpret_cast<V*>(reinterpret_cast<uint8_t*>(act) + ((4ull * lvl_off(A.L - 1) + 255) & ~255ull));
 
-    // the request count: fixed at launch, or produced on the device by an
-    // earlier kernel in the same stream (the serving loop's admission)
-    const uint32_t n_req = A.n_dev ? min(*A.n_dev, A.n) : A.n;
     uint32_t cur_model = 0;  // the LUT in shared memory is model 0's
     for (;;) {
         if (tid == 0) {
-            const uint32_t k = atomicAdd(A.queue, 1u);
+            const uint32_t k = joint ? next : atomicAdd(A.queue, 1u);
+            if (CLUSTERS) next = 0xFFFFFFFFu;
             // an optional schedule (longest brick first, or one part of a
             // split by output size) maps queue slots to requests
             uint32_t wk = 0xFFFFFFFFu;  // past the end of the queue
@@ -1445,7 +1488,8 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
                 if (S.req.brick < A.nb) S.br = A.bricks[S.req.brick];
             }
         }
-        __syncthreads();
+        if (team) cluster_sync();  // (every CTA's status is reset before another adds to it)
+        else __syncthreads();
         const uint32_t w = S.work;
         if (w == 0xFFFFFFFFu) break;
         if (w >= A.n_reqs) {  // an order entry naming no request: nothing to decode or report
@@ -1459,7 +1503,7 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
         // op records of levels 1..t in scratch, both sized for A.L levels
         const uint32_t Lb = (S.br.flags >> BF_LEVELS_SHIFT) & 15u, model = (S.br.flags >> BF_MODEL_SHIFT) & 255u;
         if (req.brick >= A.nb || t >= Lb || t >= A.L || model >= A.n_models) {
-            if (tid == 0) A.status[w] = CSV_BRICK_BADREQ;
+            if (jt == 0) A.status[w] = CSV_BRICK_BADREQ;
             __syncthreads();
             continue;
         }
@@ -1473,9 +1517,10 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
             cur_model = model;
         }
         const BrickDesc br = S.br;
-        // stage the compressed stream in shared memory (one bulk copy) while the palette loads
+        // stage the compressed stream in shared memory (one bulk copy) while the palette loads (a team's
+        // CTA reads its share from memory)
         const uint32_t E16 = (br.E + 15u) & ~15u;
-        const bool stage = stage_ok && t > 0 && !(br.flags & BF_UNIFORM) && E16 >= 16 && E16 <= A.stage_cap;
+        const bool stage = !team && stage_ok && t > 0 && !(br.flags & BF_UNIFORM) && E16 >= 16 && E16 <= A.stage_cap;
         if (stage && tid == 0) bulk_copy_g2s(S.val, A.enc + br.enc_off, E16, &S.bar);
         uint64_t* out = A.out + req.dst;
         const uint64_t* gpal = A.pal + br.pal_off;
@@ -1489,7 +1534,7 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
         __syncthreads();
 
         if (t == 0 || (br.flags & BF_UNIFORM)) {
-            fill_labels(out, 1ull << (3 * t), pal[0]);
+            fill_labels(out, 1ull << (3 * t), pal[0], jt, jT);
         } else {
             // ---- 1. rANS segments -> op records
             // (level_start is read from shared memory: a runtime index into a
@@ -1510,10 +1555,12 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
             }
             if (staged)
                 decode_segments<false, compact_lut<V>()>(A, br, reinterpret_cast<const uint8_t*>(S.val), S.lut, n_need, nseg, recs,
-                                       st, LABEL0);
+                                       st, LABEL0, jt, jT);
             else
-                decode_segments<true, compact_lut<V>()>(A, br, A.enc + br.enc_off, S.lut, n_need, nseg, recs, st, LABEL0);
-            __syncthreads();  // the staged stream is dead: its space becomes the level arrays
+                decode_segments<true, compact_lut<V>()>(A, br, A.enc + br.enc_off, S.lut, n_need, nseg, recs, st, LABEL0, jt,
+                                                           jT);
+            if (team) cluster_sync();  // all of the brick's records
+            else __syncthreads();       // the staged stream is dead: its space becomes the level arrays
             if (S.rewait) {
                 // The late copy must land before the staging region is written: a second
                 // bounded wait on the same phase.  If it gives up too, this brick is
@@ -1636,7 +1683,7 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
                     // of contiguous output.  Stop-filled parents first: chunk q is
                     // children 4(q&1) .. 4(q&1)+3 of parent q / 2.
                     const uint32_t n_chunk = 2 * n_par;
-                    for (uint32_t q = tid; q < n_chunk; q += T) {
+                    for (uint32_t q = jt; q < n_chunk; q += jT) {
                         const uint32_t p = q >> 1;
                         if (!is_active(Vw, p)) {
                             const uint64_t x = label_of(pal, Vw.val[p], LABEL0);
@@ -1657,13 +1704,13 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
                                            get_rec(Vw, i0 + 3));
                         }
                     };
-                    uint32_t g = tid >> 1, p_next = 0;
+                    uint32_t g = jt >> 1, p_next = 0;
                     uint4 r_next = make_uint4(0, 0, 0, 0);
                     if (g < n_act) fetch(g, p_next, r_next);
-                    for (; g < n_act; g += T >> 1) {
+                    for (; g < n_act; g += jT >> 1) {
                         const uint32_t p = p_next;
                         const uint4 r = r_next;
-                        if (g + (T >> 1) < n_act) fetch(g + (T >> 1), p_next, r_next);
+                        if (g + (jT >> 1) < n_act) fetch(g + (jT >> 1), p_next, r_next);
                         const uint32_t n0 = 8 * p + 4 * half;
                         const uint64_t a = label_of(pal, resolve(Vw, r.x, n0, lc, &bad), LABEL0);
                         const uint64_t b = label_of(pal, resolve(Vw, r.y, n0 + 1, lc, &bad), LABEL0);
@@ -1677,7 +1724,7 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
                     // contiguous bytes.  Stop-filled parents: chunk q is children
                     // 2q, 2q+1 of parent q / 4.
                     const uint32_t n_chunk = 4 * n_par;
-                    for (uint32_t q = tid; q < n_chunk; q += T) {
+                    for (uint32_t q = jt; q < n_chunk; q += jT) {
                         const uint32_t p = q >> 2;
                         if (!is_active(Vw, p)) {
                             const uint64_t x = label_of(pal, Vw.val[p], LABEL0);
@@ -1707,11 +1754,11 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
                             r1 = get_rec(Vw, i0 + 1);
                         }
                     };
-                    uint32_t g = tid >> 2, p_next = 0, r0_next = 0, r1_next = 0;
+                    uint32_t g = jt >> 2, p_next = 0, r0_next = 0, r1_next = 0;
                     if (g < n_act) fetch(g, p_next, r0_next, r1_next);
-                    for (; g < n_act; g += T >> 2) {
+                    for (; g < n_act; g += jT >> 2) {
                         const uint32_t p = p_next, r0 = r0_next, r1 = r1_next;
-                        if (g + (T >> 2) < n_act) fetch(g + (T >> 2), p_next, r0_next, r1_next);
+                        if (g + (jT >> 2) < n_act) fetch(g + (jT >> 2), p_next, r0_next, r1_next);
                         const uint32_t n0 = 8 * p + 2 * sub;
                         const uint64_t a = label_of(pal, resolve(Vw, r0, n0, lc, &bad), LABEL0);
                         const uint64_t b = label_of(pal, resolve(Vw, r1, n0 + 1, lc, &bad), LABEL0);
@@ -1729,7 +1776,11 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
         if (bad) st |= CSV_BRICK_BADOP;
         if (st) atomicOr(&S.status, st);
         __syncthreads();
-        if (tid == 0) A.status[w] = S.status;
+        if (team) {
+            if (cr && tid == 0 && S.status) first_cta_or(&S.status, S.status);
+            cluster_sync();
+        }
+        if (jt == 0) A.status[w] = S.status;
         __syncthreads();
     }
     // Launched as a programmatic dependent: finish only after the kernel before
@@ -1753,10 +1804,12 @@ template <class V, uint32_t KL>
 static int occupancy(int device) {
     int& occ = g_dec_occ[2 * (sizeof(V) == 1 ? 2 : sizeof(V) == 2 ? 0 : 1) + (KL == kDecLevels ? 0 : 1)][device & 63];
     if (occ == 0) {
-        cudaFuncSetAttribute(decode_kernel<V, KL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(decode_kernel<V, KL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(DecShared<V, KL>));
+        cudaFuncSetAttribute(decode_kernel<V, KL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(DecShared<V, KL>));
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_kernel<V, KL>, dec_threads<V, KL>(),
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_kernel<V, KL, false>, dec_threads<V, KL>(),
                                                       sizeof(DecShared<V, KL>));
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -1806,24 +1859,49 @@ static cudaError_t launch_variant(const DecodeArgs& A0, const DecodeScratch& scr
     }
     A.scratch_per_cta = decode_scratch_per_cta(1u << (A.L - 1), KL);
     const uint64_t cap = scr.bytes / A.scratch_per_cta;
-    if (grid > A.n) grid = A.n;
-    if (grid > cap) grid = (uint32_t)cap;
+    grid = (uint32_t)std::min<uint64_t>(grid, cap);
+    // CTAs per cluster: a brick decoded by more CTAs ends sooner while they find free SMs, and
+    // eight or four of them take up more than they bring when threads crowd.  (B200, us by CTAs per
+    // brick -- 1, 2, 4, 8.  64^3 bricks at LOD 6, 8-bit values: 4 bricks 186, 135, 106, 89; 24 bricks
+    // 210, 147, 116, 111; 74 bricks 235, 168, 155, 196; 148 bricks 240, 201, 243, 245; 290 bricks 301,
+    // 290.  16-bit values: 24 bricks 328, 212, 147, 124; 74 bricks 350, 230, 227; 148 bricks 377, 284.
+    // 32^3 bricks: 24 bricks 87, 70, 58, 56; 148 bricks 90, 75, 73, 98.)  Requests counted on the
+    // device: four, which the kernel uses while they are no more than a quarter of the CTAs.
+    uint32_t cs = 1;
+    if (!(cfg && (cfg->pdl || cfg->ctas_per_sm)) && A.L > kTeamLod) {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        const uint64_t threads = (uint64_t)A.n * dec_threads<V, KL>(), sm = (uint64_t)std::max(sms, 1);
+        if (A.n_dev) cs = 4;
+        else if (8 * threads <= 1024 * sm) cs = 8;
+        else if (4 * threads <= 1400 * sm) cs = 4;
+        else if (2 * (uint64_t)A.n <= grid) cs = 2;
+        while (cs > 1 && (A.n_dev ? cs : cs * (uint64_t)A.n) > grid) cs /= 2;  // (little scratch)
+    }
+    if (A.n_dev) grid -= grid % cs;
+    else grid = (uint32_t)std::min<uint64_t>(grid, (uint64_t)A.n * cs);
     if (grid == 0) return cudaErrorInvalidValue;
     A.stage_cap = (cfg && !cfg->stage) ? 0u : stage_cap<V, KL>();
-    if (cfg && cfg->pdl) {
+    if (cs > 1 || (cfg && cfg->pdl)) {
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(grid);
         lc.blockDim = dim3(dec_threads<V, KL>());
         lc.dynamicSmemBytes = sizeof(DecShared<V, KL>);
         lc.stream = st;
         cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = 1;
+        if (cs > 1) {
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = cs;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        } else {
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+        }
         lc.attrs = at;
         lc.numAttrs = 1;
-        return cudaLaunchKernelEx(&lc, decode_kernel<V, KL>, A);
+        return cudaLaunchKernelEx(&lc, cs > 1 ? decode_kernel<V, KL, true> : decode_kernel<V, KL, false>, A);
     }
-    decode_kernel<V, KL><<<grid, dec_threads<V, KL>(), sizeof(DecShared<V, KL>), st>>>(A);
+    decode_kernel<V, KL, false><<<grid, dec_threads<V, KL>(), sizeof(DecShared<V, KL>), st>>>(A);
     return cudaGetLastError();
 }
 
