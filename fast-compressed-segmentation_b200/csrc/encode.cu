@@ -44,8 +44,8 @@ constexpr uint32_t OP_PALNEED = 7;  // placeholder code until the palette walk d
 constexpr uint32_t EF_UNIFORM = 1u, EF_OVERFLOW = 2u;
 // Encoder counters (u64 words): 0 nibble pool head, 1 palette pool head,
 // 2..17 the sampled bricks' nibble histogram, 18 the brick work queue (low
-// 32 bits), 19 checkpoint pool head.
-constexpr uint32_t kMiscQueue = 18, kMiscCk = 19, kMiscWords = 32;
+// 32 bits), 19 checkpoint pool head, 20 stream pool head, 21 the image's length.
+constexpr uint32_t kMiscQueue = 18, kMiscCk = 19, kMiscEnc = 20, kMiscImage = 21, kMiscWords = 32;
 constexpr uint32_t kModes = 12;
 constexpr uint32_t kMaxTables = 16;
 constexpr uint32_t kModelWords = 65;  // freq[16] cum[16] total M[16] shift[16]
@@ -76,9 +76,9 @@ struct EncoderState {
     size_t pal_cap = 0;
     uint8_t* d_enc = nullptr;
     size_t enc_cap = 0;
-    uint64_t* d_enc_off = nullptr;
     uint64_t* d_rec_off = nullptr;
-    size_t off_cap = 0, rec_cap = 0;
+    size_t rec_cap = 0;
+    uint64_t enc_need = 0;  // bytes of the stream pool that the last K1 gave out
     uint8_t* d_scratch = nullptr;
     size_t scratch_cap = 0;
     unsigned long long* d_misc = nullptr;  // [0] nib head, [1] pal head, [2..17] histogram, [18] queue
@@ -89,7 +89,13 @@ struct EncoderState {
     uint32_t n_tables = 1;                       // rANS models of the last image
     uint32_t tab_freq[16][16] = {}, tab_cum[16][16] = {};
     bool v2 = false;
-    std::vector<EncMeta> h_meta;
+    // page-locked: what an encode reads back
+    EncMeta* h_meta = nullptr;
+    size_t h_meta_cap = 0;
+    struct Words {
+        unsigned long long misc[kMiscWords];
+        uint32_t model[kModelWords];
+    }* h_words = nullptr;
     bool valid = false;
 };
 
@@ -102,12 +108,13 @@ void encoder_state_free(EncoderState* s) {
     cudaFree(s->d_nib);
     cudaFree(s->d_pal);
     cudaFree(s->d_enc);
-    cudaFree(s->d_enc_off);
     cudaFree(s->d_rec_off);
     cudaFree(s->d_scratch);
     cudaFree(s->d_misc);
     cudaFree(s->d_model);
     cudaFree(s->d_image);
+    cudaFreeHost(s->h_meta);
+    cudaFreeHost(s->h_words);
     delete s;
 }
 
@@ -170,7 +177,7 @@ struct EncFixed {
     uint32_t hist[64];
     uint32_t level_r[8];  // active nodes before level l's, l = 0 .. L - 1
     uint32_t work, P, n_pd, n_act;
-    uint64_t nib_off, pal_off, ck_off;
+    uint64_t nib_off, pal_off, ck_off, enc_off;
 };
 __host__ __device__ inline uint32_t enc_lab_nodes(uint32_t L) {
     return lvl_off(L - 1 < kEncSmemLevels ? L - 1 : kEncSmemLevels);
@@ -700,6 +707,8 @@ __global__ void __launch_bounds__(T, PER_SM) enc_bricks_kernel(EncArgs A) {
             S.ck_off = atomicAdd(A.misc + kMiscCk, (unsigned long long)n_ck);
             S.nib_off = atomicAdd(A.misc + 0, (unsigned long long)((nbytes + 15) & ~15u));
             S.pal_off = atomicAdd(A.misc + 1, (unsigned long long)P);
+            // its stream: <= 2 bytes per symbol + flush
+            S.enc_off = atomicAdd(A.misc + kMiscEnc, (4ull * nbytes + 4 + 15) & ~15ull);
         }
         if (tid < 16) S.hist[tid] = 0;
         // staging: packed nibbles from position `base` (a multiple of 32) on, nibble k at bit 4 k
@@ -806,7 +815,7 @@ __global__ void __launch_bounds__(T, PER_SM) enc_bricks_kernel(EncArgs A) {
             EncMeta m;
             m.nib_off = nib_off;
             m.pal_off = pal_off;
-            m.enc_off = 0;
+            m.enc_off = S.enc_off;
             m.P = P;
             m.nsym = nsym;
             m.nbytes = nbytes;
@@ -991,7 +1000,7 @@ static_assert(sizeof(RansBrick<64>) % 128 == 16, "eight bricks' entries are read
 template <int K, uint32_t kRansBatch>
 __global__ void __launch_bounds__(32 * (K + 1)) enc_rans_kernel(EncMeta* __restrict__ meta, uint32_t nb,
                                                                 const uint8_t* __restrict__ nib_pool,
-                                                                const uint64_t* __restrict__ enc_off,
+                                                                uint64_t* __restrict__ rec_size, uint32_t rec_fixed,
                                                                 uint8_t* __restrict__ enc_pool,
                                                                 const uint32_t* __restrict__ model, uint32_t n_tables,
                                                                 Checkpoint* __restrict__ ck_all, uint32_t n_sm) {
@@ -1053,7 +1062,7 @@ __global__ void __launch_bounds__(32 * (K + 1)) enc_rans_kernel(EncMeta* __restr
         nib_off = m.nib_off;
         tables = min((m.sel >> 4) & 15u, n_tables - 1);
         ck += m.ck_off;
-        out += enc_off[i];
+        out += m.enc_off;
     }
     if (lane < 16) B.tab[lane] = rans_entry(model + tables * kModelWords, lane);
     // the packed nibbles start 16-byte aligned and are padded to 16: a chunk of 32 symbols is 16 bytes
@@ -1147,7 +1156,10 @@ __global__ void __launch_bounds__(32 * (K + 1)) enc_rans_kernel(EncMeta* __restr
             if (n == n_batches) {
                 const uint32_t x = B.end[d];
                 if (lane < 4) out[emitted + lane] = (uint8_t)(x >> (8 * lane));  // ransFlush, little-endian
-                if (lane == 0) meta[i].E = emitted + 4;
+                if (lane == 0) {
+                    meta[i].E = emitted + 4;
+                    rec_size[i] = rec_fixed + 8ull * meta[i].P + emitted + 4;  // the brick's record in the image
+                }
             }
             __syncwarp();  // its steps make room for new ones
         }
@@ -1157,16 +1169,52 @@ __global__ void __launch_bounds__(32 * (K + 1)) enc_rans_kernel(EncMeta* __restr
 }
 
 // ------------------------------------------------------------ K4 serialize
+// The records' sizes become their places in the image, after a header of `first` bytes;
+// the image's length goes to *total.  One block, 4096 records a turn.
+__global__ void __launch_bounds__(1024) place_kernel(uint64_t* __restrict__ rec, uint32_t nb, uint64_t first,
+                                                     unsigned long long* __restrict__ total) {
+    __shared__ uint64_t sh[33];
+    for (uint32_t base = 0; base < nb; base += 4096) {
+        const uint32_t i = base + 4 * threadIdx.x;
+        uint64_t v[4], sum = 0, all;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) sum += v[k] = i + k < nb ? rec[i + k] : 0ull;
+        uint64_t at = first + block_exclusive<uint64_t>(sum, sh, &all);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (i + k < nb) rec[i + k] = at;
+            at += v[k];
+        }
+        first += all;
+    }
+    if (threadIdx.x == 0) *total = first;
+}
+
 // One block per brick record: ID, P, palette, E, stream, nSymbols (fileIO.cpp:57-96).
 // Version 2 adds a u32 after the ID: the brick's table (bits 4..7) and mode (bits 0..3).
-__global__ void serialize_kernel(const EncMeta* __restrict__ meta, const uint64_t* __restrict__ rec_off,
+// Block nb writes the header: version 1, 152 bytes (fileIO.cpp:25-49); version 2, 28 bytes
+// and 128 per table.  Nothing is written when the image is longer than `cap`.
+__global__ void serialize_kernel(const EncMeta* __restrict__ meta, uint32_t nb, const uint64_t* __restrict__ rec_off,
                                  const uint64_t* __restrict__ pal_pool, const uint8_t* __restrict__ enc_pool,
-                                 const uint64_t* __restrict__ enc_off, uint8_t* __restrict__ image, uint32_t v2) {
+                                 uint8_t* __restrict__ image, uint64_t cap, const unsigned long long* __restrict__ len,
+                                 const uint32_t* __restrict__ model, uint32_t n_tables, uint32_t b) {
+    if (*len > cap) return;
     const uint32_t i = blockIdx.x;
+    const bool v2 = n_tables > 0;
+    if (i == nb) {
+        uint32_t* hdr = reinterpret_cast<uint32_t*>(image);
+        // the reference always writes BRICK_SIZE after the brick count (fileIO.cpp:28)
+        const uint32_t fixed[7] = {kMagic, v2 ? 2u : 1u, nb, b, 16u, model[32], n_tables};
+        if (threadIdx.x == 0)
+            for (uint32_t k = 0; k < (v2 ? 7u : 6u); ++k) hdr[k] = fixed[k];
+        for (uint32_t k = threadIdx.x; k < 32 * max(1u, n_tables); k += blockDim.x)
+            hdr[(v2 ? 7 : 6) + k] = model[(k >> 5) * kModelWords + (k & 31u)];
+        return;
+    }
     const EncMeta m = meta[i];
     uint8_t* dst = image + rec_off[i];
     const uint8_t* pal = reinterpret_cast<const uint8_t*>(pal_pool + m.pal_off);
-    const uint8_t* enc = enc_pool + enc_off[i];
+    const uint8_t* enc = enc_pool + m.enc_off;
     const uint64_t pb = 8ull * m.P;
     const uint64_t h = v2 ? 12 : 8;  // ID [, sel], P
     const uint64_t total = h + 8 + pb + m.E;
@@ -1373,6 +1421,7 @@ int encode_device(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W
         static_assert(sizeof(unsigned long long) == 8, "");
         if (!s->d_misc) CK(cudaMalloc(&s->d_misc, kMiscWords * sizeof(unsigned long long)));
     }
+    if (!s->h_words) CK(cudaMallocHost(&s->h_words, sizeof *s->h_words));
     const bool wide = enc_wide(levels_of(b), nb, device);
     const uint32_t grid = std::min<uint32_t>(enc_grid(device, levels_of(b), wide), std::max<uint32_t>(nb, 1));
     const size_t per_cta = enc_scratch_per_cta(levels_of(b), wide);
@@ -1419,10 +1468,11 @@ int encode_device(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W
             });
             CK(cudaGetLastError());
         }
-        unsigned long long misc[kMiscWords];
-        CK(cudaMemcpyAsync(misc, s->d_misc, sizeof misc, cudaMemcpyDeviceToHost, st));
+        const unsigned long long* misc = s->h_words->misc;
+        CK(cudaMemcpyAsync(s->h_words->misc, s->d_misc, sizeof s->h_words->misc, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         s->ck_used = misc[kMiscCk];
+        s->enc_need = misc[kMiscEnc];
         if (misc[0] <= s->nib_cap && misc[1] <= s->pal_cap && misc[kMiscCk] <= s->ck_cap_total) break;
         if (attempt == 1) {
             err = "encoder pools overflowed twice";
@@ -1433,10 +1483,7 @@ int encode_device(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W
         ck_need = std::max<size_t>(ck_need, misc[kMiscCk]);
     }
     if (hist_out) {  // a shard: stop here with the sample histogram; finish_encode_shard completes it
-        unsigned long long h[16];
-        CK(cudaMemcpyAsync(h, s->d_misc + 2, sizeof h, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        for (int k = 0; k < 16; ++k) hist_out[k] = h[k];
+        for (int k = 0; k < 16; ++k) hist_out[k] = s->h_words->misc[2 + k];
         s->bricks_done = true;
         return CSV_OK;
     }
@@ -1470,86 +1517,61 @@ static int finish_encode(EncoderState* s, const EncodeSelection* sel, cudaStream
         model_kernel<<<1, 1, 0, st>>>(s->d_misc + 2, s->d_model);
         CK(cudaGetLastError());
     }
-    s->h_meta.resize(nb);
-    if (nb) CK(cudaMemcpyAsync(s->h_meta.data(), s->d_meta, sizeof(EncMeta) * nb, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(models.data(), s->d_model, kModelWords * sizeof(uint32_t) * std::max<uint32_t>(1, n_tables),
-                       cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    const uint32_t* model = models.data();
-    s->n_tables = std::max<uint32_t>(1, n_tables);
-    for (uint32_t t = 0; t < s->n_tables; ++t)
-        for (int k = 0; k < 16; ++k) {
-            s->tab_freq[t][k] = models[t * kModelWords + k];
-            s->tab_cum[t][k] = models[t * kModelWords + 16 + k];
-        }
-    s->v2 = v2;
-    std::vector<uint64_t> enc_off(std::max<uint32_t>(nb, 1)), rec_off(std::max<uint32_t>(nb, 1));
-    uint64_t eo = 0;
-    for (uint32_t i = 0; i < nb; ++i) {
-        enc_off[i] = eo;
-        eo += (4ull * s->h_meta[i].nbytes + 4 + 15) & ~15ull;  // <= 2 bytes per symbol + flush
+    if (nb > s->h_meta_cap) {
+        cudaFreeHost(s->h_meta);
+        s->h_meta = nullptr;
+        s->h_meta_cap = 0;
+        const size_t cap = std::max<size_t>(4096, nb + nb / 2);
+        CK(cudaMallocHost(&s->h_meta, sizeof(EncMeta) * cap));
+        s->h_meta_cap = cap;
     }
-    CK(grow(&s->d_enc, &s->enc_cap, std::max<uint64_t>(eo, 16)));
-    CK(grow(&s->d_enc_off, &s->off_cap, std::max<uint32_t>(nb, 1)));
+    s->n_tables = std::max<uint32_t>(1, n_tables);
+    s->v2 = v2;
+    CK(grow(&s->d_enc, &s->enc_cap, std::max<uint64_t>(s->enc_need, 16)));
     CK(grow(&s->d_rec_off, &s->rec_cap, std::max<uint32_t>(nb, 1)));
-    CK(cudaMemcpyAsync(s->d_enc_off, enc_off.data(), 8ull * nb, cudaMemcpyHostToDevice, st));
     if (nb) {
         const uint32_t n_sm = (uint32_t)sm_count(s->device);
         auto rans = [&](auto kernel, uint32_t K) {
-            kernel<<<(nb + K - 1) / K, 32 * (K + 1), 0, st>>>(s->d_meta, nb, s->d_nib, s->d_enc_off, s->d_enc,
-                                                             s->d_model, s->n_tables, s->d_ck, n_sm);
+            kernel<<<(nb + K - 1) / K, 32 * (K + 1), 0, st>>>(s->d_meta, nb, s->d_nib, s->d_rec_off, v2 ? 20u : 16u,
+                                                             s->d_enc, s->d_model, s->n_tables, s->d_ck, n_sm);
         };
         if (nb <= 4 * n_sm) rans(enc_rans_kernel<1, 128>, 1);
         else if (nb <= 16 * n_sm) rans(enc_rans_kernel<4, 64>, 4);
         else rans(enc_rans_kernel<8, 64>, 8);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(s->h_meta.data(), s->d_meta, sizeof(EncMeta) * nb, cudaMemcpyDeviceToHost, st));
     }
-    CK(cudaStreamSynchronize(st));
-    // version 1: 152-byte header (fileIO.cpp:25-49); version 2: 28 bytes + 128 per table
-    const uint64_t hdr_bytes = v2 ? 28 + 128ull * n_tables : kHeaderBytes;
-    uint64_t ro = hdr_bytes;
-    for (uint32_t i = 0; i < nb; ++i) {
-        s->h_meta[i].enc_off = enc_off[i];
-        rec_off[i] = ro;
-        ro += (v2 ? 20 : 16) + 8ull * s->h_meta[i].P + s->h_meta[i].E;
-    }
-    CK(grow(&s->d_image, &s->image_cap, ro));
-    CK(cudaMemcpyAsync(s->d_rec_off, rec_off.data(), 8ull * nb, cudaMemcpyHostToDevice, st));
-    std::vector<uint32_t> hdr(hdr_bytes / 4);
-    hdr[0] = kMagic;
-    hdr[1] = v2 ? 2 : 1;
-    hdr[2] = nb;
-    hdr[3] = b;  // the reference always writes BRICK_SIZE here (fileIO.cpp:28)
-    hdr[4] = 16;
-    hdr[5] = model[32];
-    if (!v2) {
-        for (int k = 0; k < 16; ++k) {
-            hdr[6 + k] = model[k];
-            hdr[22 + k] = model[16 + k];
+    place_kernel<<<1, 1024, 0, st>>>(s->d_rec_off, nb, v2 ? 28 + 128ull * n_tables : kHeaderBytes,
+                                     s->d_misc + kMiscImage);
+    // The image is written without waiting for its length: once more when it is longer than the last one's buffer.
+    for (int pass = 0; pass < 2; ++pass) {
+        serialize_kernel<<<nb + 1, 256, 0, st>>>(s->d_meta, nb, s->d_rec_off, s->d_pal, s->d_enc, s->d_image, s->image_cap,
+                                                 s->d_misc + kMiscImage, s->d_model, n_tables, b);
+        CK(cudaGetLastError());
+        if (pass == 0) {
+            if (nb) CK(cudaMemcpyAsync(s->h_meta, s->d_meta, sizeof(EncMeta) * nb, cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpyAsync(s->h_words->misc + kMiscImage, s->d_misc + kMiscImage, sizeof(unsigned long long),
+                               cudaMemcpyDeviceToHost, st));
+            if (!v2)
+                CK(cudaMemcpyAsync(s->h_words->model, s->d_model, sizeof s->h_words->model, cudaMemcpyDeviceToHost, st));
         }
-    } else {
-        hdr[6] = n_tables;
-        for (uint32_t t = 0; t < n_tables; ++t)
-            for (int k = 0; k < 16; ++k) {
-                hdr[7 + 32 * t + k] = models[t * kModelWords + k];
-                hdr[7 + 32 * t + 16 + k] = models[t * kModelWords + 16 + k];
-            }
+        CK(cudaStreamSynchronize(st));
+        if (s->h_words->misc[kMiscImage] <= s->image_cap) break;
+        CK(grow(&s->d_image, &s->image_cap, s->h_words->misc[kMiscImage]));
     }
+    if (!v2) memcpy(models.data(), s->h_words->model, sizeof s->h_words->model);
+    const uint32_t* model = models.data();
+    for (uint32_t t = 0; t < s->n_tables; ++t)
+        for (int k = 0; k < 16; ++k) {
+            s->tab_freq[t][k] = models[t * kModelWords + k];
+            s->tab_cum[t][k] = models[t * kModelWords + 16 + k];
+        }
     for (int k = 0; k < 16; ++k) {
         s->freq[k] = model[k];
         s->cum[k] = model[16 + k];
     }
     s->cum[16] = model[32];
-    CK(cudaMemcpyAsync(s->d_image, hdr.data(), hdr_bytes, cudaMemcpyHostToDevice, st));
-    if (nb) {
-        serialize_kernel<<<nb, 256, 0, st>>>(s->d_meta, s->d_rec_off, s->d_pal, s->d_enc, s->d_enc_off, s->d_image,
-                                             v2 ? 1u : 0u);
-        CK(cudaGetLastError());
-    }
-    CK(cudaStreamSynchronize(st));
 #undef CK
-    s->image_len = ro;
+    s->image_len = s->h_words->misc[kMiscImage];
     s->valid = true;
     return CSV_OK;
 }

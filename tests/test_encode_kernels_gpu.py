@@ -86,3 +86,26 @@ def test_bricks_forms(codec, oracle, shape):
     n = codec.encode_device(torch.from_numpy(vol.view(np.int64)).cuda(), 32)
     img = bytes(codec.encoded_image_tensor().cpu().numpy())
     assert len(img) == n and img == oracle.encode(vol, 32)
+
+
+# the records' places in turns of 4096 bricks, and an image that outgrows the last one's buffer, then a smaller one
+@pytest.mark.parametrize("shapes", [((2, 2, 1), (32, 32, 32), (2, 482, 34), (4, 482, 34), (6, 4, 2))])
+@pytest.mark.parametrize("v2", [False, True])
+def test_record_places(codec, oracle, shapes, v2):
+    import torch
+    from csvb200 import Codec
+    fresh, b = Codec(0), 8 if v2 else 2
+    for shape in shapes:
+        shape = tuple(n * b // 2 for n in shape)
+        vol = _volume(shape, sum(shape))
+        d = torch.from_numpy(vol.view(np.int64)).cuda()
+        nb = int(np.prod([-(-n // b) for n in shape]))
+        if v2:
+            tables, sel = _tables([2, 300]), (np.arange(nb) % 2 << 4).astype(np.uint8)
+            fresh.encode_device_sel(d, b, tables, torch.from_numpy(sel).cuda())
+            want = oracle.encode_sel(vol, b, sel, tables)
+        else:
+            fresh.encode_device(d, b)
+            want = oracle.encode(vol, b)
+        assert bytes(fresh.encoded_image_tensor().cpu().numpy()) == want
+    fresh.close()
