@@ -908,41 +908,35 @@ __global__ void __launch_bounds__(T, PER_SM) enc_stats_kernel(EncArgs A, uint32_
 // (x * M) >> (31 + s) exactly for every x < 2^31 (the encoder's state bound):
 // M = 2^(31+s)/f + e with 0 <= e < 1 adds less than x / 2^(31+s) < 2^-s <= 1/f
 // to x/f, whose fractional part is at most 1 - 1/f (Granlund & Montgomery 1994).
+// One warp, a lane per symbol: 8 -> 3 us against one thread.
 __global__ void model_kernel(const unsigned long long* hist, uint32_t* model) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    uint32_t freq[16];
-    uint64_t raw = 0, norm = 0;
-    for (int i = 0; i < 16; ++i) {
-        uint32_t f = (uint32_t)hist[i];  // size_t -> uint32_t as :157
-        if (f == 0) f = 1;
-        freq[i] = f;
-        raw += f;
+    const uint32_t i = threadIdx.x, FULL = 0xFFFFFFFFu;
+    const bool on = i < 16;
+    uint32_t freq = on ? max((uint32_t)hist[i], 1u) : 0u;  // size_t -> uint32_t as :157
+    uint64_t raw = freq;
+    for (int d = 16; d > 0; d >>= 1) raw += __shfl_xor_sync(FULL, raw, d);
+    if (on) freq = (uint32_t)max((uint64_t)freq * kTot / raw, (uint64_t)1);
+    uint32_t norm = __reduce_add_sync(FULL, freq);
+    if (norm < kTot && i == 0) freq += kTot - norm;
+    for (; norm > kTot; --norm) {  // (at most 16 too many) from the first of the largest
+        const uint32_t most = __reduce_max_sync(FULL, freq);
+        if (most <= 1) break;
+        const uint32_t first = __ffs(__ballot_sync(FULL, freq == most)) - 1;
+        if (i == first) --freq;
     }
-    for (int i = 0; i < 16; ++i) {
-        uint64_t s = ((uint64_t)freq[i] * kTot) / raw;
-        if (s == 0) s = 1;
-        freq[i] = (uint32_t)s;
-        norm += s;
+    uint32_t end = freq;
+    for (int d = 1; d < 16; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, end, d);
+        if ((int)i >= d) end += y;
     }
-    while (norm < kTot) { freq[0]++; norm++; }
-    while (norm > kTot) {
-        int largest = 0;
-        for (int i = 1; i < 16; ++i)
-            if (freq[i] > freq[largest]) largest = i;
-        if (freq[largest] > 1) { freq[largest]--; norm--; } else break;
-    }
-    uint32_t acc = 0;
-    for (int i = 0; i < 16; ++i) {
-        model[i] = freq[i];
-        model[16 + i] = acc;
-        acc += freq[i];
-        uint32_t s = 0;
-        while ((1u << s) < freq[i]) ++s;
-        uint64_t M = ((1ull << (31 + s)) + freq[i] - 1) / freq[i];
-        model[33 + i] = (uint32_t)M;
+    if (on) {
+        model[i] = freq;
+        model[16 + i] = end - freq;
+        const uint32_t s = freq > 1 ? 32 - __clz(freq - 1) : 0;
+        model[33 + i] = (uint32_t)(((1ull << (31 + s)) + freq - 1) / freq);
         model[49 + i] = 31 + s;
     }
-    model[32] = acc;
+    if (i == 15) model[32] = end;
 }
 
 // ------------------------------------------------------------ K3 rANS
@@ -1190,6 +1184,19 @@ __global__ void __launch_bounds__(1024) place_kernel(uint64_t* __restrict__ rec,
     if (threadIdx.x == 0) *total = first;
 }
 
+// `n` bytes from src to dst by the block, whole words of dst where they can be (from two words
+// of src): 6.5 MB of 512 bricks' records 47 -> 13 us, 4.8 MB of 320 bricks' 65 -> 17 us against a
+// byte per thread.
+__device__ __forceinline__ void copy_bytes(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, uint64_t n) {
+    const uint64_t head = min(n, (uint64_t)(-(uintptr_t)dst & 3u)), words = (n - head) / 4, tail = head + 4 * words;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>((uintptr_t)(src + head) & ~(uintptr_t)3);
+    const uint32_t sh = 8 * ((uintptr_t)(src + head) & 3u);
+    for (uint64_t k = threadIdx.x; k < words; k += blockDim.x)
+        reinterpret_cast<uint32_t*>(dst + head)[k] = __funnelshift_r(w[k], sh ? w[k + 1] : 0u, sh);
+    if (threadIdx.x < head) dst[threadIdx.x] = src[threadIdx.x];
+    if (threadIdx.x < n - tail) dst[tail + threadIdx.x] = src[tail + threadIdx.x];
+}
+
 // One block per brick record: ID, P, palette, E, stream, nSymbols (fileIO.cpp:57-96).
 // Version 2 adds a u32 after the ID: the brick's table (bits 4..7) and mode (bits 0..3).
 // Block nb writes the header: version 1, 152 bytes (fileIO.cpp:25-49); version 2, 28 bytes
@@ -1215,20 +1222,15 @@ __global__ void serialize_kernel(const EncMeta* __restrict__ meta, uint32_t nb, 
     uint8_t* dst = image + rec_off[i];
     const uint8_t* pal = reinterpret_cast<const uint8_t*>(pal_pool + m.pal_off);
     const uint8_t* enc = enc_pool + m.enc_off;
-    const uint64_t pb = 8ull * m.P;
-    const uint64_t h = v2 ? 12 : 8;  // ID [, sel], P
-    const uint64_t total = h + 8 + pb + m.E;
-    for (uint64_t k = threadIdx.x; k < total; k += blockDim.x) {
-        uint8_t v;
-        if (k < 4) v = (uint8_t)(m.id >> (8 * k));
-        else if (k < h - 4) v = (uint8_t)((m.sel & 0xFFu) >> (8 * (k - 4)));
-        else if (k < h) v = (uint8_t)(m.P >> (8 * (k - (h - 4))));
-        else if (k < h + pb) v = pal[k - h];
-        else if (k < h + 4 + pb) v = (uint8_t)(m.E >> (8 * (k - h - pb)));
-        else if (k < h + 4 + pb + m.E) v = enc[k - h - 4 - pb];
-        else v = (uint8_t)(m.nsym >> (8 * (k - h - 4 - pb - m.E)));
-        dst[k] = v;
+    const uint32_t h = v2 ? 12 : 8;  // ID [, sel], P
+    if (threadIdx.x < h + 8) {
+        const uint32_t k = threadIdx.x;
+        const uint32_t word = k < 4 ? m.id : k < h - 4 ? m.sel & 0xFFu : k < h ? m.P : k < h + 4 ? m.E : m.nsym;
+        const uint64_t at = k < h ? k : k < h + 4 ? k + 8ull * m.P : k + 8ull * m.P + m.E;
+        dst[at] = (uint8_t)(word >> (8 * (k & 3u)));
     }
+    copy_bytes(dst + h, pal, 8ull * m.P);
+    copy_bytes(dst + h + 4 + 8ull * m.P, enc, m.E);
 }
 
 // ------------------------------------------------------------ host driver
@@ -1514,7 +1516,7 @@ static int finish_encode(EncoderState* s, const EncodeSelection* sel, cudaStream
         CK(cudaMemcpyAsync(s->d_model, models.data(), n_tables * kModelWords * sizeof(uint32_t),
                            cudaMemcpyHostToDevice, st));
     } else {  // one model from the sampled bricks' histogram (brickEncoding.hpp:481-482)
-        model_kernel<<<1, 1, 0, st>>>(s->d_misc + 2, s->d_model);
+        model_kernel<<<1, 32, 0, st>>>(s->d_misc + 2, s->d_model);
         CK(cudaGetLastError());
     }
     if (nb > s->h_meta_cap) {
