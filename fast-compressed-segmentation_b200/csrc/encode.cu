@@ -977,7 +977,7 @@ __device__ __forceinline__ void rans_enc_step(uint32_t& x, const uint4 t) {
 // more bricks than warp schedulers, so that no chain shares one; beyond, several chains
 // per warp, since a chain's step costs the scheduler as much for one lane as for many.
 // Measured against one lane per brick that did all of it (165 cycles per symbol): 512
-// bricks of 64^3, longest 84,720 symbols, 7.24 -> 1.45 ms (K = 1, 33 cycles per
+// bricks of 64^3, longest 84,720 symbols, 7.24 -> 1.28 ms (K = 1, 29 cycles per
 // symbol); 8192 bricks of 32^3 0.91 -> 0.30 ms (K = 8; 0.67 with K = 1); 60 bricks of
 // 32^3 0.60 -> 0.11 ms.  Batches of 128 against 64 with K = 1: 1.45 against 1.55 ms.
 template <uint32_t kRansBatch>
@@ -997,13 +997,21 @@ __global__ void __launch_bounds__(32 * (K + 1)) enc_rans_kernel(EncMeta* __restr
                                                                 uint64_t* __restrict__ rec_size, uint32_t rec_fixed,
                                                                 uint8_t* __restrict__ enc_pool,
                                                                 const uint32_t* __restrict__ model, uint32_t n_tables,
-                                                                Checkpoint* __restrict__ ck_all, uint32_t n_sm) {
+                                                                Checkpoint* __restrict__ ck_all) {
     constexpr uint32_t kRansRing = RansBrick<kRansBatch>::kRing;
     __shared__ RansBrick<kRansBatch> s_bricks[K];
     const uint32_t lane = threadIdx.x & 31, FULL = 0xFFFFFFFFu;
-    // the chain's warp: the first or the last one, in turn, so that the chains of an SM's blocks (of two
-    // warps each) do not meet on two of its four schedulers
-    const uint32_t chain_warp = (blockIdx.x / n_sm) & 1u ? K : 0u, warp = threadIdx.x >> 5;
+    // The chain's warp.  Warps take an SM's four schedulers in turn, by slot; of blocks of two warps, the first
+    // pair of blocks has its chains in their first warps and the next one in their second, so that four chains do
+    // not meet (512 bricks of 64^3 1.47 -> 1.28 ms against every other block).  Five and nine warps differ by one.
+    const uint32_t warp = threadIdx.x >> 5;
+    uint32_t chain_warp = 0;
+    if (K == 1) {
+        __shared__ uint32_t s_slot;
+        if (threadIdx.x == 0) asm volatile("mov.u32 %0, %%warpid;" : "=r"(s_slot));
+        __syncthreads();
+        chain_warp = s_slot >> 2 & 1u;
+    }
     if (warp == chain_warp) {
         auto& B = s_bricks[min(lane, (uint32_t)K - 1)];
         uint32_t x = kRansL;
@@ -1535,7 +1543,7 @@ static int finish_encode(EncoderState* s, const EncodeSelection* sel, cudaStream
         const uint32_t n_sm = (uint32_t)sm_count(s->device);
         auto rans = [&](auto kernel, uint32_t K) {
             kernel<<<(nb + K - 1) / K, 32 * (K + 1), 0, st>>>(s->d_meta, nb, s->d_nib, s->d_rec_off, v2 ? 20u : 16u,
-                                                             s->d_enc, s->d_model, s->n_tables, s->d_ck, n_sm);
+                                                             s->d_enc, s->d_model, s->n_tables, s->d_ck);
         };
         if (nb <= 4 * n_sm) rans(enc_rans_kernel<1, 128>, 1);
         else if (nb <= 16 * n_sm) rans(enc_rans_kernel<4, 64>, 4);
