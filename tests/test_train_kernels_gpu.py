@@ -56,3 +56,24 @@ def test_dense_layer_tiles(codec, M, N, K):
         assert torch.all((got.double() - want).abs() <= tol)
         assert torch.equal(Cb[off:off + M * N].view(M, N).cpu(), got.to(torch.bfloat16))
         assert torch.isnan(C[off + M * N:]).all()
+
+
+# a warp per brick: its block not full, one table to all sixteen, and ties between equal tables and equal modes
+@pytest.mark.parametrize("bricks", [1, 4, 9])
+@pytest.mark.parametrize("n_tables", [1, 3, 16])
+def test_exhaustive_choice(codec, oracle, bricks, n_tables):
+    import torch
+    rng = np.random.default_rng(bricks * 16 + n_tables)
+    hist = rng.integers(0, 1 << 18, (bricks, 12, 16)).astype(np.uint32)
+    hist[0, 5:] = hist[0, 5]
+    hist[-1, :, 3:] = 0
+    tables = np.full((n_tables, 16), 1, np.uint32)
+    for t in range(n_tables):
+        tables[t, rng.integers(0, 16)] += 4096 - 16
+    d = torch.from_numpy(hist.view(np.int32)).cuda()
+    sel = torch.zeros(bricks, dtype=torch.uint8, device="cuda")
+    cost = torch.zeros(bricks * 12 * n_tables, dtype=torch.int64, device="cuda")
+    codec.select_exhaustive(d, tables, sel, cost)
+    want, want_cost = oracle.select_exhaustive(hist, tables)
+    assert np.array_equal(sel.cpu().numpy(), want)
+    assert np.array_equal(cost.cpu().numpy().view(np.uint64), np.asarray(want_cost).reshape(-1))
