@@ -969,7 +969,7 @@ __device__ __forceinline__ void rans_enc_step(uint32_t& x, const uint4 t) {
 
 // A brick's symbols are one dependent chain, and the longest brick's is the kernel's
 // time, so one warp of a block does nothing else: lane k runs brick k's steps, in
-// batches of 64 or 128, on entries read ahead from shared memory, and leaves the states
+// batches of 64 or 256, on entries read ahead from shared memory, and leaves the states
 // there.  Each of the K bricks has a warp of its own that meanwhile turns the next
 // symbols into steps and works out from the last batch's states the bytes they put out,
 // their place (a ballot prefix) and the seek checkpoints among them; its global loads
@@ -977,9 +977,10 @@ __device__ __forceinline__ void rans_enc_step(uint32_t& x, const uint4 t) {
 // more bricks than warp schedulers, so that no chain shares one; beyond, several chains
 // per warp, since a chain's step costs the scheduler as much for one lane as for many.
 // Measured against one lane per brick that did all of it (165 cycles per symbol): 512
-// bricks of 64^3, longest 84,720 symbols, 7.24 -> 1.28 ms (K = 1, 29 cycles per
+// bricks of 64^3, longest 84,720 symbols, 7.24 -> 1.24 ms (K = 1, 28 cycles per
 // symbol); 8192 bricks of 32^3 0.91 -> 0.30 ms (K = 8; 0.67 with K = 1); 60 bricks of
-// 32^3 0.60 -> 0.11 ms.  Batches of 128 against 64 with K = 1: 1.45 against 1.55 ms.
+// 32^3 0.60 -> 0.11 ms.  Batches of 128 with K = 1: 1.28 ms, of 512: 1.22
+// ms, but 60 bricks of 32^3 take 0.113 ms for 0.105.
 template <uint32_t kRansBatch>
 struct RansBrick {
     static constexpr uint32_t kRing = 4 * kRansBatch;
@@ -1545,7 +1546,7 @@ static int finish_encode(EncoderState* s, const EncodeSelection* sel, cudaStream
             kernel<<<(nb + K - 1) / K, 32 * (K + 1), 0, st>>>(s->d_meta, nb, s->d_nib, s->d_rec_off, v2 ? 20u : 16u,
                                                              s->d_enc, s->d_model, s->n_tables, s->d_ck);
         };
-        if (nb <= 4 * n_sm) rans(enc_rans_kernel<1, 128>, 1);
+        if (nb <= 4 * n_sm) rans(enc_rans_kernel<1, 256>, 1);
         else if (nb <= 16 * n_sm) rans(enc_rans_kernel<4, 64>, 4);
         else rans(enc_rans_kernel<8, 64>, 8);
         CK(cudaGetLastError());
