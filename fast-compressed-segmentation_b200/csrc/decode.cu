@@ -1439,20 +1439,22 @@ __global__ void __launch_bounds__(dec_threads<V, KL>(), dec_ctas_per_sm<V, KL>()
     // and of the last level's output, and every one of them works out the levels between for
     // itself -- under a third of a brick's time, and nothing to exchange but the op records.
     // Below that the first CTA decodes it alone (LOD 4 and coarser took up to 20 us longer
-    // in teams).  With more requests, as without clusters,
+    // in teams) and the others leave at once (24 to 120 bricks of 64^3 at LOD 3 or 4 take
+    // the 20.6 and 24.7 us of single CTAs).  With more requests, as without clusters,
     // each CTA takes whole requests from the queue.
     const uint32_t cs = CLUSTERS ? cluster_size() : 1u, cr = CLUSTERS ? cluster_rank() : 0u;
     const bool joint = CLUSTERS && n_req <= gridDim.x / cs;
     uint32_t next = CLUSTERS ? blockIdx.x / cs : 0u;  // joint: the cluster's request
-    bool team = false;
-    if (joint) {
-        const uint32_t r = next < n_req ? (A.order ? A.order[next] : next) : 0xFFFFFFFFu;
-        team = r < A.n_reqs && A.reqs[r].lod >= kTeamLod;
-        if (cr && !team) return;
+    uint32_t lod = 0;
+    if (joint && next < n_req) {
+        const uint32_t r = A.order ? A.order[next] : next;
+        if (r < A.n_reqs) lod = A.reqs[r].lod;
     }
+    if (CLUSTERS && joint && cr && lod < kTeamLod) return;
+    load_lut<V>(S.lut, A.lut, tid, T);
+    const bool team = lod >= kTeamLod;
     const uint32_t jt = team ? cr * T + tid : tid, jT = team ? cs * T : T;  // of the threads of a request
 
-    load_lut<V>(S.lut, A.lut, tid, T);
     if (tid == 0) {
         mbar_init(&S.bar);
         S.rewait = 0;
@@ -1873,7 +1875,7 @@ static cudaError_t launch_variant(const DecodeArgs& A0, const DecodeScratch& scr
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         const uint64_t threads = (uint64_t)A.n * dec_threads<V, KL>(), sm = (uint64_t)std::max(sms, 1);
         if (A.n_dev) cs = 4;
-        else if (8 * threads <= 1024 * sm) cs = 8;
+        else if (8 * threads <= 1024 * sm && 8 * (uint64_t)A.n <= 2 * sm) cs = 8;
         else if (4 * threads <= 1400 * sm) cs = 4;
         else if (2 * (uint64_t)A.n <= grid) cs = 2;
         while (cs > 1 && (A.n_dev ? cs : cs * (uint64_t)A.n) > grid) cs /= 2;  // (little scratch)
@@ -1881,6 +1883,11 @@ static cudaError_t launch_variant(const DecodeArgs& A0, const DecodeScratch& scr
     if (A.n_dev) grid -= grid % cs;
     else grid = (uint32_t)std::min<uint64_t>(grid, (uint64_t)A.n * cs);
     if (grid == 0) return cudaErrorInvalidValue;
+    // a programmatic dependent follows a kernel, not this reset; with a cluster per request nothing is queued
+    if (!(cfg && cfg->pdl) && (cs == 1 || A.n_dev)) {
+        cudaError_t e = cudaMemsetAsync(scr.d_queue, 0, sizeof(uint32_t), st);
+        if (e != cudaSuccess) return e;
+    }
     A.stage_cap = (cfg && !cfg->stage) ? 0u : stage_cap<V, KL>();
     if (cs > 1 || (cfg && cfg->pdl)) {
         cudaLaunchConfig_t lc = {};
@@ -1916,10 +1923,6 @@ cudaError_t launch_decode(const DeviceDataset& ds, const csv_request* d_reqs, ui
     // the small variant when the dataset's bricks are 32^3 or smaller, when the caller
     // says every request is at LOD 5 or coarser, or when asked to take every request
     const bool small = ds.L <= kSmallLevels + 1 || (cfg && (cfg->small_only || cfg->layout == 1));
-    if (!(cfg && cfg->pdl)) {  // a programmatic dependent follows a kernel, not this reset
-        cudaError_t e = cudaMemsetAsync(scr.d_queue, 0, sizeof(uint32_t), st);
-        if (e != cudaSuccess) return e;
-    }
     DecodeArgs A;
     A.bricks = ds.d_bricks;
     A.pal = ds.d_pal;
