@@ -187,25 +187,29 @@ __device__ uint32_t sample_stats(FeatShared& S, const uint64_t* vol, uint64_t W,
 // has rows to read).  A CTA counts over its part of the rows of even y and even z (all x:
 // a quarter of the voxels, every pair within such a row, and each such voxel's +1 / +4
 // neighbours in y and z), a row per warp at a time with its four neighbour rows read
-// beside it, so that ten loads per lane are in flight; the first also takes the sample's
-// statistics.  Counts meet in the brick's feature row as whole numbers (zeroed by the
+// beside it, so that ten loads per lane are in flight.  The sample's statistics, a serial
+// walk, are a CTA of their own, and these come first.  Counts meet in the brick's feature row as whole numbers (zeroed by the
 // launch); the last CTA to add its own turns them into the features.
 // Row words: 0 .. 14 counts, 15 CTAs done | distinct << 16, 16 .. 31 op nibbles.
-// Measured (B200, 320 bricks of 64^3): 0.41 -> 0.165 ms (one CTA per brick with planes
+// Measured (B200, 320 bricks of 64^3): 0.41 -> 0.156 ms, 64 bricks 66 -> 47 us by the
+// samples apart (one CTA per brick with planes
 // kept in registers, the runs counted start by start and the sample's ops walked by one
 // thread); the rows it reads are three quarters of the volume, 0.08 ms at the HBM rate.
 __global__ void __launch_bounds__(kFThreads, 4) features_kernel(const uint64_t* __restrict__ vol, uint64_t W, uint64_t H,
                                                                 uint64_t D, uint32_t b, uint32_t nbx, uint32_t nby,
                                                                 uint32_t nbz, uint32_t parts, float* __restrict__ feat) {
     __shared__ FeatShared S;
-    const uint32_t i = blockIdx.x / parts, part = blockIdx.x % parts;
+    const uint32_t nb = nbx * nby * nbz, shares = parts > 1 ? parts - 1 : 1;
+    const bool sample = parts == 1 || blockIdx.x < nb, rows = parts == 1 || !sample;
+    const uint32_t j = parts == 1 || sample ? blockIdx.x : blockIdx.x - nb;
+    const uint32_t i = parts == 1 || sample ? j : j / shares, part = parts == 1 || sample ? 0 : j % shares;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t bz = i % nbz, by = (i / nbz) % nby, bx = i / (nbz * nby);  // split order (brick.hpp:152-154)
     const uint64_t x0 = (uint64_t)bx * b, y0 = (uint64_t)by * b, z0 = (uint64_t)bz * b;
     uint32_t* row_out = reinterpret_cast<uint32_t*>(feat + (size_t)i * kFeat);
     if (tid < 16) S.cnt[tid] = 0;
     uint32_t nibbles = 0;
-    if (part == 0) nibbles = sample_stats(S, vol, W, H, D, x0, y0, z0, b);
+    if (sample) nibbles = sample_stats(S, vol, W, H, D, x0, y0, z0, b);
     __syncthreads();
     uint32_t c[15] = {};
     // a row's runs follow from the mask of their starts: lane l keeps the mask of the warp's row l, and
@@ -232,11 +236,11 @@ __global__ void __launch_bounds__(kFThreads, 4) features_kernel(const uint64_t* 
         }
         rows_kept = 0;
     };
-    {
+    if (rows) {
         const uint32_t nch = (b + 31) / 32;  // values per lane: 1 or 2 (lane l holds x = l and x = l + 32)
         const bool interior = x0 + b <= W && y0 + b <= H && z0 + b <= D;
         const uint64_t WH = W * H;
-        const uint32_t hb = b / 2, items = hb * hb, per = (items + parts - 1) / parts;
+        const uint32_t hb = b / 2, items = hb * hb, per = (items + shares - 1) / shares;
         const uint32_t it1 = min(items, (part + 1) * per);
         for (uint32_t it = part * per + warp; it < it1; it += kFThreads / 32) {
             const uint32_t y = 2 * (it % hb), z = 2 * (it / hb);
@@ -298,12 +302,12 @@ __global__ void __launch_bounds__(kFThreads, 4) features_kernel(const uint64_t* 
     }
     __syncthreads();
     if (warp == 0) {
-        if (part == 0 && lane < 16) atomicExch(row_out + 16 + lane, nibbles);
+        if (sample && lane < 16) atomicExch(row_out + 16 + lane, nibbles);
         if (lane < 15 && S.cnt[lane]) atomicAdd(row_out + lane, S.cnt[lane]);
         __threadfence();
         __syncwarp();
         uint32_t done = 0;
-        if (lane == 0) done = atomicAdd(row_out + 15, 1u + (part == 0 ? S.distinct << 16 : 0u));
+        if (lane == 0) done = atomicAdd(row_out + 15, 1u + (sample ? S.distinct << 16 : 0u));
         done = __shfl_sync(0xffffffffu, done, 0);
         if ((done & 0xFFFFu) + 1 != parts) return;
         __threadfence();
