@@ -16,11 +16,10 @@
 // stage's mbarrier.  The network's own operands lie in global memory in that layout, chunk
 // after chunk (tiled_at), so that the same thread fills a stage with one bulk copy per
 // operand and nothing else of the block takes part; row-major operands (csv_gemm_bf16) are
-// copied by all threads with cp.async, a block barrier per chunk.  (A product
-// over 2048 rows: 30 us row-major, 20 us tiled.)  The epilogue reads the accumulator
-// with tcgen05.ld (warp w owns lanes 32w..32w+31 = rows) and applies the fused ops.  An
-// output's products are added in the order of K whatever the tile, so results do not
-// depend on it.
+// copied by all threads with cp.async, a block barrier per chunk.  (A product over 2048
+// rows: 30 us row-major, 20 us tiled.)  The epilogue reads the accumulator with tcgen05.ld
+// (warp w owns lanes 32w..32w+31 = rows) and applies the fused ops.  An output's products
+// are added in the order of K whatever the tile, so results do not depend on it.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -191,10 +191,10 @@ __device__ uint32_t sample_stats(FeatShared& S, const uint64_t* vol, uint64_t W,
 // walk, are a CTA of their own, and these come first.  Counts meet in the brick's feature row as whole numbers (zeroed by the
 // launch); the last CTA to add its own turns them into the features.
 // Row words: 0 .. 14 counts, 15 CTAs done | distinct << 16, 16 .. 31 op nibbles.
-// Measured (B200, 320 bricks of 64^3): 0.41 -> 0.156 ms, 64 bricks 66 -> 47 us by the
-// samples apart (one CTA per brick with planes
+// Measured (B200, 320 bricks of 64^3): 0.41 -> 0.156 ms (one CTA per brick with planes
 // kept in registers, the runs counted start by start and the sample's ops walked by one
-// thread); the rows it reads are three quarters of the volume, 0.08 ms at the HBM rate.
+// thread; 0.170 ms, and 66 for 47 us with 64 bricks, with the sample in a CTA that has rows
+// too); the rows it reads are three quarters of the volume, 0.08 ms at the HBM rate.
 __global__ void __launch_bounds__(kFThreads, 4) features_kernel(const uint64_t* __restrict__ vol, uint64_t W, uint64_t H,
                                                                 uint64_t D, uint32_t b, uint32_t nbx, uint32_t nby,
                                                                 uint32_t nbz, uint32_t parts, float* __restrict__ feat) {
