@@ -217,7 +217,7 @@ struct GemmArgs {
     const __nv_bfloat16* A = nullptr;  // [M][K]
     const __nv_bfloat16* B = nullptr;  // [N][K]
     uint32_t M = 0, N = 0, K = 0;      // M % 128 == 0, N % 16 == 0, K % 64 == 0
-    uint32_t tile_n = 64;              // columns per CTA, a multiple of 16 up to 64
+    uint32_t tile_n = 64;              // columns per CTA, a multiple of 16 up to 64 (256 when not tiled)
     bool tiled = false;                // A, B, mask, Cb and CbT are tiled (tiled_at), not row-major
     const float* bias = nullptr;          // [N] or null
     const __nv_bfloat16* mask = nullptr;  // [M][N] or null: multiply by (mask > 0), the ReLU gradient

@@ -6,7 +6,7 @@
 // in tensor memory, and an epilogue that adds a bias, applies ReLU or the ReLU
 // gradient mask, and writes fp32 and/or bf16, plain or transposed.
 //
-// Per CTA: one 128 x N tile (N <= 64, a multiple of 16), 128 threads.  The selector's
+// Per CTA: one 128 x N tile (N <= 64, or 256 in place, a multiple of 16), 128 threads.  The selector's
 // layers are small (2048 x 256 x 256 at the training batch), so tiles are narrow, to
 // spread over the SMs.  K runs in chunks of 64 through four stages of shared memory in the
 // canonical no-swizzle K-major layout (8-row x 16-byte core matrices; core matrix (row
@@ -33,7 +33,8 @@ namespace {
 
 constexpr uint32_t kGemmThreads = 128;
 constexpr uint32_t kKChunk = 64;               // bf16 elements per row per chunk (128 bytes)
-constexpr uint32_t kTileN = 64;                // columns per CTA at most
+constexpr uint32_t kTileN = 64;                // columns staged at a time
+constexpr uint32_t kTileInPlace = 256;         // columns per CTA at most, of row-major operands under an output
 constexpr uint32_t kStages = 4;
 constexpr uint32_t kTileA = 128 * kKChunk * 2; // 16 KB
 constexpr uint32_t kTileB = kTileN * kKChunk * 2;  // 8 KB
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
     const uint32_t mt = G.M / 128u;
     const uint32_t m0 = (blk % mt) * 128u, n0 = (blk / mt) * G.tile_n;
     const uint32_t N = min(G.tile_n, G.N - n0);
-    const uint32_t ncols = N <= 32 ? 32u : 64u;
+    const uint32_t ncols = N <= 32 ? 32u : (N <= 64 ? 64u : (N <= 128 ? 128u : 256u));
     const uint32_t sA = smem_u32(smem), sB = sA + kStages * kTileA;
     if (tid == 0) {
         for (uint32_t s = 0; s < kStages; ++s) {
@@ -189,15 +190,16 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base;
-    // M = 128, N, bf16 x bf16 -> f32, both operands K-major
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
     const uint32_t chunks = G.K / kKChunk;
     auto done = [&](uint32_t c) { return mbar_wait(smem_u32(&bars[c % kStages]), (c / kStages) & 1u); };
-    auto multiply = [&](uint32_t c) {
+    // stage c's products into columns [col, col + n) (first: they start a sum)
+    auto multiply = [&](uint32_t c, uint32_t col, uint32_t n, bool first) {
+        // M = 128, N = n, bf16 x bf16 -> f32, both operands K-major
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 #pragma unroll
         for (uint32_t s = 0; s < kKChunk / 16; ++s)
-            mma_bf16(tmem, smem_desc(sA + (c % kStages) * kTileA + s * 256u),
-                     smem_desc(sB + (c % kStages) * kTileB + s * 256u), idesc, (c > 0 || s > 0) ? 1u : 0u);
+            mma_bf16(tmem + col, smem_desc(sA + (c % kStages) * kTileA + s * 256u),
+                     smem_desc(sB + (c % kStages) * kTileB + s * 256u), idesc, (!first || s > 0) ? 1u : 0u);
         mma_commit(smem_u32(&bars[c % kStages]));
     };
     bool ok = true;
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
                 ok = landed(c);
                 waited = c + 1;
                 if (!ok) break;
-                multiply(c);
+                multiply(c, 0, N, c == 0);
                 // the stage before this one is filled again once its products are done
                 if (c > 0 && issued < chunks) {
                     ok = done(c - 1);
@@ -230,27 +232,31 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
         __syncthreads();
         ok = s_ok != 0;
     } else {
-        auto load = [&](uint32_t c) {  // chunk c into its stage; a group of copies either way
-            if (c < chunks) {
-                load_operand(sA + (c % kStages) * kTileA, G.A, G.K, m0, 128u, c * kKChunk);
-                load_operand(sB + (c % kStages) * kTileB, G.B, G.K, n0, N, c * kKChunk);
+        // 64 columns at a time, all of K each; step c is chunk c % chunks of columns 64 (c / chunks) on
+        const uint32_t steps = (N + kTileN - 1) / kTileN * chunks;
+        auto load = [&](uint32_t c) {  // step c's operands into its stage; a group of copies either way
+            if (c < steps) {
+                const uint32_t col = c / chunks * kTileN, k0 = c % chunks * kKChunk;
+                load_operand(sA + (c % kStages) * kTileA, G.A, G.K, m0, 128u, k0);
+                load_operand(sB + (c % kStages) * kTileB, G.B, G.K, n0 + col, min(N - col, kTileN), k0);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
         for (uint32_t c = 0; c + 1 < kStages; ++c) load(c);
-        for (uint32_t c = 0; c < chunks; ++c) {
+        for (uint32_t c = 0; c < steps; ++c) {
             asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             if (!(ok = __syncthreads_and(ok))) break;  // one decision for the whole block
             if (tid == 0) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                multiply(c);
+                const uint32_t col = c / chunks * kTileN;
+                multiply(c, col, min(N - col, kTileN), c % chunks == 0);
             }
             if (c > 0) ok = done(c - 1);
             if (ok) load(c + kStages - 1);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        ok = __syncthreads_and(ok && done(chunks - 1)) != 0;
+        ok = __syncthreads_and(ok && done(steps - 1)) != 0;
     }
     if (!ok && tid == 0 && G.err) atomicExch(G.err, 1u);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -652,7 +658,8 @@ static uint32_t gemm_blocks(const GemmArgs& g) { return g.M / 128 * ((g.N + g.ti
 cudaError_t launch_gemm_bf16(const GemmArgs& g, cudaStream_t st, const GemmArgs* second) {
     if (g.M == 0 || g.N == 0 || g.K == 0) return cudaSuccess;
     for (const GemmArgs* p : {&g, second})
-        if (p && (p->M % 128 || p->N % 16 || p->K % kKChunk || p->tile_n == 0 || p->tile_n % 16 || p->tile_n > kTileN))
+        if (p && (p->M % 128 || p->N % 16 || p->K % kKChunk || p->tile_n == 0 || p->tile_n % 16 ||
+                  p->tile_n > (p->tiled ? kTileN : kTileInPlace)))
             return cudaErrorInvalidValue;
     if (second && second->tiled != g.tiled) return cudaErrorInvalidValue;
     constexpr int smem = (int)((kTileA + kTileB) * kStages);
@@ -694,6 +701,19 @@ extern "C" int csv_gemm_bf16(csv_ctx* ctx, const void* d_A, const void* d_B, uin
     G.CbT = (__nv_bfloat16*)d_CbT;
     G.CT = d_CT;
     G.err = d_err;
+    // An output over an operand (a layer in place): its rows are written by the CTA that has read them,
+    // so one CTA takes the row of tiles, 256 columns, as long as that is all of them.
+    auto over = [](const void* out, size_t out_bytes, const void* in, size_t in_bytes) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(out), b = reinterpret_cast<uintptr_t>(in);
+        return out && a < b + in_bytes && b < a + out_bytes;
+    };
+    auto over_operand = [&](const void* out, size_t out_bytes) {
+        return over(out, out_bytes, d_A, 2 * (size_t)M * K) || over(out, out_bytes, d_B, 2 * (size_t)N * K);
+    };
+    const size_t mn = (size_t)M * N;
+    if (over_operand(d_C, 4 * mn) || over_operand(d_CT, 4 * mn) || over_operand(d_Cb, 2 * mn) ||
+        over_operand(d_CbT, 2 * mn))
+        G.tile_n = kTileInPlace;
     cudaError_t e = launch_gemm_bf16(G, (cudaStream_t)stream);
     if (e != cudaSuccess) return abi_cuda_fail(ctx, e, "gemm");
     return CSV_OK;

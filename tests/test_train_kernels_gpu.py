@@ -58,6 +58,28 @@ def test_dense_layer_tiles(codec, M, N, K):
         assert torch.isnan(C[off + M * N:]).all()
 
 
+# a layer in place: the output over the rows it was computed from (all columns are one CTA's), more rows of CTAs than
+# run at once, and over the other operand where one CTA reads all of it
+@pytest.mark.parametrize("M,N,over", [(128, 64, "A"), (256, 256, "A"), (128 * 700, 256, "A"), (128 * 300, 192, "A"),
+                                      (128, 256, "B")])
+def test_dense_layer_in_place(codec, M, N, over):
+    import torch
+    K = N if over == "A" else 128
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + N)
+    A = torch.randn((M, K), device="cuda", generator=g).to(torch.bfloat16)
+    B = torch.randn((N, K), device="cuda", generator=g).to(torch.bfloat16)
+    want = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    codec.gemm_bf16(A, B, relu=True, Cb=want)
+    # the sums' order does not depend on the tile: bit for bit the output beside the operands
+    if over == "A":
+        codec.gemm_bf16(A, B, relu=True, Cb=A)
+        assert torch.equal(A, want)
+    else:
+        codec.gemm_bf16(A, B, relu=True, CbT=B.view(-1))
+        assert torch.equal(B.view(-1).view(N, M), want.T)
+
+
 # a warp per brick: its block not full, one table to all sixteen, and ties between equal tables and equal modes
 @pytest.mark.parametrize("bricks", [1, 4, 9])
 @pytest.mark.parametrize("n_tables", [1, 3, 16])
