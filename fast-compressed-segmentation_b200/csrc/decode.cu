@@ -435,6 +435,9 @@ struct ChainRing {
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 4;" ::: "memory");
     }
+    // The last copies, of symbols past the chain's end (a brick that names fewer than its stream holds): none may
+    // land in a ring that the block has left.
+    __device__ __forceinline__ void drain() { asm volatile("cp.async.wait_all;" ::: "memory"); }
     __device__ __forceinline__ void window() {
         const uint32_t r = 8 * (pos & 3u), a = pos & ~3u, w1 = ring_word(a - 4);
         hi = __funnelshift_r(w1, ring_word(a), r);
@@ -700,6 +703,7 @@ __global__ void __launch_bounds__(kIndexThreads) index_symbols_kernel(
             ChainRing c;
             c.init(enc, x, pos, idx_smem + kIndexTables + ((threadIdx.x >> 5) * lanes + lane) * kRingPitch);
             more = index_walk_ring(c, br.nsym, w, sn);
+            c.drain();
         } else {
             more = index_run(enc, x, pos, g_lutf, g_lutf, g_lut, model, fast, 0, br.nsym, w, sn);
         }

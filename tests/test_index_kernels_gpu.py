@@ -58,3 +58,24 @@ def test_chain_of_every_length(codec, oracle, freq, nb, brick, longest):
     assert np.array_equal(sa, sb) and np.array_equal(a[sa == 0], b[sa == 0])
     ds.close()
     ds2.close()
+
+
+# chains that end while their ring is being filled (fewer symbols named than the stream holds; four pieces in every four
+# groups of 32 symbols), many blocks one after the other on an SM
+@pytest.mark.parametrize("nb,longest", [(40, 6000), (4000, 1600)])
+def test_chains_that_end_with_copies_on_their_way(codec, oracle, nb, longest):
+    freq, cum = (256,) * 16, 256 * np.arange(16, dtype=np.uint32)
+    rng = np.random.default_rng(nb)
+    ns = rng.integers(600, longest, nb)
+    # no stop bit in the root (its symbol is even), a state of an encoder's range
+    streams = [rng.integers(0, 256, longest, dtype=np.uint8).tobytes() +
+               struct.pack("<I", (1 << 30) | int(rng.integers(0, 8)) << 9) for _ in range(nb)]
+    ds = codec.open(image(freq, 16, streams, ns))
+    rows, states = parse_sidecar(ds.index_sidecar())
+    assert np.array_equal(rows[:, 2], -(-ns // SEED))
+    at = 0
+    for i in range(nb):
+        want = oracle.rans_states(np.asarray(freq, np.uint32), cum, streams[i], int(ns[i]), SEED)
+        assert want[-1, 1] > 512 and np.array_equal(states[at:at + rows[i, 2]], want), i
+        at += rows[i, 2]
+    ds.close()
