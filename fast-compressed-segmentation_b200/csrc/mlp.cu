@@ -25,6 +25,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "csv_internal.h"
 
@@ -619,20 +620,28 @@ __global__ void __launch_bounds__(kInferThreads, 1) mlp_infer_kernel(InferArgs G
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
-}  // namespace
+// A kernel's dynamic shared memory beyond 48 KB holds for the device that it was allowed on: once
+// for each, noted in the kernel's `allowed`.
+using AllowedOn = std::atomic<bool>[64];
+template <class Kernel>
+cudaError_t allow_smem(Kernel kernel, int bytes, AllowedOn& allowed) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess || (device < 64 && allowed[device])) return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && device < 64) allowed[device] = true;
+    return e;
+}
 
+}  // namespace
 
 cudaError_t launch_mlp_infer(const float* feat, uint32_t count, const __nv_bfloat16* W1t, const __nv_bfloat16* W2t,
                              const __nv_bfloat16* W3t, const float* b1, const float* b2, const float* b3, float* logits,
                              uint8_t* sel, uint32_t* err, int device, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e =
-            cudaFuncSetAttribute(mlp_infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static AllowedOn allowed;
+    const cudaError_t e = allow_smem(mlp_infer_kernel, (int)kInferSmem, allowed);
+    if (e != cudaSuccess) return e;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     InferArgs G;
@@ -664,12 +673,9 @@ cudaError_t launch_gemm_bf16(const GemmArgs& g, cudaStream_t st, const GemmArgs*
     if (second && second->tiled != g.tiled) return cudaErrorInvalidValue;
     constexpr int smem = (int)((kTileA + kTileB) * kStages);
     const auto kernel = g.tiled ? gemm_bf16_kernel<true> : gemm_bf16_kernel<false>;
-    static bool attr[2] = {false, false};
-    if (!attr[g.tiled]) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        attr[g.tiled] = true;
-    }
+    static AllowedOn allowed[2];
+    const cudaError_t e = allow_smem(kernel, smem, allowed[g.tiled]);
+    if (e != cudaSuccess) return e;
     const uint32_t n = gemm_blocks(g);
     kernel<<<n + (second ? gemm_blocks(*second) : 0u), kGemmThreads, smem, st>>>(g, second ? *second : g, n);
     return cudaGetLastError();
