@@ -1568,7 +1568,11 @@ static int finish_encode(EncoderState* s, const EncodeSelection* sel, cudaStream
         CK(cudaStreamSynchronize(st));
         if (s->h_words->misc[kMiscImage] <= s->image_cap) break;
         const uint64_t len = s->h_words->misc[kMiscImage];
-        CK(grow(&s->d_image, &s->image_cap, len + len / 8));  // (the next one may be a little longer)
+        // (the next one may be a little longer; where memory is short, no more than this one takes)
+        if (grow(&s->d_image, &s->image_cap, len + len / 8) != cudaSuccess) {
+            cudaGetLastError();
+            CK(grow(&s->d_image, &s->image_cap, len));
+        }
     }
     if (!v2) memcpy(models.data(), s->h_words->model, sizeof s->h_words->model);
     const uint32_t* model = models.data();

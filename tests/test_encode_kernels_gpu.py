@@ -109,3 +109,33 @@ def test_record_places(codec, oracle, shapes, v2):
             want = oracle.encode(vol, b)
         assert bytes(fresh.encoded_image_tensor().cpu().numpy()) == want
     fresh.close()
+
+
+def test_image_that_just_fits(codec):
+    """An encode whose image fits the memory that is left, but not an eighth more, succeeds."""
+    import torch
+    from csvb200 import Codec
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    vol = torch.randint(1, 2 ** 62, (192, 256, 256), device="cuda", generator=g)  # all labels distinct: a large image
+
+    def free():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    before = free()
+    roomy = Codec(0)
+    n = roomy.encode_device(vol, 32)
+    used = before - free()
+    want = roomy.encoded_image_tensor().clone()
+    roomy.close()
+    assert n > 64 << 20  # (a sixteenth is more than an allocation's granularity)
+    hog = torch.empty(free() - used + n // 16, dtype=torch.uint8, device="cuda")
+    tight = Codec(0)
+    for _ in range(2):
+        assert tight.encode_device(vol, 32) == n
+    del hog
+    torch.cuda.empty_cache()
+    assert torch.equal(tight.encoded_image_tensor(), want)
+    tight.close()
