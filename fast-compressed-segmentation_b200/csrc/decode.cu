@@ -659,24 +659,31 @@ __device__ __forceinline__ void index_finish(BrickDesc* bricks, uint32_t bi, con
 }
 
 // One lane per brick, `lanes` bricks of similar length to a warp (`order`: longest first), so
-// that a warp's chains end together.  Bound by the longest brick's dependent chain; model 0's
-// bricks take ChainRing, the others index_run's forms.
+// that a warp's chains end together.  Bound by the longest brick's dependent chain.  RING: model
+// 0's bricks take ChainRing, the others index_run's forms on tables in global memory; without,
+// model 0's take ChainFast on a table of a quarter of the shared memory.
 // Measured (B200; every brick in ChainFast's form, four to a warp): 256 bricks of 64^3,
 // longest 78,694 symbols, 4.26 -> 3.03 ms (106 -> 76 cycles a symbol); 2048 bricks of 64^3
-// 5.23 -> 4.51 ms, of 32^3 0.71 -> 0.63 ms; 32,768 bricks of 16^3 0.28 -> 0.17 ms.
+// 5.23 -> 4.35 ms, of 32^3 0.71 -> 0.60 ms; 32,768 bricks of 16^3 0.28 -> 0.17 ms.
 constexpr uint32_t kIndexThreads = 128;
 constexpr uint32_t kIndexTables = 2 * kTot * 8;
+template <bool RING>
 __global__ void __launch_bounds__(kIndexThreads) index_symbols_kernel(
     BrickDesc* __restrict__ bricks, uint32_t nb, const uint8_t* __restrict__ enc_pool, const uint32_t* __restrict__ g_lut,
     const uint32_t* __restrict__ g_lutf, uint32_t n_models, uint32_t fast_models, uint32_t lanes,
     const uint32_t* __restrict__ order, const uint64_t* __restrict__ nib_off, const uint64_t* __restrict__ snap_off,
     uint32_t* __restrict__ nib, uint2* __restrict__ snap, uint8_t* __restrict__ chain, uint32_t L, bool write_desc) {
-    uint2* t = reinterpret_cast<uint2*>(idx_smem);  // model 0's entries
-    for (uint32_t i = threadIdx.x; i < kTot; i += kIndexThreads) {
-        const uint32_t g = g_lut[i];
-        const uint2 v = make_uint2(((g >> 4) & 0x1FFFu) * 16, ((i - (g >> 17)) & (kTot - 1)) * 16 | (g & 15u));
-        t[2 * i] = v;
-        t[2 * ((i & 255u) << 4 | i >> 8) + 1] = v;
+    uint32_t* lut0f = reinterpret_cast<uint32_t*>(idx_smem);  // model 0's entries
+    if (RING) {
+        uint2* t = reinterpret_cast<uint2*>(idx_smem);
+        for (uint32_t i = threadIdx.x; i < kTot; i += kIndexThreads) {
+            const uint32_t g = g_lut[i];
+            const uint2 v = make_uint2(((g >> 4) & 0x1FFFu) * 16, ((i - (g >> 17)) & (kTot - 1)) * 16 | (g & 15u));
+            t[2 * i] = v;
+            t[2 * ((i & 255u) << 4 | i >> 8) + 1] = v;
+        }
+    } else {
+        load_fast_lut(lut0f, g_lut);
     }
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
@@ -699,13 +706,13 @@ __global__ void __launch_bounds__(kIndexThreads) index_symbols_kernel(
                      ((uint32_t)enc[br.E - 3] << 8) | enc[br.E - 4];
         const bool fast = x >= kRansL && model < 32 && ((fast_models >> model) & 1u);
         bool more;
-        if (fast && model == 0) {
+        if (RING && fast && model == 0) {
             ChainRing c;
             c.init(enc, x, pos, idx_smem + kIndexTables + ((threadIdx.x >> 5) * lanes + lane) * kRingPitch);
             more = index_walk_ring(c, br.nsym, w, sn);
             c.drain();
         } else {
-            more = index_run(enc, x, pos, g_lutf, g_lutf, g_lut, model, fast, 0, br.nsym, w, sn);
+            more = index_run(enc, x, pos, lut0f, g_lutf, g_lut, model, fast, 0, br.nsym, w, sn);
         }
         if (more)
             go = L >= 2;
@@ -1040,26 +1047,39 @@ void index_free(IndexTemps& t, cudaStream_t st) {
 
 // Pass 1 from the stream headers.  Lanes of a warp wait for each other's words done again
 // and for table bank conflicts, warps of an SM share its schedulers, and every block lays
-// out the tables, so bricks spread over warps until there are six per SM, then over lanes
-// (up to 16).  (ms by bricks per warp -- 1, 2, 4, 8, 16, 32: 256 bricks of 64^3 3.03, 3.17,
+// out the tables, so bricks spread over warps until there are six per SM, then over lanes.
+// (ms of this kernel by bricks per warp -- 1, 2, 4, 8, 16, 32: 256 bricks of 64^3 3.03, 3.17,
 // 3.50, 3.99, 4.73, 6.07; 2048 of 64^3 5.56, 4.35, 4.33, 5.03, 6.12, 8.03; 2048 of 32^3
 // 0.64, 0.60, 0.63, 0.72, 0.85, 1.10; 16,384 of 32^3 4.37, 2.39, 1.44, 0.99, 1.06, 1.28;
-// 32,768 of 16^3 1.14, 0.62, 0.35, 0.24, 0.17, 0.19.)
+// 32,768 of 16^3 1.14, 0.62, 0.35, 0.24, 0.17, 0.19.  Of all the index passes, 1, 2, 4, 8, 16:
+// 1024 bricks of 64^3 4.32, 4.09, 4.44; 3072 of 32^3 1.11, 0.89, 0.88; 6144 of 32^3 -, -, 1.31,
+// 1.28, 1.34; 24,576 of 32^3 -, -, 4.37, 3.81, 3.35.)
+// Images of several tables: the bricks of all but model 0 look their symbols up in global memory, through
+// the L1 cache, which the rings' and tables' shared memory leaves small, and the more tables and chains
+// there are the less of them it holds.  With more than 200 tables x bricks for every six warps of an SM
+// they take the form without rings, four bricks to a warp; not with two tables, where half the bricks
+// are model 0's.  (ms of all index passes with rings and without: 16 tables, 8192 bricks of 32^3 3.67,
+// 3.96, 16,384 5.37, 5.18, 65,536 of 16^3 5.50, 5.21, 131,072 11.4, 10.5; 8 tables, 16,384 of 32^3
+// 4.55, 5.25, 131,072 of 16^3 11.2, 10.6; 4 tables, 32,768 of 16^3 2.63, 2.77, 131,072 11.2, 10.8;
+// 2 tables, 65,536 of 16^3 4.92, 5.45, 131,072 10.4, 10.8.)
 cudaError_t index_pass1_serial(const DeviceDataset& ds, const IndexTemps& t, cudaStream_t st, bool write_desc) {
-    cudaError_t e = cudaFuncSetAttribute(index_symbols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kIndexTables + kIndexThreads * kRingPitch));
-    if (e != cudaSuccess) return e;
-    const uint32_t nb = ds.nb, warps = kIndexThreads / 32;
     int sms = 0;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ds.device);
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ds.device);
     if (e != cudaSuccess) return e;
-    const uint32_t in_flight = 6 * (uint32_t)std::max(1, sms), lanes = std::min(16u, (nb + in_flight - 1) / in_flight);
-    const uint32_t nm = ds.n_models ? ds.n_models : 1u;
-    index_symbols_kernel<<<(nb + warps * lanes - 1) / (warps * lanes), kIndexThreads,
-                           kIndexTables + warps * lanes * kRingPitch, st>>>(
-        ds.d_bricks, nb, ds.d_enc, ds.d_lut, t.lutf, nm, ds.fast_models, lanes, t.order, t.off, t.off + nb, t.nib,
-        t.snap, t.chain, ds.L, write_desc);
-    return cudaGetLastError();
+    const uint32_t nb = ds.nb, warps = kIndexThreads / 32, nm = ds.n_models ? ds.n_models : 1u;
+    const uint64_t six = 6 * (uint64_t)std::max(1, sms);
+    auto launch = [&](auto kernel, uint32_t lanes, uint32_t smem) {
+        kernel<<<(nb + warps * lanes - 1) / (warps * lanes), kIndexThreads, smem, st>>>(
+            ds.d_bricks, nb, ds.d_enc, ds.d_lut, t.lutf, nm, ds.fast_models, lanes, t.order, t.off, t.off + nb, t.nib,
+            t.snap, t.chain, ds.L, write_desc);
+        return cudaGetLastError();
+    };
+    if (nm > 2 && (uint64_t)nm * nb > 200 * six) return launch(index_symbols_kernel<false>, 4, 4 * kTot);
+    const uint32_t lanes = nb <= six ? 1u : (nb <= 3 * six ? 2u : (nb <= 6 * six ? 4u : (nb <= 24 * six ? 8u : 16u)));
+    e = cudaFuncSetAttribute(index_symbols_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(kIndexTables + kIndexThreads * kRingPitch));
+    if (e != cudaSuccess) return e;
+    return launch(index_symbols_kernel<true>, lanes, kIndexTables + warps * lanes * kRingPitch);
 }
 }  // namespace
 

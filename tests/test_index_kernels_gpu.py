@@ -79,3 +79,40 @@ def test_chains_that_end_with_copies_on_their_way(codec, oracle, nb, longest):
         assert want[-1, 1] > 512 and np.array_equal(states[at:at + rows[i, 2]], want), i
         at += rows[i, 2]
     ds.close()
+
+
+# images of several tables: few chains of all of them, and so many that the bricks of model 0 too take the form without
+# a ring; the states against the oracle's, the labels against the volume
+@pytest.mark.parametrize("side,n_tables", [(40, 16), (120, 3), (184, 16)])
+def test_chains_of_several_tables(codec, oracle, side, n_tables):
+    import torch
+    rng = np.random.default_rng(side)
+    vol = rng.integers(1, 9, (side // 2,) * 3).repeat(2, 0).repeat(2, 1).repeat(2, 2)
+    vol[rng.random(vol.shape) < 0.02] = 77
+    d = torch.from_numpy(vol).cuda()
+    tables = np.full((n_tables, 16), 16, np.uint32)
+    tables[np.arange(n_tables), np.arange(n_tables)] += 4096 - 256
+    nb = (side // 8) ** 3
+    sel = rng.integers(0, n_tables, nb).astype(np.uint8) << 4
+    codec.encode_device_sel(d, 8, tables, torch.from_numpy(sel).cuda())
+    img = bytes(codec.encoded_image_tensor().cpu().numpy())
+    ds = codec.open(img)
+    rows, states = parse_sidecar(ds.index_sidecar())
+    at, p = 0, 28 + 128 * n_tables
+    for i in range(nb):
+        _, s, P = struct.unpack_from("<3I", img, p)
+        E, = struct.unpack_from("<I", img, p + 12 + 8 * P)
+        stream, ns = img[p + 16 + 8 * P:p + 16 + 8 * P + E], struct.unpack_from("<I", img, p + 16 + 8 * P + E)[0]
+        p += 20 + 8 * P + E
+        f = tables[s >> 4]
+        cum = (np.cumsum(f) - f).astype(np.uint32)
+        if rows[i, 2]:
+            want = oracle.rans_states(f, cum, stream, ns, SEED)
+            assert np.array_equal(states[at:at + rows[i, 2]], want), i
+        at += rows[i, 2]
+    assert p == len(img)
+    got, st = decode_all(codec, ds, 3)
+    assert not st.any()
+    ref, _ = oracle.decode_image(oracle.encode(vol.view(np.uint64), 8), 3)
+    assert np.array_equal(np.asarray(got).reshape(-1).view(np.uint64), ref.reshape(-1).view(np.uint64))
+    ds.close()
