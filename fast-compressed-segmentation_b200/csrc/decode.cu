@@ -1904,8 +1904,7 @@ static cudaError_t launch_variant(const DecodeArgs& A0, const DecodeScratch& scr
         else if (2 * (uint64_t)A.n <= grid) cs = 2;
         while (cs > 1 && (A.n_dev ? cs : cs * (uint64_t)A.n) > grid) cs /= 2;  // (little scratch)
     }
-    if (A.n_dev) grid -= grid % cs;
-    else grid = (uint32_t)std::min<uint64_t>(grid, (uint64_t)A.n * cs);
+    grid = (uint32_t)std::min<uint64_t>(grid - grid % cs, (uint64_t)A.n * cs);
     if (grid == 0) return cudaErrorInvalidValue;
     // a programmatic dependent follows a kernel, not this reset; with a cluster per request nothing is queued
     if (!(cfg && cfg->pdl) && (cs == 1 || A.n_dev)) {

@@ -317,3 +317,30 @@ def test_serve_rgba_frames_are_the_colour_path(codec, cube16):
         assert by[0]["entered"] >= by[1]["entered"]
     srv.close()
     ds.close()
+
+
+# a brick or two: a launch whose requests are counted on the device holds no more CTAs than there can be requests,
+# four to each where bricks are shared (32^3 and larger), one where they are not
+@pytest.mark.parametrize("brick,each", [(16, 1), (64, 4)])
+def test_decode_launch_of_a_small_data_set(codec, tmp_path, brick, each):
+    import json
+
+    import torch
+    from csvb200 import Server
+    img = _image(codec, (brick, brick, 2 * brick), brick, 43)
+    ds = codec.open(img)
+    srv = Server(codec, ds, W, H, FOV)
+    lab, dep = torch.zeros(W * H, dtype=torch.int64, device="cuda"), torch.zeros(W * H, device="cuda")
+    view = _orbit_views((float(brick), brick / 2, brick / 2), 1, 3.0 * brick, 3.0 * brick)[0]
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+        srv.submit(0, *view, lab, dep)
+        srv.step()
+        frames = srv.poll(wait=True)
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(tmp_path / "t.json"))
+    grids = [e["args"]["grid"][0] for e in json.load(open(tmp_path / "t.json"))["traceEvents"]
+             if e.get("cat") == "kernel" and "decode_kernel" in e["name"]]
+    assert frames[0]["decoded"] == 2 and grids
+    assert max(grids) <= 2 * 8 * each  # (two bricks, a slot for each of eight LODs)
+    srv.close()
+    ds.close()
