@@ -344,3 +344,18 @@ def test_decode_launch_of_a_small_data_set(codec, tmp_path, brick, each):
     assert max(grids) <= 2 * 8 * each  # (two bricks, a slot for each of eight LODs)
     srv.close()
     ds.close()
+
+
+# more blocks wanted in a step than the decode has clusters of CTAs (222 for 32^3 bricks of this many labels, 74 for
+# 64^3), then fewer, some of them fine enough for a cluster each: both ways of one launch, on one server
+@pytest.mark.parametrize("brick,shape,queued", [(32, (256, 256, 288), 222), (64, (320, 320, 256), 74)])
+def test_serve_steps_on_both_sides_of_the_clusters(codec, oracle, brick, shape, queued):
+    import torch
+    vol = torch.empty(shape, dtype=torch.int64, device="cuda")
+    codec.synth_volume(vol, 1, 6000, 3000, 0.7, 2.5, 0.0, 45)
+    codec.encode_device(vol, brick)
+    img = bytes(codec.encoded_image_tensor().cpu().numpy())
+    centre = (shape[2] / 2, shape[1] / 2, shape[0] / 2)
+    views = _orbit_views(centre, 2, 310.0, 300.0) + _orbit_views(centre, 4, 110.0, 60.0)
+    seen = _run_pair(codec, oracle, img, [[(0, v)] for v in views], 2 * 8 * vol.numel(), 0)
+    assert seen["decoded"][0] > queued and 0 < min(seen["decoded"][3:]) <= queued // 2
