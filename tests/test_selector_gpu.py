@@ -227,3 +227,15 @@ def test_selector_file_drives_a_learned_encode(codec, oracle, tmp_path):
     assert np.array_equal(lab, ref)
     net.close()
     net2.close()
+
+
+# the statistics' block layouts: one block a brick (the smallest bricks, and 2048 bricks or more), a block for the sample
+# with one or several for the rows; bricks cut by the volume's end, edge 8 with its own far neighbours and runs
+@pytest.mark.parametrize("shape,brick", [((37, 26, 51), 8), ((208, 208, 208), 16), ((203, 190, 197), 16),
+                                         ((65, 70, 190), 32), ((64, 129, 70), 64)])
+def test_features_of_every_block_layout(codec, oracle, shape, brick):
+    from csvb200.selector import features
+    v = _vol(codec, shape, 9 + brick)
+    f = features(codec, v, brick).cpu().numpy()
+    ref = oracle.brick_features(v.cpu().numpy().view(np.uint64), brick)
+    assert np.array_equal(f.view(np.uint32), ref.view(np.uint32))
