@@ -60,7 +60,7 @@ int decode_batch_static(int device, const DeviceDataset& ds, const csv_request* 
         return CSV_ECUDA;
     }
     DecodeScratch scr;
-    scr.d_queue = reinterpret_cast<uint32_t*>(base);  // cleared by launch_decode before the kernel
+    scr.d_queue = reinterpret_cast<uint32_t*>(base);  // launch_decode clears it where the kernel uses it
     scr.base = base + kQueueBytes;
     scr.per_cta = per;
     scr.ctas = (uint32_t)((CSV_STATIC_SCRATCH_BYTES - kQueueBytes) / per);

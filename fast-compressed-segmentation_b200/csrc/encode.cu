@@ -142,7 +142,7 @@ __device__ __forceinline__ uint32_t morton3(uint32_t x, uint32_t y, uint32_t z) 
 struct EncArgs {
     const uint64_t* vol;
     uint64_t W, H, D;
-    uint32_t b, L, nbx, nby, nbz, nb, S;
+    uint32_t b, L, nbx, nby, nbz, nb;
     uint8_t* scratch;
     uint64_t scratch_per_cta;
     EncMeta* meta;
@@ -314,18 +314,6 @@ __device__ __forceinline__ void enc_place(BrickCtx& B, uint32_t bx, uint32_t by,
     B.z_lim = (uint32_t)min(A.D - z0, (uint64_t)A.b);
     B.interior = B.x_lim == A.b && B.y_lim == A.b && B.z_lim == A.b;
 }
-
-// A warp's word of 32 Morton-consecutive nodes of a level: where lane's node is.
-struct WordAt {
-    uint32_t x, y, z;
-    __device__ __forceinline__ WordAt(uint32_t w) {
-        const uint32_t lane = threadIdx.x & 31u, m = 32 * w;
-        x = demorton_axis(m) | (lane & 1u) | ((lane >> 2) & 2u);
-        y = demorton_axis(m >> 1) | ((lane >> 1) & 1u) | ((lane >> 3) & 2u);
-        z = demorton_axis(m >> 2) | ((lane >> 2) & 1u);
-    }
-    __device__ __forceinline__ uint32_t raster(uint32_t l) const { return x | y << l | z << (2 * l); }
-};
 
 // Position of the k-th set bit of b (k below its number of set bits).
 __device__ __forceinline__ uint32_t nth_bit(uint32_t b, uint32_t k) {
@@ -1369,7 +1357,6 @@ int encode_stats(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W,
     A.b = b; A.L = levels_of(b);
     A.nbx = (uint32_t)nbx; A.nby = (uint32_t)nby; A.nbz = (uint32_t)nbz;
     A.nb = nb;
-    A.S = s->S;
     A.scratch = s->d_scratch;
     A.scratch_per_cta = per_cta;
     A.misc = s->d_misc;
@@ -1456,7 +1443,6 @@ int encode_device(EncoderState* s, int device, const uint64_t* d_vol, uint64_t W
         A.b = b; A.L = s->L;
         A.nbx = (uint32_t)nbx; A.nby = (uint32_t)nby; A.nbz = (uint32_t)nbz;
         A.nb = nb;
-        A.S = s->S;
         A.scratch = s->d_scratch;
         A.scratch_per_cta = per_cta;
         A.meta = s->d_meta;

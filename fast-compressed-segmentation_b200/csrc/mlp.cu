@@ -364,8 +364,9 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
 //   K-chunks through a two-slot ring of bulk copies (it does not fit beside
 //   the rest), H2 = bf16(relu(acc2 + b2)) -> shared memory
 //   acc3 = H2 W3^T (TMEM cols 0..31), logits = acc3 + b3, argmax per head.
-// The MMAs are the ones the layer-by-layer GEMMs issue (same shapes, same K
-// order), so the logits are those of gemm_bf16_kernel's three launches.
+// A layer's products are added in the K order of the layer-by-layer GEMMs (whose tiles
+// are narrower, which changes no sum), so the logits are those of gemm_bf16_kernel's
+// three launches.
 // Weights come pre-tiled in the no-swizzle K-major core-matrix layout, so that
 // each K-chunk is one contiguous bulk copy: K-chunks of 64, each N/8 x 8 core matrices
 // of 8 rows x 16 bytes, core (g, c) at (g * 8 + c) * 128 bytes.

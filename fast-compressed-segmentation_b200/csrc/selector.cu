@@ -188,8 +188,9 @@ __device__ uint32_t sample_stats(FeatShared& S, const uint64_t* vol, uint64_t W,
 // a quarter of the voxels, every pair within such a row, and each such voxel's +1 / +4
 // neighbours in y and z), a row per warp at a time with its four neighbour rows read
 // beside it, so that ten loads per lane are in flight.  The sample's statistics, a serial
-// walk, are a CTA of their own, and these come first.  Counts meet in the brick's feature row as whole numbers (zeroed by the
-// launch); the last CTA to add its own turns them into the features.
+// walk, are a CTA of their own, and these come first (one CTA does both where a brick has
+// one).  Counts meet in the brick's feature row as whole numbers (zeroed by the launch);
+// the last CTA to add its own turns them into the features.
 // Row words: 0 .. 14 counts, 15 CTAs done | distinct << 16, 16 .. 31 op nibbles.
 // Measured (B200, 320 bricks of 64^3): 0.41 -> 0.156 ms (one CTA per brick with planes
 // kept in registers, the runs counted start by start and the sample's ops walked by one

@@ -79,8 +79,9 @@ typedef struct csv_dataset_info {
 
 /* ---- context --------------------------------------------------------
  * A context keeps its decode scratch (grown to the largest brick size seen)
- * and a stream-ordered memory pool for the temporaries of csv_open that holds
- * up to 1 GiB of freed memory between opens; csv_destroy releases both. */
+ * and a stream-ordered memory pool for the temporaries of csv_open and
+ * csv_encode_learned that holds up to 1 GiB of freed memory between calls;
+ * csv_destroy releases both. */
 int csv_create(int device, csv_ctx** out);
 void csv_destroy(csv_ctx* ctx);
 const char* csv_last_error(const csv_ctx* ctx);
@@ -446,7 +447,8 @@ int csv_serve_destroy(csv_server* srv);
  * NULL), max(0, .) (if relu), * (d_mask[m][n] > 0) (if d_mask, bf16 [M][N]: the
  * ReLU gradient); outputs (each optional): d_C fp32 [M][N], d_Cb bf16 [M][N],
  * d_CbT bf16 [N][M], d_CT fp32 [N][M].  M % 128 == 0, N % 16 == 0, K % 64 == 0.
- * d_err (optional) is set to 1 if a bounded wait gave up. */
+ * An output may lie over an operand (a layer in place: K == N for d_Cb over d_A)
+ * up to N = 256.  d_err (optional) is set to 1 if a bounded wait gave up. */
 int csv_gemm_bf16(csv_ctx* ctx, const void* d_A, const void* d_B, uint32_t M, uint32_t N, uint32_t K,
                   const float* d_bias, const void* d_mask, uint32_t relu, float* d_C, void* d_Cb, void* d_CbT,
                   float* d_CT, uint32_t* d_err, void* stream);
