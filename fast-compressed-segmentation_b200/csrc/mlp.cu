@@ -34,8 +34,8 @@ namespace {
 
 constexpr uint32_t kGemmThreads = 128;
 constexpr uint32_t kKChunk = 64;               // bf16 elements per row per chunk (128 bytes)
-constexpr uint32_t kTileN = 64;                // columns staged at a time
-constexpr uint32_t kTileInPlace = 256;         // columns per CTA at most, of row-major operands under an output
+constexpr uint32_t kTileN = 64;                // columns per CTA at most
+constexpr uint32_t kTileWide = 256;            // the same in the wide form, which stages kTileN of them at a time
 constexpr uint32_t kStages = 4;
 constexpr uint32_t kTileA = 128 * kKChunk * 2; // 16 KB
 constexpr uint32_t kTileB = kTileN * kKChunk * 2;  // 8 KB
@@ -159,7 +159,7 @@ __device__ __forceinline__ float loss_grad_row(const float (&z)[32], uint32_t la
 // loaded and multiplied in turn, products over the rows on 2 CTAs, bias sums by one block
 // each): 0.87 -> 0.105 ms of kernels (0.7 us at the bf16 rate); a 2048 x 256 x 256 layer
 // 74 -> 9.5 us, the 256 x 256 product over the rows 171 -> 20 us beside the next layer's.
-template <bool TILED>
+template <bool TILED, bool WIDE>
 __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, GemmArgs G1, uint32_t n_first) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t bars[kStages], full[kStages];  // a stage's products done; its copies landed (TILED)
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
     const uint32_t mt = G.M / 128u;
     const uint32_t m0 = (blk % mt) * 128u, n0 = (blk / mt) * G.tile_n;
     const uint32_t N = min(G.tile_n, G.N - n0);
-    const uint32_t ncols = N <= 32 ? 32u : (N <= 64 ? 64u : (N <= 128 ? 128u : 256u));
+    const uint32_t ncols = N <= 32 ? 32u : (!WIDE || N <= 64 ? 64u : (N <= 128 ? 128u : 256u));
     const uint32_t sA = smem_u32(smem), sB = sA + kStages * kTileA;
     if (tid == 0) {
         for (uint32_t s = 0; s < kStages; ++s) {
@@ -233,13 +233,15 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
         __syncthreads();
         ok = s_ok != 0;
     } else {
-        // 64 columns at a time, all of K each; step c is chunk c % chunks of columns 64 (c / chunks) on
-        const uint32_t steps = (N + kTileN - 1) / kTileN * chunks;
+        // a step is a chunk of K; WIDE: of 64 columns, all of K for these before the next ones
+        const uint32_t steps = WIDE ? (N + kTileN - 1) / kTileN * chunks : chunks;
+        auto col = [&](uint32_t c) { return WIDE ? c / chunks * kTileN : 0u; };
+        auto chunk = [&](uint32_t c) { return WIDE ? c % chunks : c; };
         auto load = [&](uint32_t c) {  // step c's operands into its stage; a group of copies either way
             if (c < steps) {
-                const uint32_t col = c / chunks * kTileN, k0 = c % chunks * kKChunk;
-                load_operand(sA + (c % kStages) * kTileA, G.A, G.K, m0, 128u, k0);
-                load_operand(sB + (c % kStages) * kTileB, G.B, G.K, n0 + col, min(N - col, kTileN), k0);
+                load_operand(sA + (c % kStages) * kTileA, G.A, G.K, m0, 128u, chunk(c) * kKChunk);
+                load_operand(sB + (c % kStages) * kTileB, G.B, G.K, n0 + col(c), WIDE ? min(N - col(c), kTileN) : N,
+                             chunk(c) * kKChunk);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
@@ -250,8 +252,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(GemmArgs G0, Ge
             if (!(ok = __syncthreads_and(ok))) break;  // one decision for the whole block
             if (tid == 0) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t col = c / chunks * kTileN;
-                multiply(c, col, min(N - col, kTileN), c % chunks == 0);
+                multiply(c, col(c), WIDE ? min(N - col(c), kTileN) : N, chunk(c) == 0);
             }
             if (c > 0) ok = done(c - 1);
             if (ok) load(c + kStages - 1);
@@ -669,13 +670,16 @@ cudaError_t launch_gemm_bf16(const GemmArgs& g, cudaStream_t st, const GemmArgs*
     if (g.M == 0 || g.N == 0 || g.K == 0) return cudaSuccess;
     for (const GemmArgs* p : {&g, second})
         if (p && (p->M % 128 || p->N % 16 || p->K % kKChunk || p->tile_n == 0 || p->tile_n % 16 ||
-                  p->tile_n > (p->tiled ? kTileN : kTileInPlace)))
+                  p->tile_n > (p->tiled ? kTileN : kTileWide)))
             return cudaErrorInvalidValue;
-    if (second && second->tiled != g.tiled) return cudaErrorInvalidValue;
+    if (second && (second->tiled != g.tiled || g.tile_n > kTileN || second->tile_n > kTileN))
+        return cudaErrorInvalidValue;
     constexpr int smem = (int)((kTileA + kTileB) * kStages);
-    const auto kernel = g.tiled ? gemm_bf16_kernel<true> : gemm_bf16_kernel<false>;
-    static AllowedOn allowed[2];
-    const cudaError_t e = allow_smem(kernel, smem, allowed[g.tiled]);
+    const int form = g.tiled ? 0 : (g.tile_n <= kTileN ? 1 : 2);
+    const auto kernel = form == 0 ? gemm_bf16_kernel<true, false>
+                                  : (form == 1 ? gemm_bf16_kernel<false, false> : gemm_bf16_kernel<false, true>);
+    static AllowedOn allowed[3];
+    const cudaError_t e = allow_smem(kernel, smem, allowed[form]);
     if (e != cudaSuccess) return e;
     const uint32_t n = gemm_blocks(g);
     kernel<<<n + (second ? gemm_blocks(*second) : 0u), kGemmThreads, smem, st>>>(g, second ? *second : g, n);
@@ -708,8 +712,9 @@ extern "C" int csv_gemm_bf16(csv_ctx* ctx, const void* d_A, const void* d_B, uin
     G.CbT = (__nv_bfloat16*)d_CbT;
     G.CT = d_CT;
     G.err = d_err;
-    // An output over an operand (a layer in place): its rows are written by the CTA that has read them,
-    // so one CTA takes the row of tiles, 256 columns, as long as that is all of them.
+    // An output over an operand (a layer in place): its rows are written by the CTA that has read them, so one CTA
+    // takes the row of tiles, 256 columns, as long as that is all of them.  (89,600 rows x 256 x 256: 0.134 ms, 0.119
+    // beside the operands; 2048 rows 40 and 22 us.)
     auto over = [](const void* out, size_t out_bytes, const void* in, size_t in_bytes) {
         const uintptr_t a = reinterpret_cast<uintptr_t>(out), b = reinterpret_cast<uintptr_t>(in);
         return out && a < b + in_bytes && b < a + out_bytes;
@@ -720,7 +725,7 @@ extern "C" int csv_gemm_bf16(csv_ctx* ctx, const void* d_A, const void* d_B, uin
     const size_t mn = (size_t)M * N;
     if (over_operand(d_C, 4 * mn) || over_operand(d_CT, 4 * mn) || over_operand(d_Cb, 2 * mn) ||
         over_operand(d_CbT, 2 * mn))
-        G.tile_n = kTileInPlace;
+        G.tile_n = kTileWide;
     cudaError_t e = launch_gemm_bf16(G, (cudaStream_t)stream);
     if (e != cudaSuccess) return abi_cuda_fail(ctx, e, "gemm");
     return CSV_OK;

@@ -52,14 +52,14 @@ cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t smem, cud
 }
 cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; return e; }
 
-// what = 0: csv_gemm_bf16; 1: a product of the network's tiled operands; 2: the fused forward
+// what = 0: csv_gemm_bf16; 1: a product of the network's tiled operands; 2: the fused forward; 3: csv_gemm_bf16 in place
 int run(int what, int dev) {
     csv_ctx ctx;
     ctx.device = dev;
     csv::DeviceGuard guard(dev);
     static __nv_bfloat16 A[128 * 64], B[64 * 64], out[128 * 64];
-    if (what == 0)
-        return csv_gemm_bf16(&ctx, A, B, 128, 64, 64, nullptr, nullptr, 0, nullptr, out, nullptr, nullptr, nullptr, nullptr);
+    if (what == 0 || what == 3)
+        return csv_gemm_bf16(&ctx, A, B, 128, 64, 64, nullptr, nullptr, 0, nullptr, what ? A : out, nullptr, nullptr, nullptr, nullptr);
     if (what == 1) {
         csv::GemmArgs g;
         g.A = A; g.B = B; g.M = 128; g.N = 64; g.K = 64; g.tiled = true; g.Cb = out;
@@ -89,7 +89,7 @@ def fake(tmp_path_factory):
     return C.CDLL(so)
 
 
-@pytest.mark.parametrize("what", [0, 1, 2])
+@pytest.mark.parametrize("what", [0, 1, 2, 3])
 def test_shared_memory_is_allowed_on_every_device(fake, what):
     n = fake.launch_count()
     for dev in (0, 1, 0, 70, 1):
